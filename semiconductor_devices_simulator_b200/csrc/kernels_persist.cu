@@ -1,25 +1,38 @@
 // Persistent linear solves: one cooperative launch runs a whole multigrid-preconditioned
-// Krylov solve of an instance - every iteration, both V-cycles of a BiCGSTAB iteration,
-// and for the refined path every FP64 refinement step around its FP32 inner solves -
-// with grid-wide barriers between the dependent passes instead of kernel boundaries.
+// Krylov solve of an instance - the hierarchy set-up, every iteration, both V-cycles of a
+// BiCGSTAB iteration, and for the refined path every FP64 refinement step around its FP32
+// inner solves - with grid-wide barriers between the dependent passes instead of kernel
+// boundaries.
 //
-// Why: on a 576k-node device a V-cycle is ~26 dependent passes of 1-10 MB each.  Launched
-// one kernel per pass (the device-looped CUDA graphs of kernels_la.cu) every pass costs a
-// launch and a grid ramp (~6-9 us) for ~1-2 us of memory traffic; a resident grid pays a
-// barrier (~1-2 us) instead and keeps the level descriptors and the small levels on chip.
+// What bounds it: a V-cycle is a chain of dependent half sweeps, each a pass over a part of
+// one level that is resident in the L2 (below ~1M nodes), so a solve costs (passes) x
+// (barrier + one pass's latency and L2 traffic).  The layout and the passes are built for that:
+//   * the solve keeps its own copy of every level, colour by colour (SLev, semisim.h): a half
+//     sweep reads its couplings, pivots and right-hand side as contiguous pairs and the other
+//     colour's values as contiguous pairs too.  In the natural order every sector of a half
+//     sweep is half unused (576,000 nodes, FP32: a finest-level pass takes 2.3 us, 4.2 us in the
+//     natural order with 1024 threads);
+//   * the red-black D-ILU application is written as red solve / black update with the D-ILU
+//     pivot / red solve.  Red rows are then exact after every application, so no residual array
+//     is kept: the restriction sums black residuals only, the way up needs no residual pass
+//     (its first red solve reads the prolonged black values), and A M^-1 b on red rows is b itself;
+//   * whoever writes a right-hand side also writes the first red values D b, so the first black
+//     half sweep reads them directly;
+//   * the BiCGSTAB iteration's rho comes from the two dot products rh.s and rh.t taken with the
+//     passes before, so x, r and the next p are updated in one pass; PCG takes its step length
+//     from z.A z and the recurrence q = A z + beta q, with one reduction per iteration.
 //
 // Layout of the work:
 //   * every block runs the passes of the large levels (0 .. Ls-1) as grid-stride loops
 //     over the pass's index space, one barrier after each pass;
 //   * block 0 keeps the small levels (Ls .. coarsest) in its shared memory for the whole
-//     solve (staged once at the start, not per V-cycle) and runs their part of every
-//     V-cycle with block barriers, while the other blocks wait at the next grid barrier;
+//     solve and runs their part of every V-cycle with barriers of as many warps as the level
+//     has work for, while the other blocks wait at the next grid barrier;
 //   * reductions: each block writes its partial record, and after the barrier every block
 //     sums all records in block order, so every block holds bit-identical totals and takes
 //     the same stop decisions with no extra barrier.
 //
-// The arithmetic per node is the per-pass kernels' (the shared helpers of la_common.cuh);
-// the stop rules are the reference's (pcg semiconductor_3d.c:2182-2210, bicgstab_core
+// The stop rules are the reference's (pcg semiconductor_3d.c:2182-2210, bicgstab_core
 // :2234-2320) as the per-pass path applies them, and the refinement the same FP64 rule.
 //
 // Safety: the launch is cooperative (all blocks co-resident).  Every barrier wait is
@@ -44,6 +57,11 @@
 
 namespace ss {
 
+// 512 threads of 128 registers: with 1024 of 64 the half sweeps' operands spilled to local
+// memory, which every barrier's acquire throws out of the L1 (a BiCGSTAB solve of the
+// 576,000-node MOSFET: 1278 us with 1024 threads, 1035 us with 512, FP64 1586 and 1095 us)
+constexpr int PT_TPB = 512;
+
 enum PKind { PK_PCG = 0, PK_BICG = 1, PK_REFINED = 2 };
 
 struct PArgs {
@@ -51,9 +69,7 @@ struct PArgs {
     int deep;        // levels (from the finest) with two smoother applications
     int sweeps2;     // 1: the second application is on
     int maxsteps;    // refinement steps at most (PK_REFINED)
-    int fuse_up;     // 1: prolongation deferred into the residual and post-smoothing passes
-    int setup;       // 1: build the hierarchy first (the per-launch mg_setup of kernels_la.cu)
-    int qsign;       // its Slotboom weights: 0 none (Poisson), +1 electrons, -1 holes
+    int qsign;       // Slotboom weights of the hierarchy: 0 none (Poisson), +1 electrons, -1 holes
     unsigned long long *trace;   // barrier timeline of this launch (null: off)
     int ntrace;
     int barmode;                 // grid-barrier form (persist_common.cuh)
@@ -64,215 +80,230 @@ struct PArgs {
     double rtol, atol;   // stop rule of the FP64 BiCGSTAB start (PK_BICG)
 };
 
+// ---------------------------------------------------------------- layout on the host
+// 256-byte aligned arrays of every level and the level-0 vectors, from `base`
+template <class T>
+size_t persist_work_layout(char *base, const int dims[][6], int nlev, SWork<T> *w) {
+    size_t off = 0;
+    auto take = [&](size_t n) {
+        T *p = base ? reinterpret_cast<T *>(base + off) : nullptr;
+        off += (n * sizeof(T) + 255) & ~size_t(255);
+        return p;
+    };
+    for (int L = 0; L < nlev; L++) {
+        SLev<T> v{};
+        v.Nx = dims[L][0]; v.Ny = dims[L][1]; v.Nz = dims[L][2];
+        v.N = v.Nx * v.Ny * v.Nz;
+        v.cx = dims[L][3]; v.cy = dims[L][4]; v.cz = dims[L][5];
+        v.last = L == nlev - 1;
+        v.hx = (((v.Nx + 1) / 2) + 1) & ~1;
+        v.sz = v.hx * v.Ny;
+        v.H = v.sz * v.Nz;
+        v.ap = (2 * v.H + 31) & ~31;
+        v.n8 = (v.Nx + 7) / 8;
+        v.fr = fast_div(v.hx / 2);
+        v.fy = fast_div(v.Ny);
+        v.f8 = fast_div(v.n8);
+        v.A = take((size_t)6 * v.ap);
+        v.G = take((size_t)2 * v.H);
+        v.D = take(v.last ? std::max((size_t)2 * v.H, (size_t)COARSE_MAX * COARSE_MAX) : (size_t)2 * v.H);
+        v.pw = take((size_t)2 * v.H);
+        if (L) { v.x = take((size_t)2 * v.H); v.b = take((size_t)2 * v.H); }
+        if (w) w->lev[L] = v;
+    }
+    const size_t n0 = 2 * (size_t)(((((dims[0][0] + 1) / 2) + 1) & ~1)) * dims[0][1] * dims[0][2];
+    for (int q = 0; q < PW_VEC; q++) { T *p = take(n0); if (w) w->vec[q] = p; }
+    T *p = take(n0);
+    if (w) w->w0 = p;
+    return off;
+}
+template size_t persist_work_layout<double>(char *, const int[][6], int, SWork<double> *);
+template size_t persist_work_layout<float>(char *, const int[][6], int, SWork<float> *);
+
 // ---------------------------------------------------------------- on-chip tables
-// Every descriptor a pass needs (level views, vector pointers) is copied into shared
-// memory once per launch: after each grid barrier the acquire invalidates L1, so a
-// descriptor read from global memory would cost a chain of dependent L2 round trips per
-// pass, more than the pass's own loads on the small levels.
+template <class T> __device__ __forceinline__ const SWork<T> *swork(const DevP &P);
+template <> __device__ __forceinline__ const SWork<double> *swork<double>(const DevP &P) { return P.pwd; }
+template <> __device__ __forceinline__ const SWork<float> *swork<float>(const DevP &P) { return P.pwf; }
+
+// Every descriptor a pass needs is copied into shared memory once per launch: after each
+// grid barrier the acquire invalidates L1, so a descriptor read from global memory would
+// cost a chain of dependent L2 round trips per pass.
 template <class T>
 struct PTab {
-    LevView<T> lev[MAXLEV];      // every level; level 0's x and b are set per V-cycle
-    T *vec[8];                   // level-0 work vectors of precision T
-    T *sol, *rhs;
-    const T *w0;                 // level-0 row weights (continuity systems)
-    const double *A64;           // the FP64 level-0 operator (coupling q at A64 + q * ap64 + k)
+    SWork<T> w;
+    SLev<T> sv[MAXLEV];          // block 0: the levels it keeps in shared memory (index L - Ls)
+    int slot[COARSE_MAX];        // block 0: the coarsest level's slots in the order of its dense inverse
+    SLev<T> cur0;                // level 0 with the running V-cycle's b and x
+    const double *A64;           // the FP64 level-0 operator in natural order (coupling q at A64 + q * ap64 + k)
     int ap64;
-    LevView<T> cur0;             // level 0 with the running V-cycle's b and x
 };
-template <class T>
-__device__ __forceinline__ void ptab_fill(const DevP &P, PTab<T> &tb) {
-    const int nl = P.nlev, t = threadIdx.x;
-    if (t < nl) tb.lev[t] = levview<T>(P, t, 0, 0);
-    if (t >= 32 && t < 40) tb.vec[t - 32] = PT<T>::wk(P, t - 32);
-    if (t == 40) {
-        tb.sol = PT<T>::sol(P);
-        tb.rhs = PT<T>::rhs(P);
-        tb.w0 = PT<T>::w0(P);
-        tb.A64 = P.A[0];
-        tb.ap64 = (int)(P.A[1] - P.A[0]);
-    }
-}
 // level 0 with the V-cycle's b and x, for the passes to read from shared memory (every
 // thread of the block calls it: it ends with a block barrier)
 template <class T>
 __device__ __forceinline__ void set_lev0(PTab<T> &tb, int bsel, int xsel) {
     if (threadIdx.x == 0) {
-        tb.cur0 = tb.lev[0];
-        tb.cur0.b = tb.vec[bsel];
-        tb.cur0.x = tb.vec[xsel];
+        tb.cur0 = tb.w.lev[0];
+        tb.cur0.b = tb.w.vec[bsel];
+        tb.cur0.x = tb.w.vec[xsel];
     }
     __syncthreads();
 }
 
-// ---------------------------------------------------------------- grid passes of a level
-// (i, j, l) and node index of item t of a half sweep over one colour
-struct HItem { int k, i, j, l; bool ok; };
-template <class T>
-__device__ __forceinline__ HItem hitem(const LevView<T> &v, int t, int tot, int color) {
-    HItem h;
-    h.ok = t < tot;
-    if (!h.ok) { h.k = h.i = h.j = h.l = 0; return h; }
-    const int hx = (v.Nx + 1) >> 1;
-    const int row = t / hx, ti = t - row * hx;
-    h.l = row / v.Ny;
-    h.j = row - h.l * v.Ny;
-    h.i = 2 * ti + ((h.j + h.l + color) & 1);
-    h.ok = h.i < v.Nx;
-    h.k = h.i + v.Nx * row;
-    return h;
+// ---------------------------------------------------------------- slots
+template <class T> struct alignas(2 * sizeof(T)) Two { T a, b; };
+template <class T> __device__ __forceinline__ Two<T> ld2(const T *p) { return *reinterpret_cast<const Two<T> *>(p); }
+template <class T> __device__ __forceinline__ void st2(T *p, T a, T b) { *reinterpret_cast<Two<T> *>(p) = Two<T>{a, b}; }
+__device__ __forceinline__ int fdiv(int n, FastDiv f) {
+    return (int)((__umulhi((unsigned)n, f.mul) + (unsigned)n) >> f.sh);
 }
-// new x (and the z parked in r for the other colour's sweep) of one node of a half sweep,
-// without storing: the smoother update of smooth_node (la_common.cuh) split into its
-// loads and its stores, so that two nodes' loads can be in flight together (a node of the
-// sweep's colour reads only the other colour's nodes and itself)
+// slot of node (i, j, l), colour included
 template <class T>
-struct SmRes { T x, r; };
+__device__ __forceinline__ int sslot(const SLev<T> &v, int i, int j, int l) {
+    return (((i + j + l) & 1) ? v.H : 0) + v.hx * (j + v.Ny * l) + (i >> 1);
+}
+// values of the other colour as a half sweep reads them: two neighbouring slots of row
+// (j, l), or one (whose slot may lie just outside the row: its coupling is then zero)
 template <class T>
-__device__ __forceinline__ SmRes<T> smooth_eval(const LevView<T> &v, const HItem &h, int mode, int color) {
-    SmRes<T> o;
-    const int k = h.k;
-    if (mode == 2) {
-        if (color) {
-            const T z = (v.b[k] - lv_apply<T>(v, v.x, k, h.i, h.j, h.l)) * v.D[k];
-            o.x = v.x[k] + z;
-            o.r = z;
-        } else {
-            o.x = v.x[k] - lv_offdiag<T>(v, v.r, k, h.i, h.j, h.l) * v.D[k];
-            o.r = 0;
-        }
-        return o;
+struct SrcX {
+    const T *x;
+    __device__ __forceinline__ Two<T> two(int m, int, int) const { return ld2(x + m); }
+    __device__ __forceinline__ T one(int m, int, int) const { return x[m]; }
+};
+// black values with the coarse correction added: x + al pw xc
+template <class T>
+struct SrcP {
+    const T *x, *pw, *xc;
+    T al;
+    int hx, Ny, cx, cy, cz, cNx, cNy, chx, cH;
+    __device__ __forceinline__ SrcP(const SLev<T> &v, const SLev<T> &c, T al_)
+        : x(v.x + v.H), pw(v.pw + v.H), xc(c.x), al(al_), hx(v.hx), Ny(v.Ny), cx(v.cx), cy(v.cy), cz(v.cz),
+          cNx(c.Nx), cNy(c.Ny), chx(c.hx), cH(c.H) {}
+    __device__ __forceinline__ T coarse(int t, int j, int l) const {
+        const int J = j >> cy, K = l >> cz;
+        const int I = min(cx ? t : 2 * t + ((j + l + 1) & 1), cNx - 1);   // (past the row: a padding slot, weight zero)
+        return xc[(((I + J + K) & 1) ? cH : 0) + chx * (J + cNy * K) + (I >> 1)];
     }
-    const T *src = mode ? v.r : v.b;
-    T z;
-    if (color) z = (src[k] - lv_offdiag_scaled<T>(v, src, k, h.i, h.j, h.l)) * v.D[k];
-    else z = (src[k] - lv_offdiag<T>(v, mode ? v.r : v.x, k, h.i, h.j, h.l)) * v.D[k];
-    o.x = mode ? v.x[k] + z : z;
-    o.r = z;
-    return o;
-}
-// the stores of smooth_eval's result (r only where the sweep parks z: black, modes 1, 2)
-template <class T>
-__device__ __forceinline__ void smooth_store(const LevView<T> &v, const HItem &h, const SmRes<T> &o, int mode,
-                                             int color) {
-    v.x[h.k] = o.x;
-    if (color && mode) v.r[h.k] = o.r;
-}
-// prolongation of the coarse correction to node h (added by the deferred way up)
-template <class T>
-__device__ __forceinline__ T prol_at(const LevView<T> &f, const LevView<T> &cl, T al, int k, int i, int j, int l) {
-    const int I = f.cx ? i >> 1 : i, J = f.cy ? j >> 1 : j, K = f.cz ? l >> 1 : l;
-    return al * f.pw[k] * cl.x[I + cl.Nx * (J + cl.Ny * K)];
-}
-// half sweep of one colour, two nodes per thread and loop trip; cl non-null: post-
-// smoothing with the deferred prolongation added to each node first (mode 1)
-template <class T>
-__device__ PG_PASS void pg_smooth(const LevView<T> &vr, int mode, int color, const PS &s,
-                                       const LevView<T> *clr = nullptr, T al = 0) {
-    const LevView<T> v = vr;                      // register copies of the shared-memory views
-    LevView<T> clv;
-    const LevView<T> *cl = nullptr;
-    if (clr) { clv = *clr; cl = &clv; }
-    const int hx = (v.Nx + 1) >> 1, tot = hx * v.Ny * v.Nz;
-    for (int t = s.tid; t < tot; t += 2 * s.nth) {
-        const HItem h1 = hitem(v, t, tot, color), h2 = hitem(v, t + s.nth, tot, color);
-        SmRes<T> o1{0, 0}, o2{0, 0};
-        T p1 = 0, p2 = 0;
-        if (h1.ok) {
-            o1 = smooth_eval<T>(v, h1, mode, color);
-            if (cl) p1 = prol_at<T>(v, *cl, al, h1.k, h1.i, h1.j, h1.l);
-        }
-        if (h2.ok) {
-            o2 = smooth_eval<T>(v, h2, mode, color);
-            if (cl) p2 = prol_at<T>(v, *cl, al, h2.k, h2.i, h2.j, h2.l);
-        }
-        if (h1.ok) { o1.x += p1; smooth_store<T>(v, h1, o1, mode, color); }
-        if (h2.ok) { o2.x += p2; smooth_store<T>(v, h2, o2, mode, color); }
+    __device__ __forceinline__ Two<T> two(int m, int j, int l) const {
+        const Two<T> v = ld2(x + m), p = ld2(pw + m);
+        const int t = m - hx * (j + Ny * l);
+        return Two<T>{v.a + al * p.a * coarse(t, j, l), v.b + al * p.b * coarse(t + 1, j, l)};
     }
-}
-// weighted residual of every fine node summed into its 2x2x2 aggregate: 8 lanes per
-// coarse node (lane bits di, dj, dl), whole warps per loop trip, two trips' loads together
-template <class T>
-__device__ __forceinline__ T rr_val(const LevView<T> &f, const LevView<T> &cl, const T *w, int t) {
-    const int K = t >> 3, sub = t & 7;
-    if (K >= cl.N) return 0;
-    const Node c = unidx(K, cl.Nx, cl.Ny);
-    const int di = sub & 1, dj = (sub >> 1) & 1, dl = sub >> 2;
-    const int i = f.cx ? 2 * c.i + di : c.i, j = f.cy ? 2 * c.j + dj : c.j, l = f.cz ? 2 * c.l + dl : c.l;
-    const bool ok = i < f.Nx && j < f.Ny && l < f.Nz && (f.cx || di == 0) && (f.cy || dj == 0) && (f.cz || dl == 0);
-    if (!ok) return 0;
-    const int k = i + f.Nx * (j + f.Ny * l);
-    const T r = f.b[k] - lv_apply<T>(f, f.x, k, i, j, l);
-    return w ? w[k] * r : r;
-}
-template <class T>
-__device__ __forceinline__ T oct_sum(T v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    return v;
-}
-template <class T>
-__device__ PG_PASS void pg_resid_restrict(const LevView<T> &fr, const LevView<T> &clr, const T *w, const PS &s) {
-    const LevView<T> f = fr, cl = clr;            // register copies of the shared-memory views
-    const int nK = ((cl.N + 3) >> 2) << 5;
-    for (int t = s.tid; t < nK; t += 2 * s.nth) {
-        const int t2 = t + s.nth;                 // whole warps: nK and nth are multiples of 32
-        T v1 = rr_val<T>(f, cl, w, t);
-        T v2 = t2 < nK ? rr_val<T>(f, cl, w, t2) : T(0);
-        v1 = oct_sum<T>(v1);
-        if (t2 < nK) v2 = oct_sum<T>(v2);
-        if ((t & 7) == 0 && (t >> 3) < cl.N) cl.b[t >> 3] = v1;
-        if (t2 < nK && (t2 & 7) == 0 && (t2 >> 3) < cl.N) cl.b[t2 >> 3] = v2;
+    __device__ __forceinline__ T one(int m, int j, int l) const {
+        int t = m - hx * (j + Ny * l);
+        t = t < 0 ? 0 : (t > hx - 1 ? hx - 1 : t);
+        return x[m] + al * pw[m] * coarse(t, j, l);
     }
-}
-template <class T>
-__device__ PG_PASS void pg_prolong(const LevView<T> &fr, const LevView<T> &clr, T al, const PS &s) {
-    const LevView<T> f = fr, cl = clr;
-    for (int k = s.tid; k < f.N; k += s.nth) {
-        const Node a = unidx(k, f.Nx, f.Ny);
-        f.x[k] += prol_at<T>(f, cl, al, k, a.i, a.j, a.l);
-    }
-}
-template <class T>
-__device__ PG_PASS void pg_resid(const LevView<T> &fr, const PS &s) {
-    const LevView<T> f = fr;
-    for (int k = s.tid; k < f.N; k += s.nth) {
-        const Node a = unidx(k, f.Nx, f.Ny);
-        f.r[k] = f.b[k] - lv_apply<T>(f, f.x, k, a.i, a.j, a.l);
-    }
+};
+
+// sum of a_kj x_j over the neighbours of the slots m, m + 1 of colour c in row (j, l)
+template <class T, class S>
+__device__ __forceinline__ Two<T> nb_sum(const SLev<T> &v, int c, int m, int j, int l, const S &src) {
+    const T *A = v.A + c * v.H + m;
+    const int o = (j + l + c) & 1;                          // node i = 2 (slot in row) + o
+    int me = o ? m + 2 : m - 1;
+    me = me < 0 ? 0 : (me > v.H - 1 ? v.H - 1 : me);
+    const bool jm = j > 0, jp = j < v.Ny - 1, lm = l > 0, lp = l < v.Nz - 1;
+    const Two<T> axm = ld2(A), axp = ld2(A + v.ap), aym = ld2(A + 2 * v.ap), ayp = ld2(A + 3 * v.ap),
+                 azm = ld2(A + 4 * v.ap), azp = ld2(A + 5 * v.ap);
+    const Two<T> xc = src.two(m, j, l);
+    const T e = src.one(me, j, l);
+    const Two<T> ym = src.two(jm ? m - v.hx : m, jm ? j - 1 : j, l), yp = src.two(jp ? m + v.hx : m, jp ? j + 1 : j, l);
+    const Two<T> zm = src.two(lm ? m - v.sz : m, j, lm ? l - 1 : l), zp = src.two(lp ? m + v.sz : m, j, lp ? l + 1 : l);
+    Two<T> s;
+    s.a = axm.a * (o ? xc.a : e) + axp.a * (o ? xc.b : xc.a);
+    s.b = axm.b * (o ? xc.b : xc.a) + axp.b * (o ? e : xc.b);
+    s.a += aym.a * ym.a; s.b += aym.b * ym.b;
+    s.a += ayp.a * yp.a; s.b += ayp.b * yp.b;
+    s.a += azm.a * zm.a; s.b += azm.b * zm.b;
+    s.a += azp.a * zp.a; s.b += azp.b * zp.b;
+    return s;
 }
 
-// The way up, with the prolongation deferred: the residual pass reads the prolonged
-// x + al pw P xc at each stencil point without writing it, and each post-smoothing half
-// sweep adds the prolongation to its own colour's nodes - the same operations as a
-// prolongation pass followed by a residual pass, one barrier fewer.
-template <class T>
-__device__ __forceinline__ T xprol(const LevView<T> &f, const LevView<T> &cl, T al, int m, int i, int j, int l) {
-    return f.x[m] + prol_at<T>(f, cl, al, m, i, j, l);
+// ---------------------------------------------------------------- passes of a level
+// Half sweeps over one colour.  SM_B0: black from the first red values; SM_R: red, solving
+// its rows exactly; SM_B: black update with the full residual; SM_RP / SM_BP: the same two
+// with the coarse correction added to the black values as they are read.
+enum { SM_B0, SM_R, SM_B, SM_RP, SM_BP };
+template <class T, int MODE>
+__device__ PG_PASS void pg_smooth(const SLev<T> &vr, int tid, int nth, const SLev<T> *clr = nullptr, T al = 0) {
+    const SLev<T> v = vr;                                   // register copy of the shared-memory view
+    constexpr int c = (MODE == SM_R || MODE == SM_RP) ? 0 : 1;
+    const int np = v.H >> 1;
+    for (int t = tid; t < np; t += nth) {
+        const int row = fdiv(t, v.fr), l = fdiv(row, v.fy), j = row - l * v.Ny, m = 2 * t;
+        const int k = c * v.H + m;
+        const Two<T> D = ld2(v.D + k), b = ld2(v.b + k);
+        if constexpr (MODE == SM_RP) {
+            const Two<T> s = nb_sum<T>(v, c, m, j, l, SrcP<T>(v, *clr, al));
+            st2(v.x + k, (b.a - s.a) * D.a, (b.b - s.b) * D.b);
+        } else {
+            const SrcX<T> src{v.x + (1 - c) * v.H};
+            if constexpr (MODE == SM_B0 || MODE == SM_R) {
+                const Two<T> s = nb_sum<T>(v, c, m, j, l, src);
+                st2(v.x + k, (b.a - s.a) * D.a, (b.b - s.b) * D.b);
+            } else {
+                Two<T> x;
+                if constexpr (MODE == SM_BP) x = SrcP<T>(v, *clr, al).two(m, j, l);
+                else x = ld2(v.x + k);
+                const Two<T> g = ld2(v.G + k);
+                const Two<T> s = nb_sum<T>(v, c, m, j, l, src);
+                st2(v.x + k, x.a + (b.a - g.a * x.a - s.a) * D.a, x.b + (b.b - g.b * x.b - s.b) * D.b);
+            }
+        }
+    }
 }
+// black values with the coarse correction added
 template <class T>
-__device__ __forceinline__ T pr_val(const LevView<T> &f, const LevView<T> &cl, T al, int k) {
-    const int NxNy = f.Nx * f.Ny;
-    const Node a = unidx(k, f.Nx, f.Ny);
-    const int i = a.i, j = a.j, l = a.l;
-    T sum = f.a(0, k) * xprol<T>(f, cl, al, k, i, j, l);
-    if (i > 0) sum += f.a(1, k) * xprol<T>(f, cl, al, k - 1, i - 1, j, l);
-    if (i < f.Nx - 1) sum += f.a(2, k) * xprol<T>(f, cl, al, k + 1, i + 1, j, l);
-    if (j > 0) sum += f.a(3, k) * xprol<T>(f, cl, al, k - f.Nx, i, j - 1, l);
-    if (j < f.Ny - 1) sum += f.a(4, k) * xprol<T>(f, cl, al, k + f.Nx, i, j + 1, l);
-    if (l > 0) sum += f.a(5, k) * xprol<T>(f, cl, al, k - NxNy, i, j, l - 1);
-    if (l < f.Nz - 1) sum += f.a(6, k) * xprol<T>(f, cl, al, k + NxNy, i, j, l + 1);
-    return f.b[k] - sum;
+__device__ PG_PASS void pg_prolong(const SLev<T> &vr, const SLev<T> &cl, T al, int tid, int nth) {
+    const SLev<T> v = vr;
+    const SrcP<T> src(v, cl, al);
+    for (int t = tid; t < (v.H >> 1); t += nth) {
+        const int row = fdiv(t, v.fr), l = fdiv(row, v.fy), j = row - l * v.Ny;
+        const Two<T> x = src.two(2 * t, j, l);
+        st2(v.x + v.H + 2 * t, x.a, x.b);
+    }
 }
+// residual of one black slot m (red rows are exact after a sweep)
 template <class T>
-__device__ PG_PASS void pg_prolong_resid(const LevView<T> &fr, const LevView<T> &clr, T al, const PS &s) {
-    const LevView<T> f = fr, cl = clr;            // register copies of the shared-memory views
-    for (int k = s.tid; k < f.N; k += 2 * s.nth) {
-        const int k2 = k + s.nth;
-        const T r1 = pr_val<T>(f, cl, al, k);
-        const T r2 = k2 < f.N ? pr_val<T>(f, cl, al, k2) : T(0);
-        f.r[k] = r1;
-        if (k2 < f.N) f.r[k2] = r2;
+__device__ __forceinline__ T black_resid(const SLev<T> &v, int m, int j, int l) {
+    const T *A = v.A + v.H + m, *x = v.x;
+    const int o = (j + l + 1) & 1;
+    int xm = m - 1 + o, xp = m + o;
+    xm = xm < 0 ? 0 : xm;
+    xp = xp > v.H - 1 ? v.H - 1 : xp;
+    const int ym = j > 0 ? m - v.hx : m, yp = j < v.Ny - 1 ? m + v.hx : m;
+    const int zm = l > 0 ? m - v.sz : m, zp = l < v.Nz - 1 ? m + v.sz : m;
+    T s = A[0] * x[xm] + A[v.ap] * x[xp] + A[2 * v.ap] * x[ym] + A[3 * v.ap] * x[yp] + A[4 * v.ap] * x[zm] +
+          A[5 * v.ap] * x[zp];
+    return v.b[v.H + m] - v.G[v.H + m] * x[v.H + m] - s;
+}
+// Weighted residual summed into the 2x2x2 aggregates: a warp takes 8 coarse nodes along x
+// times the aggregate's 4 rows (lane = 8 (dj + 2 dl) + node), so the fine reads of 8 lanes
+// are contiguous; `pre` also writes the coarse level's first red values D b.
+template <class T>
+__device__ PG_PASS void pg_restrict(const SLev<T> &fr, const SLev<T> &clr, const T *w, int tid, int nth, bool pre) {
+    const SLev<T> f = fr, cl = clr;
+    const int lane = tid & 31, sub = lane >> 3, dj = sub & 1, dl = sub >> 1;
+    const int ng = cl.n8 * cl.Ny * cl.Nz, nw = nth >> 5;
+    for (int g = tid >> 5; g < ng; g += nw) {
+        const int row = fdiv(g, cl.f8), K = fdiv(row, cl.fy), J = row - K * cl.Ny;
+        const int I = 8 * (g - row * cl.n8) + (lane & 7);
+        const int j = f.cy ? 2 * J + dj : J, l = f.cz ? 2 * K + dl : K;
+        bool ok = I < cl.Nx && j < f.Ny && l < f.Nz && (f.cy || !dj) && (f.cz || !dl);
+        if (!f.cx) ok = ok && ((I + j + l) & 1);
+        T r = 0;
+        if (ok) {
+            const int m = (f.cx ? I : I >> 1) + f.hx * (j + f.Ny * l);
+            r = black_resid<T>(f, m, j, l);
+            if (w) r *= w[f.H + m];
+        }
+        r += __shfl_xor_sync(0xffffffffu, r, 8);
+        r += __shfl_xor_sync(0xffffffffu, r, 16);
+        if (sub == 0 && I < cl.Nx) {
+            const int q = sslot(cl, I, J, K);
+            cl.b[q] = r;
+            if (pre && !((I + J + K) & 1)) cl.x[q] = cl.D[q] * r;
+        }
     }
 }
 
@@ -281,158 +312,208 @@ __device__ PG_PASS void pg_prolong_resid(const LevView<T> &fr, const LevView<T> 
         if (!pg_sync(s)) return false; \
     } while (0)
 
-// The passes of one level on the way down (pre-smoothing, residual restricted to the next
-// level) and on the way up (prolongation, residual, post-smoothing), each pass followed by
-// `sync` - the grid barrier, or the first cluster's hardware barrier for the levels it runs
-// alone.  The same passes as the per-pass path (vcycle_t in kernels_la.cu).
+// The passes of one level on the way down (pre-smoothing from zero, residual restricted to
+// the next level) and on the way up (prolongation, post-smoothing), each pass followed by
+// `sync` - the grid barrier, a cluster's, or a barrier of some warps of block 0.
 template <class T, class Sync>
-__device__ __forceinline__ bool pg_level_down(const PS &e, const PArgs &a, PTab<T> &tb, int L, int wsel, Sync sync) {
-    const LevView<T> &v = L ? tb.lev[L] : tb.cur0;
-    pg_smooth<T>(v, 0, 1, e);
+__device__ __forceinline__ bool pg_level_down(int tid, int nth, const SLev<T> &v, const SLev<T> &cl, bool twice,
+                                              const T *w, bool pre, Sync sync) {
+    pg_smooth<T, SM_B0>(v, tid, nth);
     if (!sync()) return false;
-    pg_smooth<T>(v, 0, 0, e);
+    pg_smooth<T, SM_R>(v, tid, nth);
     if (!sync()) return false;
-    if (L < a.deep && a.sweeps2) {
-        pg_smooth<T>(v, 2, 1, e);
+    if (twice) {
+        pg_smooth<T, SM_B>(v, tid, nth);
         if (!sync()) return false;
-        pg_smooth<T>(v, 2, 0, e);
+        pg_smooth<T, SM_R>(v, tid, nth);
         if (!sync()) return false;
     }
-    pg_resid_restrict<T>(v, tb.lev[L + 1], (L == 0 && wsel) ? tb.w0 : nullptr, e);
+    pg_restrict<T>(v, cl, w, tid, nth, pre);
     return sync();
 }
-template <class T, class Sync>
-__device__ __forceinline__ bool pg_level_up(const PS &e, const PArgs &a, PTab<T> &tb, int L, Sync sync) {
-    const T al = (T)a.alpha;
-    const LevView<T> &v = L ? tb.lev[L] : tb.cur0;
-    const LevView<T> &cl = tb.lev[L + 1];
-    if (a.fuse_up) {
-        pg_prolong_resid<T>(v, cl, al, e);
+template <class T, bool FUSED, class Sync>
+__device__ __forceinline__ bool pg_level_up(int tid, int nth, const SLev<T> &v, const SLev<T> &cl, bool twice, T al,
+                                            Sync sync) {
+    if constexpr (FUSED) {
+        pg_smooth<T, SM_RP>(v, tid, nth, &cl, al);
         if (!sync()) return false;
-        pg_smooth<T>(v, 1, 1, e, &cl, al);
+        pg_smooth<T, SM_BP>(v, tid, nth, &cl, al);
         if (!sync()) return false;
-        pg_smooth<T>(v, 1, 0, e, &cl, al);
+        pg_smooth<T, SM_R>(v, tid, nth);
         if (!sync()) return false;
-    } else {
-        pg_prolong<T>(v, cl, al, e);
+    } else {                         // a barrier among a few warps costs less than gathering through the weights
+        pg_prolong<T>(v, cl, al, tid, nth);
         if (!sync()) return false;
-        pg_resid<T>(v, e);
-        if (!sync()) return false;
-        pg_smooth<T>(v, 1, 1, e);
-        if (!sync()) return false;
-        pg_smooth<T>(v, 1, 0, e);
-        if (!sync()) return false;
+        for (int q = 0; q < 2; q++) {
+            pg_smooth<T, SM_R>(v, tid, nth);
+            if (!sync()) return false;
+            if (q) break;
+            pg_smooth<T, SM_B>(v, tid, nth);
+            if (!sync()) return false;
+        }
     }
-    if (L < a.deep && a.sweeps2) {
-        pg_smooth<T>(v, 2, 1, e);
+    if (twice) {
+        pg_smooth<T, SM_B>(v, tid, nth);
         if (!sync()) return false;
-        pg_smooth<T>(v, 2, 0, e);
+        pg_smooth<T, SM_R>(v, tid, nth);
         if (!sync()) return false;
     }
     return true;
 }
 
-// one V(1,1) cycle x = M^-1 b on the level-0 vectors (bsel -> xsel).  Levels 0 .. Lc-1: the
-// whole grid, grid barriers; levels Lc .. Ls-1: the first cluster alone, cluster barriers
-// (0.3 us against 2.2 us for a grid barrier); levels Ls ..: block 0 in shared memory.
+// barrier of the first n threads of the block (whole warps), one hardware barrier per level
+__device__ __forceinline__ bool warps_sync(int id, int n) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+    return true;
+}
+// The levels Ls .. coarsest of a V-cycle in block 0's shared memory.  Level L runs on its
+// first nt threads (as many as it has pairs of slots; fewer on the deeper levels): the other
+// warps wait at the barrier of the level above.  1024-thread barriers and the natural-order
+// loops took 15 us a cycle on 1200 + 160 + 24 unknowns, this 8 us.
 template <class T>
-__device__ __noinline__ bool pg_vcycle(PS &s, const PArgs &a, PTab<T> &tb, const LevView<T> *sv, int nl, int bsel, int xsel,
-                          int wsel) {
+__device__ __noinline__ void blk_cycle(const PTab<T> &tb, int Ls, int nl, T al, int deep) {
+    const SLev<T> *sv = tb.sv;
+    const int tid = threadIdx.x;
+    int L = Ls;
+    for (; L < nl - 1; L++) {
+        const int nt = sv[L - Ls].nt;
+        if (tid >= nt) break;
+        pg_level_down<T>(tid, nt, sv[L - Ls], sv[L + 1 - Ls], L < deep, nullptr, L + 1 < nl - 1,
+                         [&]() { return warps_sync(1 + L - Ls, nt); });
+    }
+    if (L == nl - 1) {                            // coarsest level: x = inverse b, 8 lanes per row
+        const SLev<T> &v = sv[nl - 1 - Ls];
+        const int n = v.N, q0 = tid & 7;
+        const int *slot = tb.slot;
+        if (tid < v.nt) {
+            for (int r = tid >> 3; r < ((n + 3) & ~3); r += v.nt >> 3) {
+                T sum = 0;
+                if (r < n) {
+#pragma unroll 4
+                    for (int q = q0; q < n; q += 8) sum += v.D[r * n + q] * v.b[slot[q]];
+                }
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                if (q0 == 0 && r < n) v.x[slot[r]] = sum;
+            }
+        }
+    }
+    // each level's threads meet again: the ones that stopped above it, and those that come up
+    for (L = (L == nl - 1 ? nl - 2 : L); L >= Ls; L--) {
+        const int nt = sv[L - Ls].nt;
+        if (tid >= nt) continue;
+        warps_sync(1 + L - Ls, nt);
+        pg_level_up<T, false>(tid, nt, sv[L - Ls], sv[L + 1 - Ls], L < deep, al, [&]() { return warps_sync(1 + L - Ls, nt); });
+    }
+}
+
+// one V(1,1) cycle x = M^-1 b on the level-0 vectors (bsel -> xsel; the first red values D b
+// already in x).  Levels 0 .. Lc-1: the whole grid, grid barriers; levels Lc .. Ls-1: the first
+// cluster alone, cluster barriers; levels Ls ..: block 0 in shared memory.
+template <class T>
+__device__ __noinline__ bool pg_vcycle(PS &s, const PArgs &a, PTab<T> &tb, int nl, int bsel, int xsel, int wsel) {
     const int Ls = a.Ls, Lc = (a.csz && !a.onecl) ? a.Lc : Ls;
     const T al = (T)a.alpha;
+    const int deep = a.sweeps2 ? a.deep : 0;
     set_lev0<T>(tb, bsel, xsel);
     auto gsync = [&]() { return pg_sync(s); };
+    auto lev = [&](int L) -> const SLev<T> & { return L ? tb.w.lev[L] : tb.cur0; };
+    auto wt = [&](int L) -> const T * { return (L == 0 && wsel) ? tb.w.w0 : nullptr; };
     for (int L = 0; L < Lc; L++)
-        if (!pg_level_down<T>(s, a, tb, L, wsel, gsync)) return false;
+        if (!pg_level_down<T>(s.tid, s.nth, lev(L), lev(L + 1), L < deep, wt(L), L + 1 < Ls, gsync)) return false;
     if ((int)blockIdx.x < (Lc < Ls ? a.csz : 1)) {         // the first cluster (or block 0 alone)
-        PS e = s;
-        const int rank = (int)blockIdx.x;                  // a 1-D grid: the first cluster is blocks 0 .. csz-1
-        e.tid = rank * blockDim.x + threadIdx.x;
-        e.nth = (Lc < Ls ? a.csz : 1) * blockDim.x;
+        const int tid = blockIdx.x * blockDim.x + threadIdx.x;   // a 1-D grid: the first cluster is blocks 0 .. csz-1
+        const int nth = (Lc < Ls ? a.csz : 1) * blockDim.x;
         auto csync = [&]() {
             if (Lc < Ls) cooperative_groups::this_cluster().sync();
             else __syncthreads();
             return true;
         };
-        for (int L = Lc; L < Ls; L++) pg_level_down<T>(e, a, tb, L, wsel, csync);
+        for (int L = Lc; L < Ls; L++)
+            pg_level_down<T>(tid, nth, lev(L), lev(L + 1), L < deep, wt(L), L + 1 < Ls, csync);
         if (blockIdx.x == 0) {
-            const LevView<T> &g = tb.lev[Ls];
-            blk_copy<T>(sv[0].b, g.b, g.N);
+            const SLev<T> &g = tb.w.lev[Ls];
+            const SLev<T> v = tb.sv[0];
+            const int n = 2 * v.H;
+            for (int q = threadIdx.x; q < n; q += blockDim.x) {
+                const T b = g.b[q];
+                v.b[q] = b;
+                if (!v.last && q < v.H) v.x[q] = v.D[q] * b;   // (the coarsest level's D is its inverse)
+            }
             __syncthreads();
-            blk_vcycle_small<T>(sv, Ls, nl, al);
-            blk_copy<T>(g.x, sv[0].x, g.N);
+            blk_cycle<T>(tb, Ls, nl, al, deep);
+            __syncthreads();
+            for (int q = threadIdx.x; q < n; q += blockDim.x) g.x[q] = v.x[q];
         }
         csync();
-        for (int L = Ls - 1; L >= Lc; L--) pg_level_up<T>(e, a, tb, L, csync);
+        for (int L = Ls - 1; L >= Lc; L--) pg_level_up<T, true>(tid, nth, lev(L), lev(L + 1), L < deep, al, csync);
     }
     if (!pg_sync(s)) return false;
     for (int L = Lc - 1; L >= 0; L--)
-        if (!pg_level_up<T>(s, a, tb, L, gsync)) return false;
+        if (!pg_level_up<T, true>(s.tid, s.nth, lev(L), lev(L + 1), L < deep, al, gsync)) return false;
     if (blockIdx.x == 0 && threadIdx.x == 0) s.g->vcycles++;
     return true;
 }
 
-// y = A x on level 0 at node k
+// ---------------------------------------------------------------- Krylov loops
+// y = A x on the black rows, x a preconditioner's result (its red rows give A x = b)
 template <class T>
-__device__ __forceinline__ T spmv_at(const LevView<T> &l0, const T *x, int k) {
-    const Node nd = unidx(k, l0.Nx, l0.Ny);
-    return lv_apply<T>(l0, x, k, nd.i, nd.j, nd.l);
+__device__ __forceinline__ Two<T> black_apply(const SLev<T> &v, const T *x, int t) {
+    const int row = fdiv(t, v.fr), l = fdiv(row, v.fy), j = row - l * v.Ny, m = 2 * t;
+    const Two<T> g = ld2(v.G + v.H + m), xk = ld2(x + v.H + m);
+    const Two<T> s = nb_sum<T>(v, 1, m, j, l, SrcX<T>{x});
+    return Two<T>{g.a * xk.a + s.a, g.b * xk.b + s.b};
 }
 
-// ---------------------------------------------------------------- Krylov loops
 // BiCGSTAB iterations (semiconductor_3d.c:2281-2316) on the records `sk` of precision T
-// while it is active; the reduction of rh.r for the next iteration rides on the x update.
+// while it is active, from r = rh = p with the first red values D p in ph (d holds
+// nothing yet: the first update writes it).  v and t exist on black slots only: on red rows
+// A ph = p and A sh = s.
 template <class T>
-__device__ bool pg_bicg(PS &s, const PArgs &a, PTab<T> &tb, const LevView<T> *sv, int nl, int N, KrylovS &sk) {
-    T *r = tb.vec[0], *rh = tb.vec[1], *p = tb.vec[2], *v = tb.vec[3];
-    T *ph = tb.vec[4], *sh = tb.vec[5], *t = tb.vec[6];
-    T *x = tb.sol;
-    const LevView<T> l0 = tb.lev[0];
-    bool have_rho = false;
-    double rho_next = 0.0;
+__device__ bool pg_bicg(PS &s, const PArgs &a, PTab<T> &tb, int nl, KrylovS &sk) {
+    T *r = tb.w.vec[0], *rh = tb.w.vec[1], *p = tb.w.vec[2], *v = tb.w.vec[3];
+    T *ph = tb.w.vec[4], *sh = tb.w.vec[5], *t = tb.w.vec[6], *d = tb.w.vec[7];
+    const int H = tb.w.lev[0].H, np = H >> 1;               // pairs of slots per colour
+    const T *Dr = tb.w.lev[0].D;
+    bool first = true;
     while (sk.active) {
-        double acc[2] = {0.0, 0.0}, a1[1] = {0.0};
-        if (have_rho) a1[0] = rho_next;
-        else {
-            for (int k = s.tid; k < N; k += s.nth) a1[0] += (double)rh[k] * (double)r[k];
-            if (!pg_sum<1>(s, a1)) return false;
-        }
+        double acc[3], a1[1], a2[2];
         if (threadIdx.x == 0) {
             if (sk.it >= sk.maxit) { sk.active = 0; sk.status = 3; }
             else {
                 sk.it++;
-                double rho1 = a1[0];
                 sk.pad0 = 0;
-                if (fabs(rho1) < 1e-300) {          // breakdown: restart the shadow residual
-                    rho1 = sk.rr;
-                    sk.rho = sk.al = sk.om = 1.0;
+                if (fabs(sk.rho1) < 1e-300) {               // breakdown: restart the shadow residual
+                    sk.rho1 = sk.rr;
                     sk.pad0 = 1;
-                    if (!(rho1 > 0.0)) { sk.active = 0; sk.status = 2; }
+                    if (!(sk.rho1 > 0.0)) { sk.active = 0; sk.status = 2; }
                 }
-                sk.rho1 = rho1;
-                sk.be = (rho1 / sk.rho) * (sk.al / sk.om);
             }
         }
         __syncthreads();
         if (!sk.active) break;
-        {
-            const T be = (T)sk.be, om = (T)sk.om;
-            const int restart = sk.pad0;
-            for (int k = s.tid; k < N; k += s.nth) {
-                if (restart) { rh[k] = r[k]; p[k] = r[k]; v[k] = 0; }
-                else p[k] = r[k] + be * (p[k] - om * v[k]);
+        if (sk.pad0) {
+            for (int q = s.tid; q < 2 * np; q += s.nth) {
+                const int m = 2 * q;
+                const Two<T> rk = ld2(r + m);
+                st2(rh + m, rk.a, rk.b);
+                st2(p + m, rk.a, rk.b);
+                if (m < H) { const Two<T> D = ld2(Dr + m); st2(ph + m, D.a * rk.a, D.b * rk.b); }
             }
+            PG_SYNC();
         }
-        PG_SYNC();
-        if (!pg_vcycle<T>(s, a, tb, sv, nl, 2, 4, 1)) return false;      // ph = M p
-        a1[0] = 0.0;
-        for (int k = s.tid; k < N; k += 2 * s.nth) {
-            const int k2 = k + s.nth;
-            const T q1 = spmv_at<T>(l0, ph, k);
-            const T q2 = k2 < N ? spmv_at<T>(l0, ph, k2) : T(0);
-            v[k] = q1;
-            a1[0] += (double)rh[k] * (double)q1;
-            if (k2 < N) { v[k2] = q2; a1[0] += (double)rh[k2] * (double)q2; }
+        if (!pg_vcycle<T>(s, a, tb, nl, 2, 4, 1)) return false;          // ph = M p
+        {
+            const SLev<T> l0 = tb.w.lev[0];
+            a1[0] = 0.0;
+            for (int q = s.tid; q < np; q += s.nth) {
+                const int m = 2 * q;
+                const Two<T> y = black_apply<T>(l0, ph, q), hb = ld2(rh + H + m), hr = ld2(rh + m), pr = ld2(p + m);
+                st2(v + H + m, y.a, y.b);
+                a1[0] += (double)hb.a * (double)y.a + (double)hb.b * (double)y.b + (double)hr.a * (double)pr.a +
+                         (double)hr.b * (double)pr.b;
+            }
         }
         if (!pg_sum<1>(s, a1)) return false;
         if (threadIdx.x == 0) {
@@ -442,216 +523,590 @@ __device__ bool pg_bicg(PS &s, const PArgs &a, PTab<T> &tb, const LevView<T> *sv
         __syncthreads();
         if (!sk.active) break;
         const T al = (T)sk.al;
-        a1[0] = 0.0;
-        for (int k = s.tid; k < N; k += s.nth) {
-            const T q = r[k] - al * v[k];
-            r[k] = q;
-            a1[0] += (double)q * (double)q;
+        a2[0] = a2[1] = 0.0;
+        for (int q = s.tid; q < 2 * np; q += s.nth) {       // s = r - al v; rh.s; D s
+            const int m = 2 * q;
+            const Two<T> rk = ld2(r + m), vk = ld2((m < H ? p : v) + m), h = ld2(rh + m);
+            const T x = rk.a - al * vk.a, y = rk.b - al * vk.b;
+            st2(r + m, x, y);
+            if (m < H) { const Two<T> D = ld2(Dr + m); st2(sh + m, D.a * x, D.b * y); }
+            a2[0] += (double)x * (double)x + (double)y * (double)y;
+            a2[1] += (double)h.a * (double)x + (double)h.b * (double)y;
         }
-        if (!pg_sum<1>(s, a1)) return false;
+        if (!pg_sum<2>(s, a2)) return false;
+        const double rhs_ = a2[1];
         if (threadIdx.x == 0) {
-            sk.ss = a1[0];
-            if (sqrt(a1[0]) <= sk.tgt) { sk.half = 1; sk.rr = a1[0]; }
+            sk.ss = a2[0];
+            if (sqrt(a2[0]) <= sk.tgt) { sk.half = 1; sk.rr = a2[0]; }
         }
         __syncthreads();
-        if (sk.half) {                                // half-step exit: x += al ph
-            for (int k = s.tid; k < N; k += s.nth) x[k] += al * ph[k];
+        if (sk.half) {                                      // half-step exit: d += al ph
+            for (int q = s.tid; q < 2 * np; q += s.nth) {
+                const int m = 2 * q;
+                const Two<T> x = ld2(ph + m);
+                Two<T> y{0, 0};
+                if (!first) y = ld2(d + m);
+                st2(d + m, y.a + al * x.a, y.b + al * x.b);
+            }
             if (threadIdx.x == 0) { sk.active = 0; sk.status = 1; }
             PG_SYNC();
-            break;
+            return true;
         }
-        if (!pg_vcycle<T>(s, a, tb, sv, nl, 0, 5, 1)) return false;      // sh = M r
-        acc[0] = acc[1] = 0.0;
-        for (int k = s.tid; k < N; k += 2 * s.nth) {
-            const int k2 = k + s.nth;
-            const T q1 = spmv_at<T>(l0, sh, k);
-            const T q2 = k2 < N ? spmv_at<T>(l0, sh, k2) : T(0);
-            t[k] = q1;
-            acc[0] += (double)q1 * (double)q1;
-            acc[1] += (double)q1 * (double)r[k];
-            if (k2 < N) {
-                t[k2] = q2;
-                acc[0] += (double)q2 * (double)q2;
-                acc[1] += (double)q2 * (double)r[k2];
+        if (!pg_vcycle<T>(s, a, tb, nl, 0, 5, 1)) return false;          // sh = M s
+        {
+            const SLev<T> l0 = tb.w.lev[0];
+            acc[0] = acc[1] = acc[2] = 0.0;
+            for (int q = s.tid; q < np; q += s.nth) {
+                const int m = 2 * q;
+                const Two<T> y = black_apply<T>(l0, sh, q), rb = ld2(r + H + m), rr = ld2(r + m);
+                const Two<T> hb = ld2(rh + H + m), hr = ld2(rh + m);
+                st2(t + H + m, y.a, y.b);
+                const double rs = (double)rr.a * (double)rr.a + (double)rr.b * (double)rr.b;
+                acc[0] += (double)y.a * (double)y.a + (double)y.b * (double)y.b + rs;
+                acc[1] += (double)y.a * (double)rb.a + (double)y.b * (double)rb.b + rs;
+                acc[2] += (double)hb.a * (double)y.a + (double)hb.b * (double)y.b + (double)hr.a * (double)rr.a +
+                          (double)hr.b * (double)rr.b;
             }
         }
-        if (!pg_sum<2>(s, acc)) return false;
+        if (!pg_sum<3>(s, acc)) return false;
         if (threadIdx.x == 0) {
             sk.tt = acc[0]; sk.ts = acc[1];
             sk.om = acc[0] > 0.0 ? acc[1] / acc[0] : 0.0;
+            const double rho = rhs_ - sk.om * acc[2];        // rh . (s - om t)
+            sk.be = sk.om != 0.0 ? (rho / sk.rho1) * (sk.al / sk.om) : 0.0;
+            sk.rho1 = rho;
         }
         __syncthreads();
+        a1[0] = 0.0;
         {
-            const T om = (T)sk.om;
-            acc[0] = acc[1] = 0.0;
-            for (int k = s.tid; k < N; k += s.nth) {
-                x[k] += al * ph[k] + om * sh[k];
-                const T q = r[k] - om * t[k];
-                r[k] = q;
-                acc[0] += (double)q * (double)q;
-                acc[1] += (double)rh[k] * (double)q;
+            const T om = (T)sk.om, be = (T)sk.be;
+            for (int q = s.tid; q < 2 * np; q += s.nth) {
+                const int m = 2 * q;
+                const bool red = m < H;
+                const Two<T> rk = ld2(r + m), pk = ld2(p + m), x = ld2(ph + m), z = ld2(sh + m);
+                const Two<T> vk = red ? pk : ld2(v + m), tk = red ? rk : ld2(t + m);
+                Two<T> y{0, 0};
+                if (!first) y = ld2(d + m);
+                st2(d + m, y.a + (al * x.a + om * z.a), y.b + (al * x.b + om * z.b));
+                const T ra = rk.a - om * tk.a, rb = rk.b - om * tk.b;
+                const T pa = ra + be * (pk.a - om * vk.a), pb = rb + be * (pk.b - om * vk.b);
+                st2(r + m, ra, rb);
+                st2(p + m, pa, pb);
+                if (red) { const Two<T> D = ld2(Dr + m); st2(ph + m, D.a * pa, D.b * pb); }
+                a1[0] += (double)ra * (double)ra + (double)rb * (double)rb;
             }
         }
-        if (!pg_sum<2>(s, acc)) return false;
+        first = false;
+        if (!pg_sum<1>(s, a1)) return false;
         if (threadIdx.x == 0) {
-            sk.rr = acc[0];
-            const double rn = sqrt(acc[0]);
+            sk.rr = a1[0];
+            const double rn = sqrt(a1[0]);
             if (rn <= sk.tgt || sk.om == 0.0) { sk.active = 0; sk.status = 1; }
             else {
                 if (rn < 0.99 * sk.rbest) { sk.rbest = rn; sk.stall = 0; }
                 else if (++sk.stall > 40) { sk.active = 0; sk.status = 2; }
-                if (sk.active) sk.rho = sk.rho1;
             }
         }
-        have_rho = true;
-        rho_next = acc[1];
         __syncthreads();
+    }
+    if (first) {                                            // nothing was added: d = 0
+        for (int q = s.tid; q < 2 * np; q += s.nth) st2(d + 2 * q, T(0), T(0));
+        PG_SYNC();
     }
     return true;
 }
 
-// PCG iterations (semiconductor_3d.c:2194-2206) on the records `sk` while active
+// PCG iterations (semiconductor_3d.c:2194-2206) from r with the first red values D r in z:
+// one reduction per iteration for rz = r.z and z.A z, the step length from
+// p.A p = z.A z - be^2 (p.A p of the last iteration) and A p by the recurrence A z + be A p.
 template <class T>
-__device__ bool pg_pcg(PS &s, const PArgs &a, PTab<T> &tb, const LevView<T> *sv, int nl, int N, KrylovS &sk) {
-    T *r = tb.vec[0], *z = tb.vec[1], *p = tb.vec[2], *q = tb.vec[3];
-    T *x = tb.sol;
-    const LevView<T> l0 = tb.lev[0];
-    while (sk.active) {
-        double acc[1] = {0.0};
-        for (int k = s.tid; k < N; k += 2 * s.nth) {
-            const int k2 = k + s.nth;
-            const T q1 = spmv_at<T>(l0, p, k);
-            const T q2 = k2 < N ? spmv_at<T>(l0, p, k2) : T(0);
-            q[k] = q1;
-            acc[0] += (double)p[k] * (double)q1;
-            if (k2 < N) { q[k2] = q2; acc[0] += (double)p[k2] * (double)q2; }
-        }
-        if (!pg_sum<1>(s, acc)) return false;
-        if (threadIdx.x == 0) {
-            sk.it++;
-            const double pq = acc[0];
-            if (!(pq > 0.0)) { sk.active = 0; sk.status = 2; sk.al = 0.0; }
-            else sk.al = sk.rz / pq;
-        }
-        __syncthreads();
-        if (!sk.active) break;
+__device__ bool pg_pcg(PS &s, const PArgs &a, PTab<T> &tb, int nl, KrylovS &sk) {
+    T *r = tb.w.vec[0], *z = tb.w.vec[1], *p = tb.w.vec[2], *q = tb.w.vec[3], *w = tb.w.vec[4], *d = tb.w.vec[7];
+    const int H = tb.w.lev[0].H, np = H >> 1;
+    const T *Dr = tb.w.lev[0].D;
+    bool first = true;
+    for (;;) {
+        if (!pg_vcycle<T>(s, a, tb, nl, 0, 1, 0)) return false;          // z = M r
+        double acc[2] = {0.0, 0.0};
         {
-            const T al = (T)sk.al;
-            for (int k = s.tid; k < N; k += s.nth) { x[k] += al * p[k]; r[k] -= al * q[k]; }
+            const SLev<T> l0 = tb.w.lev[0];
+            for (int u = s.tid; u < np; u += s.nth) {       // on red rows A z = r
+                const int m = 2 * u;
+                const Two<T> y = black_apply<T>(l0, z, u), zb = ld2(z + H + m), zr = ld2(z + m), rb = ld2(r + H + m),
+                             rr = ld2(r + m);
+                st2(w + H + m, y.a, y.b);
+                const double red = (double)rr.a * (double)zr.a + (double)rr.b * (double)zr.b;
+                acc[0] += (double)rb.a * (double)zb.a + (double)rb.b * (double)zb.b + red;
+                acc[1] += (double)zb.a * (double)y.a + (double)zb.b * (double)y.b + red;
+            }
         }
-        PG_SYNC();
-        if (!pg_vcycle<T>(s, a, tb, sv, nl, 0, 1, 0)) return false;      // z = M r
-        acc[0] = 0.0;
-        for (int k = s.tid; k < N; k += s.nth) acc[0] += (double)r[k] * (double)z[k];
-        if (!pg_sum<1>(s, acc)) return false;
+        if (!pg_sum<2>(s, acc)) return false;
         if (threadIdx.x == 0) {
             const double rz = acc[0];
-            if (!(rz > sk.rtol * sk.rtol * sk.rz0)) { sk.active = 0; sk.status = 1; }
+            sk.be = 0.0;
+            if (first) {
+                sk.rz0 = rz;
+                sk.it = 0;
+                sk.status = rz > 0.0 ? 0 : 2;
+                sk.active = rz > 0.0;
+                sk.pq = acc[1];
+            } else if (!(rz > sk.rtol * sk.rtol * sk.rz0)) { sk.active = 0; sk.status = 1; }
             else if (sk.it >= sk.maxit) { sk.active = 0; sk.status = 3; }
-            else { sk.be = rz / sk.rz; sk.rz = rz; }
+            else {
+                sk.be = rz / sk.rz;
+                sk.pq = acc[1] - sk.be * sk.be * sk.pq;
+            }
+            if (sk.active) {
+                sk.rz = rz;
+                sk.it++;
+                if (!(sk.pq > 0.0)) { sk.active = 0; sk.status = 2; sk.al = 0.0; }
+                else sk.al = rz / sk.pq;
+            }
         }
         __syncthreads();
         if (!sk.active) break;
-        {
-            const T be = (T)sk.be;
-            for (int k = s.tid; k < N; k += s.nth) p[k] = z[k] + be * p[k];
+        const T al = (T)sk.al, be = (T)sk.be;
+        for (int u = s.tid; u < 2 * np; u += s.nth) {
+            const int m = 2 * u;
+            const bool red = m < H;
+            const Two<T> zk = ld2(z + m), rk = ld2(r + m), wk = red ? rk : ld2(w + m);
+            Two<T> pk = zk, qk = wk, y{0, 0};
+            if (!first) {
+                const Two<T> po = ld2(p + m), qo = ld2(q + m);
+                pk = Two<T>{zk.a + be * po.a, zk.b + be * po.b};
+                qk = Two<T>{wk.a + be * qo.a, wk.b + be * qo.b};
+                y = ld2(d + m);
+            }
+            st2(p + m, pk.a, pk.b);
+            st2(q + m, qk.a, qk.b);
+            st2(d + m, y.a + al * pk.a, y.b + al * pk.b);
+            const T ra = rk.a - al * qk.a, rb = rk.b - al * qk.b;
+            st2(r + m, ra, rb);
+            if (red) { const Two<T> D = ld2(Dr + m); st2(z + m, D.a * ra, D.b * rb); }
         }
+        first = false;
+        PG_SYNC();
+    }
+    if (first) {
+        for (int u = s.tid; u < 2 * np; u += s.nth) st2(d + 2 * u, T(0), T(0));
         PG_SYNC();
     }
     return true;
 }
 
-// (A x)_k of the FP64 level-0 operator and, in fl, sum_j |a_kj x_j|
-template <class X>
-__device__ __forceinline__ double a64_at(const double *A, int ap, const X *x, int k, int i, int j, int l, int Nx,
-                                         int Ny, int Nz, double *fl) {
+// ---------------------------------------------------------------- set-up
+// nodes (2t, j, l) and (2t + 1, j, l) of slot u = t + hx row: both colours of one slot
+struct Pair { int t, j, l, row; };
+template <class T>
+__device__ __forceinline__ Pair slot_row(const SLev<T> &v, int u) {
+    Pair p;
+    p.row = fdiv(u >> 1, v.fr);
+    p.t = u - p.row * v.hx;
+    p.l = fdiv(p.row, v.fy);
+    p.j = p.row - p.l * v.Ny;
+    return p;
+}
+// sum_j a_kj x_j of the natural-order FP64 row k and, in fl, sum_j |a_kj x_j|; a[] keeps the row
+// Couplings that leave the domain are taken as zero and their neighbour is the node itself, so
+// every load is unconditional (loads behind branches are waited for one by one)
+template <class F>
+__device__ __forceinline__ double row64(const double *A, int ap, int k, int i, int j, int l, int Nx, int Ny, int Nz,
+                                        double (&a)[7], F x, double &fl) {
     const int NxNy = Nx * Ny;
-    double t = A[k] * (double)x[k], sum = t, f = fabs(t);
-    if (i > 0) { t = A[ap + k] * (double)x[k - 1]; sum += t; f += fabs(t); }
-    if (i < Nx - 1) { t = A[2 * ap + k] * (double)x[k + 1]; sum += t; f += fabs(t); }
-    if (j > 0) { t = A[3 * ap + k] * (double)x[k - Nx]; sum += t; f += fabs(t); }
-    if (j < Ny - 1) { t = A[4 * ap + k] * (double)x[k + Nx]; sum += t; f += fabs(t); }
-    if (l > 0) { t = A[5 * ap + k] * (double)x[k - NxNy]; sum += t; f += fabs(t); }
-    if (l < Nz - 1) { t = A[6 * ap + k] * (double)x[k + NxNy]; sum += t; f += fabs(t); }
-    if (fl) *fl = f;
+    const bool e[6] = {i > 0, i < Nx - 1, j > 0, j < Ny - 1, l > 0, l < Nz - 1};
+    double y[7];
+#pragma unroll
+    for (int q = 0; q < 7; q++) a[q] = A[q * ap + k];
+    y[0] = x(k, i, j, l);
+    y[1] = x(e[0] ? k - 1 : k, e[0] ? i - 1 : i, j, l);
+    y[2] = x(e[1] ? k + 1 : k, e[1] ? i + 1 : i, j, l);
+    y[3] = x(e[2] ? k - Nx : k, i, e[2] ? j - 1 : j, l);
+    y[4] = x(e[3] ? k + Nx : k, i, e[3] ? j + 1 : j, l);
+    y[5] = x(e[4] ? k - NxNy : k, i, j, e[4] ? l - 1 : l);
+    y[6] = x(e[5] ? k + NxNy : k, i, j, e[5] ? l + 1 : l);
+    double t = a[0] * y[0], sum = t;
+    fl = fabs(t);
+#pragma unroll
+    for (int q = 1; q < 7; q++) {
+        if (!e[q - 1]) a[q] = 0.0;
+        t = a[q] * y[q];
+        sum += t;
+        fl += fabs(t);
+    }
     return sum;
 }
-
-// r = b - A x with the FP64 operator, its squared norm and the squared rounding floor
-// (sum_k (sum_j |a_kj x_j| + |b_k|)^2) - the start of the FP64 BiCGSTAB and of the
-// refinement (semiconductor_3d.c:2244-2268).  Writes r (FP64 work vector 0) and, when
-// r32 is not null, its FP32 copy; with rh, also rh = r and p = v = 0.
-template <class T>
-__device__ __forceinline__ void pg_start64(const DevP &P, const PTab<T> &tb, const PS &s, float *r32, bool bicg,
-                                           double (&acc)[2]) {
-    const double *b = P.rhs, *x = P.sol;
-    double *r = P.wk[0], *rh = P.wk[1], *p = P.wk[2], *v = P.wk[3];
-    const int Nx = P.Nx, Ny = P.Ny, Nz = P.Nz, N = P.N;
-    for (int k = s.tid; k < N; k += s.nth) {
-        const Node a = unidx(k, Nx, Ny);
-        double fl;
-        const double sum = a64_at<double>(tb.A64, tb.ap64, x, k, a.i, a.j, a.l, Nx, Ny, Nz, &fl);
-        fl += fabs(b[k]);
-        const double rk = b[k] - sum;
-        r[k] = rk;
-        if (bicg) { rh[k] = rk; p[k] = 0.0; v[k] = 0.0; }
-        if (r32) r32[k] = (float)rk;
-        acc[0] += rk * rk;
-        acc[1] += fl * fl;
+// The level-0 system of the launch: r = b - A x with the FP64 operator (its squared norm and
+// the squared rounding floor sum_k (sum_j |a_kj x_j| + |b_k|)^2 in acc,
+// semiconductor_3d.c:2244-2268), and the colour-ordered copy of the operator, the row weights
+// and r (rh = p = r) in precision T; padding slots are zeroed.  FP32 PCG starts from x = 0.
+template <class T, int KIND>
+__device__ __forceinline__ void pg_load(const DevP &P, const PTab<T> &tb, const PS &s, double (&acc)[2]) {
+    const SLev<T> v = tb.w.lev[0];
+    constexpr bool zero_x = KIND == PK_PCG && std::is_same<T, float>::value;
+    const double *x = P.sol;
+    for (int u = s.tid; u < v.H; u += s.nth) {
+        const Pair p = slot_row(v, u);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int i = 2 * p.t + q, m = (((i + p.j + p.l) & 1) ? v.H : 0) + u;
+            double a[7] = {0, 0, 0, 0, 0, 0, 0}, rk = 0.0, w = 0.0;
+            if (i < v.Nx) {
+                const int k = i + v.Nx * p.row;
+                double fl;
+                const double b = P.rhs[k];
+                const double sum = row64(tb.A64, tb.ap64, k, i, p.j, p.l, v.Nx, v.Ny, v.Nz, a,
+                                         [&](int kk, int, int, int) { return zero_x ? 0.0 : x[kk]; }, fl);
+                fl += fabs(b);
+                rk = b - sum;
+                acc[0] += rk * rk;
+                acc[1] += fl * fl;
+                if (KIND == PK_REFINED) P.wk[0][k] = rk;
+                if (KIND != PK_PCG) w = P.dsc[k];
+            }
+            const T g = (T)a[0];
+            v.G[m] = g;
+            if (!((i + p.j + p.l) & 1) && i < v.Nx) v.D[m] = g != T(0) ? T(1) / g : T(1);   // red pivot
+#pragma unroll
+            for (int e = 0; e < 6; e++) v.A[e * v.ap + m] = (T)a[1 + e];
+            tb.w.vec[0][m] = (T)rk;
+            if (KIND != PK_PCG) {
+                tb.w.vec[1][m] = (T)rk;
+                tb.w.vec[2][m] = (T)rk;
+                tb.w.w0[m] = (T)w;
+            }
+            if (i >= v.Nx) { v.pw[m] = 0; v.D[m] = 0; }
+        }
     }
 }
-
-// ---------------------------------------------------------------- hierarchy set-up
-// The multigrid set-up of the system now in the level-0 operator (mg_setup_t in
-// kernels_la.cu, the reference's mg_setup semiconductor_3d.c:2126-2148): for T = float
-// the FP32 copy of the operator and row weights, then per level the Slotboom weights with
-// the next level's reference potentials and the smoother pivots (one pass: the pivots
-// read only the level's own operator), the Galerkin coarse operator (one pass), and the
-// coarsest level's dense inverse (block 0, in its shared memory).
+// reciprocal red-black D-ILU pivots of the black slots, a_kk - sum a_kr a_rk / a_rr, guarded
+// as the reference guards its ILU pivots (semiconductor_3d.c:1937-1938); the red ones, 1 / a_rr,
+// are written with the operator
 template <class T>
-__device__ __noinline__ bool pg_setup(const DevP &P, PS &s, const PArgs &a, const PTab<T> &tb, unsigned char *scratch) {
-    const int nl = P.nlev, qsign = a.qsign;
-    if constexpr (std::is_same<T, float>::value) {
-        float *A32 = const_cast<float *>(tb.lev[0].A);
-        const int ap = tb.lev[0].ap;
-        for (int k = s.tid; k < P.N; k += s.nth) {
+__device__ __forceinline__ void pg_pivots(const SLev<T> &vr, int tid, int nth) {
+    const SLev<T> v = vr;
+    for (int u = tid; u < v.H; u += nth) {
+        const Pair p = slot_row(v, u);
+        const int o = (p.j + p.l + 1) & 1, i = 2 * p.t + o, m = v.H + u;
+        const bool ok[6] = {i > 0, i < v.Nx - 1, p.j > 0, p.j < v.Ny - 1, p.l > 0, p.l < v.Nz - 1};
+        const int nbr[6] = {u - 1 + o, u + o, u - v.hx, u + v.hx, u - v.sz, u + v.sz};
+        const T *A = v.A + m, *R = v.A;
+        const T g = v.G[m];
+        T sum = 0;
 #pragma unroll
-            for (int q = 0; q < 7; q++) A32[q * ap + k] = (float)tb.A64[q * tb.ap64 + k];
-            if (qsign) P.dsc32[k] = (float)P.dsc[k];
+        for (int e = 0; e < 6; e++) {
+            const int n = ok[e] ? nbr[e] : u;
+            const T c = A[e * v.ap] * R[(e ^ 1) * v.ap + n] * v.D[n];
+            sum += ok[e] ? c : T(0);
         }
+        T d = g - sum;
+        if (!(d > T(1e-8) * fabs(g))) d = g;
+        if (!(d != T(0))) d = 1;
+        v.D[m] = i < v.Nx ? T(1) / d : T(0);
+    }
+}
+// Slotboom weights of the level's nodes towards the next one, and that level's reference
+// potentials (semiconductor_3d.c:2092-2117); thread per coarse node.  phf / phc: the levels'
+// reference potentials in natural order (phf null: level 0, from the state)
+template <class T>
+__device__ __forceinline__ void pg_weights(const DevP &P, const SLev<T> &f, const SLev<T> &cl, const double *phf,
+                                           double *phc, int qsign, int tid, int nth) {
+    for (int K = tid; K < cl.N; K += nth) {
+        const Node c = unidx(K, cl.Nx, cl.Ny);
+        const Agg g = agg_range(f, c.i, c.j, c.l);
+        double p[8], mx = PH_NONE;
+        if (qsign) {
+#pragma unroll
+            for (int q = 0; q < 8; q++) {                   // (an aggregate cut short repeats its last nodes)
+                const int k = min(g.i0 + (q & 1), g.i1) +
+                              f.Nx * (min(g.j0 + ((q >> 1) & 1), g.j1) + f.Ny * min(g.l0 + (q >> 2), g.l1));
+                p[q] = phf ? phf[k] : ph0(P, k, qsign);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) mx = fmax(mx, p[q]);
+            phc[K] = mx;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            T wt = 1;
+            if (qsign) {
+                const double e = (p[q] <= 0.5 * PH_NONE) ? -800.0 : p[q] - mx;
+                wt = (T)(e < -700.0 ? 0.0 : exp(e));
+            }
+            f.pw[sslot(f, min(g.i0 + (q & 1), g.i1), min(g.j0 + ((q >> 1) & 1), g.j1), min(g.l0 + (q >> 2), g.l1))] = wt;
+        }
+    }
+}
+// Petrov-Galerkin coarse operator P^T W A P (semiconductor_3d.c:2003-2027), summed in FP64:
+// lanes as in pg_restrict, each lane the two nodes of one of the aggregate's rows
+template <class T>
+__device__ __forceinline__ void pg_galerkin(const SLev<T> &fr, const SLev<T> &clr, const T *w, int tid, int nth) {
+    const SLev<T> f = fr, cl = clr;
+    const int lane = tid & 31, sub = lane >> 3, dj = sub & 1, dl = sub >> 1;
+    const int ng = cl.n8 * cl.Ny * cl.Nz, nw = nth >> 5;
+    for (int g = tid >> 5; g < ng; g += nw) {
+        const int row = fdiv(g, cl.f8), K = fdiv(row, cl.fy), J = row - K * cl.Ny;
+        const int I = 8 * (g - row * cl.n8) + (lane & 7);
+        const int j = f.cy ? 2 * J + dj : J, l = f.cz ? 2 * K + dl : K;
+        const bool ok = I < cl.Nx && j < f.Ny && l < f.Nz && (f.cy || !dj) && (f.cz || !dl);
+        double a[7] = {0, 0, 0, 0, 0, 0, 0};
+        if (ok) {
+            const int i0 = f.cx ? 2 * I : I, i1 = f.cx ? min(2 * I + 1, f.Nx - 1) : I;
+            const int j0 = f.cy ? 2 * J : J, j1 = f.cy ? min(2 * J + 1, f.Ny - 1) : J;
+            const int l0 = f.cz ? 2 * K : K, l1 = f.cz ? min(2 * K + 1, f.Nz - 1) : K;
+            const bool ej0 = j > 0, ej1 = j < f.Ny - 1, el0 = l > 0, el1 = l < f.Nz - 1;
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int i = i0 + q;
+                const bool in = i <= i1;
+                const int ii = in ? i : i0, m = sslot(f, ii, j, l);
+                const T *A = f.A + m;
+                const double wk = in ? (w ? (double)w[m] : 1.0) : 0.0;
+                // (a coupling that leaves the domain is zero: any weight will do)
+                const T g0 = f.G[m], p0 = f.pw[m];
+                const T am[6] = {A[0], A[f.ap], A[2 * f.ap], A[3 * f.ap], A[4 * f.ap], A[5 * f.ap]};
+                const T pn[6] = {f.pw[sslot(f, max(ii - 1, 0), j, l)], f.pw[sslot(f, min(ii + 1, f.Nx - 1), j, l)],
+                                 f.pw[sslot(f, ii, ej0 ? j - 1 : j, l)], f.pw[sslot(f, ii, ej1 ? j + 1 : j, l)],
+                                 f.pw[sslot(f, ii, j, el0 ? l - 1 : l)], f.pw[sslot(f, ii, j, el1 ? l + 1 : l)]};
+                const bool inner[6] = {ii - 1 >= i0, ii + 1 <= i1, j - 1 >= j0, j + 1 <= j1, l - 1 >= l0, l + 1 <= l1};
+                a[0] += wk * (double)g0 * (double)p0;
+#pragma unroll
+                for (int e = 0; e < 6; e++) {
+                    const double c = wk * (double)am[e] * (double)pn[e];
+                    a[0] += inner[e] ? c : 0.0;
+                    a[1 + e] += inner[e] ? 0.0 : c;
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 7; q++) {
+            a[q] += __shfl_xor_sync(0xffffffffu, a[q], 8);
+            a[q] += __shfl_xor_sync(0xffffffffu, a[q], 16);
+        }
+        if (sub == 0 && I < 2 * cl.hx) {                    // (padding slots: zeros, a[] is zero there)
+            const int q = sslot(cl, I, J, K);
+            if (I >= cl.Nx) {
+                if (!cl.last) cl.pw[q] = 0;
+                cl.x[q] = 0;
+                cl.b[q] = 0;
+            } else if (a[0] == 0. && a[1] == 0. && a[2] == 0. && a[3] == 0. && a[4] == 0. && a[5] == 0. && a[6] == 0.) a[0] = 1.;
+            const T g = (T)a[0];
+            cl.G[q] = g;
+            if (!cl.last && !((I + J + K) & 1))              // red pivot (0 in a padding slot)
+                cl.D[q] = I >= cl.Nx ? T(0) : (g != T(0) ? T(1) / g : T(1));
+#pragma unroll
+            for (int e = 0; e < 6; e++) cl.A[e * cl.ap + q] = (T)a[1 + e];
+        }
+    }
+}
+// Dense inverse of the coarsest level (n <= 64) by Gauss-Jordan with partial pivoting in FP64
+// (tiny pivots guarded as semiconductor_3d.c:2066 does), by the first 8 n threads: 8 lanes
+// hold a row in registers, rows are never moved (row piv[c] plays row c), and per column the
+// lanes exchange the column and the pivot row through shared memory (two barriers of those
+// warps).  For 24 unknowns 19 us, a matrix in shared memory with row swaps 29 us, a thread per
+// row with a serial pivot search 50 us.
+template <class T>
+__device__ __noinline__ void blk_invert(const SLev<T> &v) {
+    __shared__ double col[2][COARSE_MAX], prow[2][COARSE_MAX];
+    __shared__ int piv[COARSE_MAX];
+    const int n = v.N, nt = (8 * n + 31) & ~31, tid = threadIdx.x, lane = tid & 31, r = tid >> 3, q0 = tid & 7;
+    if (tid < nt) {
+        double a[8];
+        const bool row = r < n;
+        {
+            const Node c = unidx(row ? r : 0, v.Nx, v.Ny);
+            const int m = sslot(v, c.i, c.j, c.l);
+            const T *A = v.A + m;
+            const T g = v.G[m], e[6] = {A[0], A[v.ap], A[2 * v.ap], A[3 * v.ap], A[4 * v.ap], A[5 * v.ap]};
+            const int NxNy = v.Nx * v.Ny;
+            const bool ok[6] = {c.i > 0, c.i < v.Nx - 1, c.j > 0, c.j < v.Ny - 1, c.l > 0, c.l < v.Nz - 1};
+            const int at[6] = {r - 1, r + 1, r - v.Nx, r + v.Nx, r - NxNy, r + NxNy};
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int q = q0 + 8 * i;
+                double x = q == r ? (double)g : 0.0;
+#pragma unroll
+                for (int w = 0; w < 6; w++)
+                    if (ok[w] && q == at[w]) x = (double)e[w];   // (a dimension of 1 or 2 nodes: one neighbour each)
+                a[i] = x;
+            }
+        }
+        unsigned long long used = 0;
+        int mine = 0;                                        // the column this row was the pivot of
+        for (int c = 0; c < n; c++) {
+            double *cc = col[c & 1], *pr = prow[c & 1];
+            if (row && q0 == (c & 7)) {
+                double x = 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) x = i == (c >> 3) ? a[i] : x;
+                cc[r] = x;
+            }
+            warps_sync(1, nt);
+            unsigned key = 0;                                // |a| to 17 bits, ties to the lower row
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int rr = lane + 32 * h;
+                if (rr < n && !((used >> rr) & 1)) {
+                    const unsigned hi = (unsigned)__double2hiint(cc[rr]) & 0x7fffffffu;
+                    const unsigned k = ((hi >> 5) << 6) | (unsigned)(63 - rr);
+                    key = k > key ? k : key;
+                }
+            }
+            const int p = 63 - (int)(__reduce_max_sync(0xffffffffu, key) & 63u);
+            used |= 1ull << p;
+            const double d = cc[p], inv = 1.0 / (fabs(d) > 1e-300 ? d : 1e-300);
+            if (r == p) {
+                mine = c;
+                if (q0 == 0) piv[c] = p;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int q = q0 + 8 * i;
+                    a[i] = (q == c ? 1.0 : a[i]) * inv;
+                    if (q < n) pr[q] = a[i];
+                }
+            }
+            warps_sync(1, nt);
+            if (row && r != p) {
+                const double f = cc[r];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int q = q0 + 8 * i;
+                    if (q < n) a[i] = (q == c ? 0.0 : a[i]) - f * pr[q];
+                }
+            }
+        }
+        if (row)
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int q = q0 + 8 * i;
+                if (q < n) v.D[mine * n + piv[q]] = (T)a[i];
+            }
+    }
+    __syncthreads();
+}
+// bytes of block 0's shared memory: a level's arrays, and the coarsest level's inverse with
+// its scratch
+template <class T>
+__host__ __device__ inline size_t ssm_level(int H, int ap, int n, bool last) {
+    if (last)
+        return al16((size_t)6 * ap * sizeof(T)) + 3 * al16((size_t)2 * H * sizeof(T)) + al16((size_t)n * n * sizeof(T));
+    return al16((size_t)6 * ap * sizeof(T)) + 5 * al16((size_t)2 * H * sizeof(T));
+}
+// views of the levels Ls .. nl-1 in block 0's shared memory (thread 0)
+template <class T>
+__device__ void ssm_views(PTab<T> &tb, int Ls, int nl, unsigned char *base) {
+    for (int L = Ls; L < nl; L++) {
+        SLev<T> v = tb.w.lev[L];
+        const size_t nb = al16((size_t)2 * v.H * sizeof(T));
+        unsigned char *p = base;
+        v.A = reinterpret_cast<T *>(p); p += al16((size_t)6 * v.ap * sizeof(T));
+        v.G = reinterpret_cast<T *>(p); p += nb;
+        v.D = reinterpret_cast<T *>(p); p += v.last ? al16((size_t)v.N * v.N * sizeof(T)) : nb;
+        if (!v.last) { v.pw = reinterpret_cast<T *>(p); p += nb; }
+        v.x = reinterpret_cast<T *>(p); p += nb;
+        v.b = reinterpret_cast<T *>(p);
+        tb.sv[L - Ls] = v;
+        base += ssm_level<T>(v.H, v.ap, v.N, v.last);
+    }
+    // threads of a level: a pair of slots each, a warp per 8 coarse nodes of its restriction, 8
+    // lanes per row of the dense inverse, and no fewer than the level below
+    int ntc = 0;
+    for (int L = nl - 1; L >= Ls; L--) {
+        SLev<T> &v = tb.sv[L - Ls];
+        int nt = v.last ? 8 * v.N : v.H >> 1;
+        if (!v.last) {
+            const SLev<T> &c = tb.sv[L + 1 - Ls];
+            nt = max(max(nt, 32 * c.n8 * c.Ny * c.Nz), ntc);
+        }
+        ntc = v.nt = min((nt + 31) & ~31, (int)blockDim.x);
+    }
+}
+// The multigrid set-up of the system loaded by pg_load (the reference's mg_setup,
+// semiconductor_3d.c:2126-2148): one grid pass per large level - its pivots, the Galerkin
+// operator of the next level and that level's weights - and the small levels in block 0's
+// shared memory.  `xr` takes the first red values D r of the solve.
+template <class T>
+__device__ __noinline__ bool pg_setup(const DevP &P, PS &s, const PArgs &a, PTab<T> &tb, int nl, T *xr,
+                                      unsigned char *smem) {
+    const int Ls = a.Ls, qsign = a.qsign;
+    for (int L = 0; L < Ls; L++) {
+        const SLev<T> &f = tb.w.lev[L], &cl = tb.w.lev[L + 1];
+        pg_galerkin<T>(f, cl, (L == 0 && qsign) ? tb.w.w0 : nullptr, s.tid, s.nth);
+        pg_pivots<T>(f, s.tid, s.nth);
+        if (L == 0)
+            for (int u = s.tid; u < f.H; u += s.nth) xr[u] = f.D[u] * tb.w.vec[0][u];
+        if (L + 1 < Ls) pg_weights<T>(P, cl, tb.w.lev[L + 2], PT<T>::lev(P, L + 1).ph, PT<T>::lev(P, L + 2).ph, qsign, s.tid, s.nth);
         PG_SYNC();
     }
-    for (int L = 0; L < nl - 1; L++) {
-        const LevView<T> &f = tb.lev[L];
-        const LevelT<T> &cl = PT<T>::lev(P, L + 1);
-        for (int K = s.tid; K < cl.N; K += s.nth) mg_weights_node<T>(P, f, cl, L, qsign, K);
-        for (int k = s.tid; k < f.N; k += s.nth) ilu_diag_node<T>(f, k);
-        PG_SYNC();
-        const T *w = (L == 0 && qsign) ? tb.w0 : nullptr;
-        for (int K = s.tid; K < cl.N; K += s.nth) galerkin_node<T>(f, cl, w, K);
-        PG_SYNC();
-    }
-    if (blockIdx.x == 0 && nl > 1) {
-        double *M = reinterpret_cast<double *>(scratch);
-        int *perm = reinterpret_cast<int *>(M + COARSE_MAX * (COARSE_MAX + 1));
-        blk_coarse_setup<T>(PT<T>::lev(P, nl - 1), M, perm, perm + COARSE_MAX);
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) ssm_views<T>(tb, Ls, nl, smem);
         __syncthreads();
+        const int tid = threadIdx.x, nth = blockDim.x;
+        {
+            const SLev<T> &g = tb.w.lev[Ls];
+            const SLev<T> v = tb.sv[0];
+            for (int q = tid; q < 2 * v.H; q += nth) {
+                const int u = q < v.H ? q : q - v.H;
+                const Pair p = slot_row(v, u);
+                const int i = 2 * p.t + ((p.j + p.l + (q >= v.H)) & 1);
+                const bool ok = i < v.Nx;                   // padding slots: zero (nothing writes them in global memory)
+                v.G[q] = ok ? g.G[q] : T(0);
+                if (!v.last && q < v.H) v.D[q] = ok ? g.D[q] : T(0);
+                for (int e = 0; e < 6; e++) v.A[e * v.ap + q] = ok ? g.A[e * v.ap + q] : T(0);
+            }
+        }
+        for (int L = Ls; L < nl - 1; L++) {
+            const SLev<T> v = tb.sv[L - Ls], cl = tb.sv[L + 1 - Ls];
+            for (int q = tid; q < 2 * v.H; q += nth) { v.pw[q] = 0; v.x[q] = 0; v.b[q] = 0; }
+            for (int q = tid; q < 2 * cl.H; q += nth) {
+                cl.G[q] = 0;
+                for (int e = 0; e < 6; e++) cl.A[e * cl.ap + q] = 0;
+            }
+            __syncthreads();
+            pg_weights<T>(P, v, cl, PT<T>::lev(P, L).ph, PT<T>::lev(P, L + 1).ph, qsign, tid, nth);
+            pg_pivots<T>(v, tid, nth);
+            __syncthreads();
+            pg_galerkin<T>(v, cl, nullptr, tid, nth);
+            __syncthreads();
+        }
+        const SLev<T> &v = tb.sv[nl - 1 - Ls];
+        for (int q = tid; q < 2 * v.H; q += nth) v.x[q] = v.b[q] = 0;
+        if (tid < v.N) {
+            const Node c = unidx(tid, v.Nx, v.Ny);
+            tb.slot[tid] = sslot(v, c.i, c.j, c.l);
+        }
+        __syncthreads();
+        blk_invert<T>(v);
     }
     return true;
 }
-// dynamic shared memory the set-up's dense inverse needs (block 0)
-constexpr size_t PG_SETUP_SMEM = sizeof(double) * COARSE_MAX * (COARSE_MAX + 1) + sizeof(int) * (COARSE_MAX + 1);
+
+// natural-order sol += d
+template <class T>
+__device__ __forceinline__ void pg_add_solution(const DevP &P, const PTab<T> &tb, const PS &s, bool assign) {
+    const SLev<T> v = tb.w.lev[0];
+    const T *d = tb.w.vec[7];
+    for (int u = s.tid; u < v.H; u += s.nth) {
+        const Pair p = slot_row(v, u);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int i = 2 * p.t + q;
+            if (i >= v.Nx) continue;
+            const double x = (double)d[(((i + p.j + p.l) & 1) ? v.H : 0) + u];
+            double *sol = P.sol + i + v.Nx * p.row;
+            *sol = assign ? x : *sol + x;
+        }
+    }
+}
 
 // ---------------------------------------------------------------- the solve kernels
 // T: precision of the Krylov iterations and the hierarchy.  PK_PCG: the Poisson Newton
-// system from the present sol (T = float: sol starts at 0 and the result is copied to the
-// FP64 sol when it converged).  PK_BICG (T = double): the continuity system from the
-// present sol.  PK_REFINED (T = float): FP64 refinement steps around FP32 BiCGSTAB.
+// system from the present sol (T = float: from zero, and the result goes to the FP64 sol
+// when it converged).  PK_BICG (T = double): the continuity system from the present sol.
+// PK_REFINED (T = float): FP64 refinement steps around FP32 BiCGSTAB.
 template <class T, int KIND>
-__global__ void __launch_bounds__(PG_TPB, 1024 / PG_TPB) k_persist(const DevP *Ps, PArgs a) {
+__global__ void __launch_bounds__(PT_TPB, 1) k_persist(const DevP *Ps, PArgs a) {
     const DevP &P = Ps[0];
     extern __shared__ __align__(16) unsigned char sraw[];
-    __shared__ LevView<T> sv[MAXLEV];
     __shared__ PTab<T> tb;
     __shared__ KrylovS sk, so;                    // the loop's record (and the outer one: PK_REFINED)
     PS s;
@@ -665,143 +1120,110 @@ __global__ void __launch_bounds__(PG_TPB, 1024 / PG_TPB) k_persist(const DevP *P
     s.ntrace = a.ntrace;
     s.mode = a.barmode;
     s.onecl = a.onecl;
-    const int nl = P.nlev, N = P.N;
-    ptab_fill<T>(P, tb);
-    __syncthreads();
-    if (a.setup && !pg_setup<T>(P, s, a, tb, sraw)) return;
-    if (blockIdx.x == 0) {                        // the small levels stay in block 0's shared memory
-        if (threadIdx.x < nl - a.Ls) sv[threadIdx.x] = smem_view<T>(P, a.Ls + threadIdx.x, a.Ls, sraw);
-        __syncthreads();
-        blk_stage_small<T>(P, sv, a.Ls, nl);
-    }
-    if (threadIdx.x == 0) {
-        sk = *PT<T>::ks(P);
-        so = *P.ks;
-    }
-    __syncthreads();
-    KrylovS &rec = sk;
-    if constexpr (KIND == PK_PCG) {
-        T *r0 = tb.vec[0];
-        if constexpr (std::is_same<T, double>::value) {
-            for (int k = s.tid; k < N; k += s.nth) {
-                const Node nd = unidx(k, P.Nx, P.Ny);
-                r0[k] = P.rhs[k] - a64_at<double>(tb.A64, tb.ap64, P.sol, k, nd.i, nd.j, nd.l, P.Nx, P.Ny, P.Nz,
-                                                  nullptr);
-            }
-        } else {
-            float *b32 = tb.rhs, *x32 = tb.sol;
-            for (int k = s.tid; k < N; k += s.nth) {
-                const float b = (float)P.rhs[k];
-                b32[k] = b;
-                r0[k] = b;
-                x32[k] = 0.f;
-            }
-        }
-        if (!pg_sync(s)) return;
-        if (!pg_vcycle<T>(s, a, tb, sv, nl, 0, 1, 0)) return;        // z = M r
-        double acc[1] = {0.0};
-        const T *z = tb.vec[1];
-        for (int k = s.tid; k < N; k += s.nth) acc[0] += (double)r0[k] * (double)z[k];
-        if (!pg_sum<1>(s, acc)) return;
+    const int nl = P.nlev;
+    {
+        const int *src = reinterpret_cast<const int *>(swork<T>(P));
+        int *dst = reinterpret_cast<int *>(&tb.w);
+        for (int q = threadIdx.x; q < (int)(sizeof(SWork<T>) / sizeof(int)); q += blockDim.x) dst[q] = src[q];
         if (threadIdx.x == 0) {
-            const double rz = acc[0];
-            rec.rz = rec.rz0 = rz; rec.it = 0; rec.status = 0;
-            rec.active = (rz > 0.0) ? 1 : 0;
-            if (!(rz > 0.0)) rec.status = 2;
+            tb.A64 = P.A[0];
+            tb.ap64 = (int)(P.A[1] - P.A[0]);
+            sk = *PT<T>::ks(P);
+            so = *P.ks;
         }
-        __syncthreads();
-        if (rec.active) {
-            T *p = tb.vec[2];
-            for (int k = s.tid; k < N; k += s.nth) p[k] = z[k];
-            if (!pg_sync(s)) return;
-            if (!pg_pcg<T>(s, a, tb, sv, nl, N, rec)) return;
-        }
-        if constexpr (std::is_same<T, float>::value) {
-            if (rec.status == 1)
-                for (int k = s.tid; k < N; k += s.nth) P.sol[k] = (double)tb.sol[k];
-        }
-    } else if constexpr (KIND == PK_BICG) {
-        double acc[2] = {0.0, 0.0};
-        pg_start64<T>(P, tb, s, nullptr, true, acc);
-        if (!pg_sum<2>(s, acc)) return;
+    }
+    __syncthreads();
+    // the system, its first residual and (level 0 -> 1) weights
+    double acc[2] = {0.0, 0.0};
+    pg_load<T, KIND>(P, tb, s, acc);
+    pg_weights<T>(P, tb.w.lev[0], tb.w.lev[1], nullptr, PT<T>::lev(P, 1).ph, a.qsign, s.tid, s.nth);
+    if (!pg_sum<2>(s, acc)) return;
+    if constexpr (KIND != PK_PCG) {
         if (threadIdx.x == 0) {
+            KrylovS &rec = KIND == PK_REFINED ? so : sk;
+            const double rtol = KIND == PK_REFINED ? so.rtol : a.rtol, atol = KIND == PK_REFINED ? so.atol : a.atol;
             rec.rr = acc[0]; rec.fl = acc[1];
             rec.r0 = sqrt(acc[0]);
-            rec.tgt = fmax(a.rtol * rec.r0, a.atol * sqrt(acc[1]));
-            rec.rho = rec.al = rec.om = 1.0; rec.rbest = rec.r0; rec.stall = 0; rec.it = 0; rec.half = 0;
+            rec.tgt = fmax(rtol * rec.r0, atol * sqrt(acc[1]));
+            rec.rbest = rec.r0; rec.stall = 0; rec.it = 0; rec.half = 0; rec.rho1 = acc[0];
             if (!(rec.r0 > rec.tgt)) { rec.active = 0; rec.status = 1; }
             else { rec.active = 1; rec.status = 0; }
         }
         __syncthreads();
-        if (!pg_bicg<T>(s, a, tb, sv, nl, N, rec)) return;
-    } else {                                      // PK_REFINED
-        double acc[2] = {0.0, 0.0};
-        float *rhs32 = tb.rhs;
-        pg_start64<T>(P, tb, s, rhs32, false, acc);
-        if (!pg_sum<2>(s, acc)) return;
-        if (threadIdx.x == 0) {
-            so.rr = acc[0]; so.fl = acc[1];
-            so.r0 = sqrt(acc[0]);
-            so.tgt = fmax(so.rtol * so.r0, so.atol * sqrt(acc[1]));
-            so.rbest = so.r0; so.stall = 0; so.it = 0; so.half = 0;
-            if (!(so.r0 > so.tgt)) { so.active = 0; so.status = 1; }
-            else { so.active = 1; so.status = 0; }
+    }
+    const bool go = KIND == PK_PCG || (KIND == PK_REFINED ? so.active : sk.active) != 0;
+    int steps = 0;
+    if (go) {
+        if (!pg_setup<T>(P, s, a, tb, nl, tb.w.vec[KIND == PK_PCG ? 1 : 4], sraw)) return;
+        if constexpr (KIND == PK_PCG) {
+            if (!pg_pcg<T>(s, a, tb, nl, sk)) return;
+            if (std::is_same<T, double>::value || sk.status == 1)
+                pg_add_solution<T>(P, tb, s, std::is_same<T, float>::value);
+        } else if constexpr (KIND == PK_BICG) {
+            if (!pg_bicg<T>(s, a, tb, nl, sk)) return;
+            pg_add_solution<T>(P, tb, s, false);
+        } else {                                  // PK_REFINED
+            double *x = P.sol, *r64 = P.wk[0];
+            double r32 = so.rr;                   // squared norm of the FP32 right-hand side (the FP64 one's, rounded)
+            for (; steps < a.maxsteps && so.active; steps++) {
+                if (threadIdx.x == 0) {
+                    sk.rr = r32;
+                    sk.r0 = sqrt(r32);
+                    sk.tgt = fmax(sk.rtol * sk.r0, sk.atol * so.tgt);
+                    sk.rho1 = r32; sk.rbest = sk.r0; sk.stall = 0; sk.it = 0; sk.half = 0;
+                    sk.body_runs = 0;
+                    sk.maxit = so.maxit - so.it;
+                    sk.status = 0;
+                    sk.active = (sk.r0 > sk.tgt && sk.maxit > 0) ? 1 : 0;
+                }
+                __syncthreads();
+                if (!pg_bicg<T>(s, a, tb, nl, sk)) return;
+                // x += d; r -= A d (FP64 operator); the next inner start r = rh = p = (float) r
+                double au[2] = {0.0, 0.0};
+                {
+                    const SLev<T> v = tb.w.lev[0];
+                    const T *d = tb.w.vec[7];
+                    for (int u = s.tid; u < v.H; u += s.nth) {
+                        const Pair p = slot_row(v, u);
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            const int i = 2 * p.t + q, c = (i + p.j + p.l) & 1, m = (c ? v.H : 0) + u;
+                            if (i >= v.Nx) continue;
+                            const int k = i + v.Nx * p.row;
+                            double fl, row[7];
+                            const double sum = row64(tb.A64, tb.ap64, k, i, p.j, p.l, v.Nx, v.Ny, v.Nz, row,
+                                                     [&](int, int ii, int jj, int ll) { return (double)d[sslot(v, ii, jj, ll)]; }, fl);
+                            x[k] += (double)d[m];
+                            const double rk = r64[k] - sum;
+                            r64[k] = rk;
+                            const T f = (T)rk;
+                            tb.w.vec[0][m] = f; tb.w.vec[1][m] = f; tb.w.vec[2][m] = f;
+                            if (!c) tb.w.vec[4][m] = v.D[m] * f;
+                            au[0] += rk * rk;
+                            au[1] += (double)f * (double)f;
+                        }
+                    }
+                }
+                if (!pg_sum<2>(s, au)) return;
+                r32 = au[1];
+                if (threadIdx.x == 0) {
+                    so.it += sk.it;
+                    so.body_runs++;
+                    so.rr = au[0];
+                    const double rn = sqrt(au[0]);
+                    if (rn <= so.tgt) { so.active = 0; so.status = 1; }
+                    else if (!(rn < 0.5 * so.rbest)) { so.active = 0; so.status = 4; }
+                    else if (so.it >= so.maxit) { so.active = 0; so.status = 3; }
+                    else so.rbest = rn;
+                }
+                __syncthreads();
+            }
         }
-        __syncthreads();
-        int steps = 0;
-        double *x = P.sol, *r64 = P.wk[0];
-        const int Nx = P.Nx, Ny = P.Ny, Nz = P.Nz;
-        for (; steps < a.maxsteps && so.active; steps++) {
-            // inner start: d = 0, r = rh = rhs32, p = v = 0
-            float *r = tb.vec[0], *rh = tb.vec[1], *p = tb.vec[2], *v = tb.vec[3], *d = tb.sol;
-            double ai[1] = {0.0};
-            for (int k = s.tid; k < N; k += s.nth) {
-                const float bk = rhs32[k];
-                r[k] = bk; rh[k] = bk; p[k] = 0.f; v[k] = 0.f; d[k] = 0.f;
-                ai[0] += (double)bk * (double)bk;
-            }
-            if (!pg_sum<1>(s, ai)) return;
-            if (threadIdx.x == 0) {
-                sk.rr = ai[0];
-                sk.r0 = sqrt(ai[0]);
-                sk.tgt = fmax(sk.rtol * sk.r0, sk.atol * so.tgt);
-                sk.rho = sk.al = sk.om = 1.0; sk.rbest = sk.r0; sk.stall = 0; sk.it = 0; sk.half = 0;
-                sk.body_runs = 0;
-                sk.maxit = so.maxit - so.it;
-                sk.status = 0;
-                sk.active = (sk.r0 > sk.tgt && sk.maxit > 0) ? 1 : 0;
-            }
-            __syncthreads();
-            if (!pg_bicg<float>(s, a, tb, sv, nl, N, sk)) return;
-            // x += d; r -= A d (FP64 operator); rhs32 = (float) r; the outer stop test
-            double au[1] = {0.0};
-            for (int k = s.tid; k < N; k += s.nth) {
-                const Node nd = unidx(k, Nx, Ny);
-                const double sum = a64_at<float>(tb.A64, tb.ap64, d, k, nd.i, nd.j, nd.l, Nx, Ny, Nz, nullptr);
-                x[k] += (double)d[k];
-                const double rk = r64[k] - sum;
-                r64[k] = rk;
-                rhs32[k] = (float)rk;
-                au[0] += rk * rk;
-            }
-            if (!pg_sum<1>(s, au)) return;
-            if (threadIdx.x == 0) {
-                so.it += sk.it;
-                so.body_runs++;
-                so.rr = au[0];
-                const double rn = sqrt(au[0]);
-                if (rn <= so.tgt) { so.active = 0; so.status = 1; }
-                else if (!(rn < 0.5 * so.rbest)) { so.active = 0; so.status = 4; }
-                else if (so.it >= so.maxit) { so.active = 0; so.status = 3; }
-                else so.rbest = rn;
-            }
-            __syncthreads();
-        }
-        if (blockIdx.x == 0 && threadIdx.x == 0) s.g->steps = steps;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *PT<T>::ks(P) = sk;
         if (KIND == PK_REFINED) *P.ks = so;
+        s.g->steps = steps;
         s.g->iters = KIND == PK_REFINED ? so.it : sk.it;
     }
 }
@@ -842,7 +1264,6 @@ bool g_coop_ok = false;    // the device supports cooperative launches
 unsigned long long *g_trace = nullptr;   // armed barrier timeline (test hook): device buffer
 int g_trace_n = 0, g_trace_used = 0;     // its barriers; 1 once a launch has filled it
 int g_last_blocks = 0;                   // blocks of the last persistent launch
-int g_fuse_up = 1;         // deferred prolongation on the way up (SEMISIM_B200_FUSEUP=0: off)
 int g_barmode = 1;         // grid-barrier form (SEMISIM_B200_BARMODE; 1 measured faster than 0)
 int g_clusters = 1;        // cluster launches: 0 off, 1 grids of one cluster, 2 every grid (SEMISIM_B200_CLUSTERS)
 int g_csz = 8;             // CTAs per cluster (SEMISIM_B200_CSZ: 8 portable, 16 non-portable)
@@ -861,7 +1282,7 @@ int cluster_occupancy(const void *fn, size_t smem) {
     }
     cudaLaunchConfig_t q = {};
     q.gridDim = dim3(g_csz);
-    q.blockDim = dim3(PG_TPB);
+    q.blockDim = dim3(PT_TPB);
     q.dynamicSmemBytes = smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -879,7 +1300,7 @@ int occupancy(const void *fn, size_t smem) {
         return 0;
     }
     int per = 0, dev = 0, nsm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, PG_TPB, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, PT_TPB, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -895,7 +1316,6 @@ int persist_enabled() {
         const char *e = std::getenv("SEMISIM_B200_PERSIST");
         g_persist_mode = (e && std::atoi(e) == 0) ? 0 : 1;
         if (const char *b = std::getenv("SEMISIM_B200_PBLOCKS")) g_persist_blocks = std::atoi(b);
-        if (const char *f = std::getenv("SEMISIM_B200_FUSEUP")) g_fuse_up = std::atoi(f) != 0;
         if (const char *m = std::getenv("SEMISIM_B200_BARMODE")) g_barmode = std::atoi(m) ? 1 : 0;
         if (const char *m = std::getenv("SEMISIM_B200_CLUSTERS")) g_clusters = std::atoi(m) < 0 ? 0 : (std::atoi(m) > 2 ? 2 : std::atoi(m));
         if (const char *m = std::getenv("SEMISIM_B200_CLEVEL")) g_clevel = std::atoi(m) < 1 ? 1 : std::atoi(m);
@@ -944,7 +1364,7 @@ static int persist_run(const Ctx &c, int Ls, size_t smem, const PArgs &a, PGrid 
     int nb = ki.blocks;
     // small systems take a part of the GPU (about two nodes per thread), so that several
     // instances' solves can run side by side
-    const int want = (c.maxN + 2 * PG_TPB - 1) / (2 * PG_TPB);
+    const int want = (c.maxN + 2 * PT_TPB - 1) / (2 * PT_TPB);
     if (want < nb) nb = want < 4 ? 4 : want;
     if (g_persist_blocks > 0 && g_persist_blocks < nb) nb = g_persist_blocks;
     if (c.pblocks > 0 && c.pblocks < nb) nb = c.pblocks;
@@ -991,7 +1411,7 @@ static int persist_run(const Ctx &c, int Ls, size_t smem, const PArgs &a, PGrid 
     g_last_blocks = nb;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nb);
-    cfg.blockDim = dim3(PG_TPB);
+    cfg.blockDim = dim3(PT_TPB);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.st;
     cudaLaunchAttribute at[2];
@@ -1032,19 +1452,16 @@ static int persist_run(const Ctx &c, int Ls, size_t smem, const PArgs &a, PGrid 
     return 1;
 }
 
-// algorithmic bytes of one V-cycle of precision T (the passes the persistent kernel runs)
+// algorithmic bytes of one V-cycle of precision T (the passes the persistent kernel runs): a
+// half sweep reads 6 couplings, pivot, right-hand side and the other colour and writes its
+// own (10 words a node of its colour; the diagonal and own values too in a black update)
 template <class T>
 static double vcycle_bytes(const MGHost &mg, int Ls, int deep, int sweeps2) {
-    const double w = sizeof(T) / 8.0;
     double b = 0.0;
     for (int L = 0; L < Ls; L++) {
-        const double n = mg.maxN[L];
-        const int sm = (L < deep && sweeps2) ? 2 : 1;
-        // smoother half sweeps (black, red) per application, pre and post; residual +
-        // restriction; prolongation and residual on the way up
-        b += n * w * (2.0 * sm * (kProfBytesPerNode[PF_SMOOTH_B] + kProfBytesPerNode[PF_SMOOTH_R]) +
-                      kProfBytesPerNode[PF_RESID_RESTRICT] + kProfBytesPerNode[PF_PROLONG] +
-                      kProfBytesPerNode[PF_LEVEL_RESID]);
+        const double half = 0.5 * mg.maxN[L] * sizeof(T);
+        const double twice = (L < deep && sweeps2) ? 2.0 * (10.0 + 12.0) : 0.0;
+        b += half * (10.0 + 10.0 + 10.25 + 11.25 + 13.25 + 10.0 + twice);
     }
     b += 2.0 * mg.maxN[Ls] * sizeof(T);             // b in, x out of the shared-memory levels
     return b;
@@ -1077,11 +1494,14 @@ static int persist_plan(const Ctx &c, const MGHost &mg, size_t *smem) {
     while (L < mg.maxlev - 1 && mg.maxN[L] > lim) L++;
     auto bytes = [&](int Ls) {
         size_t b = 0;
-        for (int q = Ls; q < mg.maxlev; q++) b += smem_level_bytes<T>(mg.maxN[q], q == mg.maxlev - 1);
+        for (int q = Ls; q < mg.maxlev; q++) {
+            const int hx = (((mg.maxNx[q] + 1) / 2) + 1) & ~1, H = hx * mg.maxRows[q], ap = (2 * H + 31) & ~31;
+            b += ssm_level<T>(H, ap, mg.maxN[q], q == mg.maxlev - 1);
+        }
         return b;
     };
     while (L < mg.maxlev - 1 && bytes(L) > cap) L++;
-    if (bytes(L) > cap) return -1;
+    if (bytes(L) > cap || mg.maxlev - L > 15) return -1;    // (one hardware barrier per level)
     *smem = bytes(L);
     return L;
 }
@@ -1090,18 +1510,15 @@ static int persist_plan(const Ctx &c, const MGHost &mg, size_t *smem) {
 // records hold the result), 0 (not applicable: nothing was changed) or -1 (abandoned: the
 // caller restores the start and uses the per-pass solve).
 int persist_pcg(const Ctx &c, const MGHost &mg, int mixed) {
-    if (c.ninst != 1 || !persist_enabled()) return 0;
+    if (c.ninst != 1 || !c.h.pwd || !persist_enabled()) return 0;
     size_t smem = 0;
     PArgs a{};
     a.Ls = mixed ? persist_plan<float>(c, mg, &smem) : persist_plan<double>(c, mg, &smem);
     if (a.Ls < 1) return 0;
-    a.setup = 1;
     a.qsign = 0;
-    smem = std::max(smem, PG_SETUP_SMEM);
     a.deep = g_deep_levels;
     a.sweeps2 = g_l0_sweeps > 1;
     a.alpha = mg.alpha;
-    a.fuse_up = g_fuse_up;
     a.barmode = g_barmode;
     PGrid h{};
     const int rc = mixed ? persist_run<float, PK_PCG>(c, a.Ls, smem, a, &h)
@@ -1117,18 +1534,15 @@ int persist_pcg(const Ctx &c, const MGHost &mg, int mixed) {
     return rc;
 }
 int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int qsign) {
-    if (c.ninst != 1 || !persist_enabled()) return 0;
+    if (c.ninst != 1 || !c.h.pwd || !persist_enabled()) return 0;
     size_t smem = 0;
     PArgs a{};
     a.Ls = persist_plan<double>(c, mg, &smem);
     if (a.Ls < 1) return 0;
-    a.setup = 1;
     a.qsign = qsign;
-    smem = std::max(smem, PG_SETUP_SMEM);
     a.deep = g_deep_levels;
     a.sweeps2 = g_l0_sweeps > 1;
     a.alpha = mg.alpha;
-    a.fuse_up = g_fuse_up;
     a.barmode = g_barmode;
     a.rtol = rtol;
     a.atol = atol;
@@ -1143,18 +1557,15 @@ int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int q
     return rc;
 }
 int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign) {
-    if (c.ninst != 1 || !persist_enabled()) return 0;
+    if (c.ninst != 1 || !c.h.pwd || !persist_enabled()) return 0;
     size_t smem = 0;
     PArgs a{};
     a.Ls = persist_plan<float>(c, mg, &smem);
     if (a.Ls < 1) return 0;
-    a.setup = 1;
     a.qsign = qsign;
-    smem = std::max(smem, PG_SETUP_SMEM);
     a.deep = g_deep_levels;
     a.sweeps2 = g_l0_sweeps > 1;
     a.alpha = mg.alpha;
-    a.fuse_up = g_fuse_up;
     a.barmode = g_barmode;
     a.maxsteps = maxsteps;
     PGrid h{};

@@ -72,6 +72,39 @@ struct LevelT {
     double *ph;                  // reference level / VT of the Slotboom weights (set-up only)
 };
 
+// n / d for 0 <= n < 2^31 without a division: (umulhi(n, mul) + n) >> sh
+struct FastDiv {
+    unsigned mul, sh;
+};
+inline FastDiv fast_div(unsigned d) {
+    FastDiv f;
+    f.sh = 0;
+    while ((1ull << f.sh) < d) f.sh++;
+    f.mul = (unsigned)((((1ull << f.sh) - d) << 32) / d + 1);
+    return f;
+}
+
+// One level of the persistent solves' own copy of the hierarchy, colour by colour: node
+// (i, j, l) of colour c = (i + j + l) & 1 (0 red, 1 black) sits at slot i/2 of row j + Ny l of
+// its colour, i.e. at c*H + hx*(j + Ny*l) + i/2 (hx slots per row, padded to a pair; padding
+// slots hold zeros).  A half sweep then reads its own couplings and the other colour's
+// values as contiguous pairs.  Couplings: 0 xm, 1 xp, 2 ym, 3 yp, 4 zm, 5 zp at
+// A[q*ap + c*H + slot], zero where there is no neighbour; G the diagonal.
+template <class T>
+struct SLev {
+    T *A, *G, *D, *pw, *x, *b;   // D: reciprocal pivots (coarsest level: the dense inverse, nodes in natural order)
+    int ap, H, hx, sz;           // sz = hx * Ny
+    int Nx, Ny, Nz, N, cx, cy, cz, last;
+    FastDiv fr, fy, f8;          // by hx/2, by Ny, by the groups of 8 nodes along x
+    int n8, nt;                  // those groups; threads of the one-block part of a cycle
+};
+constexpr int PW_VEC = 8;        // level-0 vectors of the persistent solves
+template <class T>
+struct SWork {
+    SLev<T> lev[MAXLEV];
+    T *vec[PW_VEC], *w0;         // Krylov vectors and row weights in the same order
+};
+
 // per-instance Krylov scalars (device resident; written by the reduction finalisers)
 struct KrylovS {
     double rho, al, om, rho1, be, rv, ss, tt, ts, rr, r0, tgt, rbest, fl;
@@ -182,6 +215,10 @@ struct DevP {
     float *wk32[8];
     KrylovS *ksi;                 // Krylov record of the FP32 inner solve
     PGrid *pgrid;                 // barrier and reduction records of the persistent solves
+    // the persistent solves' colour-by-colour hierarchy and vectors; the FP64 and the FP32
+    // tables describe the same memory (one solve at a time; each builds what it needs)
+    SWork<double> *pwd;
+    SWork<float> *pwf;
     // multigrid (FP64 and FP32 hierarchies)
     LevelT<double> *lev;          // device array of nlev levels
     LevelT<float> *levf;

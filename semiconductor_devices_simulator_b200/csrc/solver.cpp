@@ -92,7 +92,7 @@ struct Carver {
 
 // Lay out every device array of an instance in one block (two passes: size, then place).
 static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &levs, std::vector<LevelT<float>> &levsf,
-                  int nlev, const int dims[][6]) {
+                  SWork<double> &pwd, SWork<float> &pwf, int nlev, const int dims[][6]) {
     const size_t N = d.N;
     P.flags = cv.take<uint32_t>(N);
     P.Nd = cv.take<double>(N); P.Na = cv.take<double>(N); P.Nf = cv.take<double>(N);
@@ -178,6 +178,13 @@ static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &lev
         v.pw = cv.take<float>(n);
         v.ph = levs[L].ph;              // set-up scratch, shared with the FP64 twin
     }
+    if (!d.unstr) {                      // the persistent solves' hierarchy (graph meshes have their own)
+        P.pwd = cv.take<SWork<double>>(1);
+        P.pwf = cv.take<SWork<float>>(1);
+        char *area = cv.take<char>(persist_work_layout<double>(nullptr, dims, nlev, nullptr));
+        persist_work_layout<double>(area, dims, nlev, &pwd);
+        persist_work_layout<float>(area, dims, nlev, &pwf);
+    }
 }
 
 // 2x2x2 aggregation hierarchy shape (semiconductor_3d.c:1894-1921)
@@ -227,7 +234,7 @@ void gpu_free(Inst &d) {
 }
 
 static int gpu_alloc(Inst &d) {
-    if (d.g.ready && d.g.h.Nx == d.Nx && d.g.h.Ny == d.Ny && d.g.h.Nz == d.Nz) return 1;
+    if (d.g.ready && d.g.h.Nx == d.Nx && d.g.h.Ny == d.Ny && d.g.h.Nz == d.Nz && (d.unstr || d.g.h.pwd)) return 1;
     gpu_free(d);
     if (!gpu_available()) {
         std::fprintf(stderr, "semisim-b200: no CUDA device available - the solver has no CPU path\n");
@@ -253,7 +260,9 @@ static int gpu_alloc(Inst &d) {
     DevP P{};
     std::vector<LevelT<double>> levs;
     std::vector<LevelT<float>> levsf;
-    carve(d, cv, P, levs, levsf, nl, dims);       // sizing pass
+    SWork<double> pwd{};
+    SWork<float> pwf{};
+    carve(d, cv, P, levs, levsf, pwd, pwf, nl, dims);       // sizing pass
     const size_t bytes = cv.off;
     void *blk = nullptr;
     CK(cudaMalloc(&blk, bytes));
@@ -261,7 +270,7 @@ static int gpu_alloc(Inst &d) {
     Carver cv2;
     cv2.base = static_cast<char *>(blk);
     P = DevP{};
-    carve(d, cv2, P, levs, levsf, nl, dims);
+    carve(d, cv2, P, levs, levsf, pwd, pwf, nl, dims);
     P.Nx = d.Nx; P.Ny = d.Ny; P.Nz = d.Nz; P.N = (int)d.N; P.nlev = nl;
     d.g.block = blk;
     d.g.bytes = bytes;
@@ -283,6 +292,10 @@ static int gpu_alloc(Inst &d) {
             }
     CK(cudaMemcpy(P.lev, levs.data(), sizeof(LevelT<double>) * nl, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(P.levf, levsf.data(), sizeof(LevelT<float>) * nl, cudaMemcpyHostToDevice));
+    if (P.pwd) {
+        CK(cudaMemcpy(P.pwd, &pwd, sizeof pwd, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(P.pwf, &pwf, sizeof pwf, cudaMemcpyHostToDevice));
+    }
     MGHost &mg = d.g.mg;
     mg.maxlev = mg.minlev = nl;
     for (int L = 0; L < nl; L++) {

@@ -264,6 +264,10 @@ void vcycle(const Ctx &c, const MGHost &mg, int bsel, int xsel, int wsel, int mg
 int pcg_solve(const Ctx &c, const MGHost &mg, int maxit, double rtol, int check_every, int mixed = 0);
 // persistent (one cooperative launch per solve) forms, kernels_persist.cu: 1 done, 0 not
 // applicable, -1 abandoned (the caller restores the start and solves per pass)
+// lays the persistent solves' hierarchy and vectors of precision T out from `base` (null: sizes
+// only) and describes them in *w; returns the bytes
+template <class T>
+size_t persist_work_layout(char *base, const int dims[][6], int nlev, SWork<T> *w);
 int persist_enabled();
 void persist_set(int mode, int blocks);
 int persist_get_blocks();
