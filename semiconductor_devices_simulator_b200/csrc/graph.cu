@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "device_common.cuh"
+#include "ccl_common.cuh"
 #include "exact_sum.cuh"
 #include "physics_hd.cuh"
 #include "prof.h"
@@ -492,31 +493,26 @@ __global__ void k_floor_g(const DevP *__restrict__ Ps, const double *b, const do
 }
 
 // ------------------------------------------------------------------ labelling
-// floating blocks: labels take the smallest label of a labelled neighbour
-__global__ void k_ff_prop_g(const DevP *__restrict__ Ps, int *changed) {
+// floating blocks: join every labelled node with its lower neighbours (ccl_common.cuh)
+__global__ void k_ff_merge_g(const DevP *__restrict__ Ps) {
     const DevP &P = Ps[0];
     const int N = P.N, D = P.gD;
     int *lab = P.ccl;
-    int ch = 0;
     SS_GRID_LOOP(k, N) {
-        int a = lab[k];
-        if (a < 0) continue;
+        if (lab[k] < 0) continue;
         for (int q = 0; q < D; q++) {
             const int j = P.gcol[(size_t)q * N + k];
-            if (j < 0) continue;
-            const int b = lab[j];
-            if (b >= 0 && b < a) a = b;
+            if (j >= 0 && j < k && lab[j] >= 0) uf_union(lab, k, j);
         }
-        if (a < lab[k]) { lab[k] = a; ch = 1; }
     }
-    if (ch) *changed = 1;
 }
 __global__ void k_ff_anchor_g(const DevP *__restrict__ Ps) {
     const DevP &P = Ps[0];
     const int N = P.N, D = P.gD;
     SS_GRID_LOOP(k, N) {
-        const int lb = P.ccl[k];
-        if (lb < 0) continue;
+        if (P.ccl[k] < 0) continue;
+        const int lb = uf_find(P.ccl, k);
+        P.ccl[k] = lb;
         for (int q = 0; q < D; q++) {
             const int j = P.gcol[(size_t)q * N + k];
             if (j < 0) continue;
@@ -774,19 +770,10 @@ int bicg_graph(Inst &d, int maxit, double rtol, double atol, double *rn_out, dou
 
 // floating majority blocks of the graph: label, anchor, boundary (float_fix_g); the
 // recombination balance and the rescaling are the tensor path's node-wise kernels
-int ff_label_g(Inst &d, int *changed) {
+void ff_label_g(Inst &d) {
     Ctx c = make_ctx(d);
-    int h = 1, cycles = 0;
-    const int maxcyc = (int)d.N + 8;
-    while (h && cycles < maxcyc) {
-        cudaMemsetAsync(changed, 0, sizeof(int), c.st);
-        for (int q = 0; q < 8; q++) SS_LAUNCH(PF_CCL, d.N, k_ff_prop_g, gblocks(c), TPB, c.st, c.dP, changed);
-        cudaMemcpyAsync(&h, changed, sizeof(int), cudaMemcpyDeviceToHost, c.st);
-        cudaStreamSynchronize(c.st);
-        cycles += 8;
-    }
+    SS_LAUNCH(PF_CCL, d.N, k_ff_merge_g, gblocks(c), TPB, c.st, c.dP);
     SS_LAUNCH(PF_CCL, d.N, k_ff_anchor_g, gblocks(c), TPB, c.st, c.dP);
-    return 1;
 }
 void ff_boundary_g(Inst &d, int hole, unsigned long long *Aout, unsigned long long *Bin) {
     Ctx c = make_ctx(d);

@@ -4,14 +4,17 @@
 // (net outflow + recombination inside = 0) holds; Newton in ln(lambda) per block.
 //
 // The reference finds the blocks by a breadth-first search.  Here the components are
-// labelled on the device by min-label propagation with line sweeps along x, y, z
-// (each sweep carries labels the whole length of a line), the anchoring test and the
-// block sums are per-node kernels adding into per-block exact accumulators (exact_sum.cuh),
-// so that the sums, and the rescaled solution, do not depend on the order of the threads.
+// labelled on the device by union-find (ccl_common.cuh) in one merging pass, the anchoring
+// test and the block sums are per-node kernels adding into per-block exact accumulators
+// (exact_sum.cuh), so that the sums, and the rescaled solution, do not depend on the order of
+// the threads.  What bounds it is launches and the wait for the block count, not memory: four
+// short kernels and one wait per call (576,000 nodes: 107 us of kernels; min-label propagation by line
+// sweeps until nothing changed took 305 us in ~15 launches, and a wait for every turn).
 #include <cmath>
 #include <cstdio>
 #include <vector>
 
+#include "ccl_common.cuh"
 #include "device_common.cuh"
 #include "exact_sum.cuh"
 #include "prof.h"
@@ -31,42 +34,48 @@ __device__ __forceinline__ bool ff_maj(const DevP &P, int k, int hole) {
     return c >= oth && c >= hd && s >= hd && c > 10.0 * niK(P, m, k);
 }
 
-__global__ void k_ff_init(const DevP *__restrict__ Ps, int hole) {
+// majority nodes start as the first node of their run inside a warp along x (runs of
+// consecutive majority nodes of one row), the others as -1
+__global__ void k_ff_init(const DevP *__restrict__ Ps, int hole, int *count) {
     const DevP &P = Ps[blockIdx.y];
-    SS_GRID_LOOP(k, P.N) {
-        P.ccl[k] = ff_maj(P, k, hole) ? k : -1;
-        P.cclaux[k] = 0;
+    const int lane = threadIdx.x & 31, nw = (P.N + 31) & ~31;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
+    SS_GRID_LOOP(k, nw) {                             // whole warps
+        const bool in = k < P.N, maj = in && ff_maj(P, k, hole);
+        const bool head = !maj || P.gcol || k % P.Nx == 0;      // (graph nodes are no rows)
+        const unsigned m = __ballot_sync(0xffffffffu, maj), h = __ballot_sync(0xffffffffu, head);
+        if (in) {
+            // the run starts after the last non-majority lane, or at the last row start, below or here
+            const unsigned below = (2u << lane) - 1u;
+            const unsigned starts = ((h & m) | (m & ~(m << 1))) & below;
+            P.ccl[k] = maj ? k - lane + (31 - __clz(starts)) : -1;
+            P.cclaux[k] = 0;
+        }
     }
 }
-__global__ void k_ff_sweep(const DevP *__restrict__ Ps, int ax, int *changed) {
+// join every majority node with its lower neighbours; a link along y or z is left out where
+// the previous node along x has the same one (the two rows' runs are already joined there)
+__global__ void k_ff_merge(const DevP *__restrict__ Ps) {
     const DevP &P = Ps[blockIdx.y];
-    const int n = ax == 0 ? P.Nx : (ax == 1 ? P.Ny : P.Nz);
-    const int st = ax == 0 ? 1 : (ax == 1 ? P.Nx : P.Nx * P.Ny);
-    const int nlines = P.N / n;
     int *lab = P.ccl;
-    int ch = 0;
-    SS_GRID_LOOP(t, nlines) {
-        int k0;
-        if (ax == 0) k0 = t * P.Nx;
-        else if (ax == 1) { const int i = t % P.Nx, l = t / P.Nx; k0 = i + l * P.Nx * P.Ny; }
-        else k0 = t;
-        for (int q = 1; q < n; q++) {
-            const int k = k0 + q * st, a = lab[k], b = lab[k - st];
-            if (a >= 0 && b >= 0 && b < a) { lab[k] = b; ch = 1; }
-        }
-        for (int q = n - 2; q >= 0; q--) {
-            const int k = k0 + q * st, a = lab[k], b = lab[k + st];
-            if (a >= 0 && b >= 0 && b < a) { lab[k] = b; ch = 1; }
-        }
+    const int Nx = P.Nx, NxNy = P.Nx * P.Ny;
+    SS_GRID_LOOP(k, P.N) {
+        if (lab[k] < 0) continue;
+        const Node a = unidx(k, Nx, P.Ny);
+        const bool left = a.i > 0 && lab[k - 1] >= 0;
+        if (left && (k & 31) == 0) uf_union(lab, k, k - 1);      // a run cut at a warp's edge
+        if (a.j > 0 && lab[k - Nx] >= 0 && !(left && lab[k - Nx - 1] >= 0)) uf_union(lab, k, k - Nx);
+        if (a.l > 0 && lab[k - NxNy] >= 0 && !(left && lab[k - NxNy - 1] >= 0)) uf_union(lab, k, k - NxNy);
     }
-    if (ch) *changed = 1;
 }
-// a block touching a semiconductor contact node is anchored
+// every node gets its component's root; a block touching a semiconductor contact node is
+// anchored
 __global__ void k_ff_anchor(const DevP *__restrict__ Ps) {
     const DevP &P = Ps[blockIdx.y];
     SS_GRID_LOOP(k, P.N) {
-        const int lb = P.ccl[k];
-        if (lb < 0) continue;
+        if (P.ccl[k] < 0) continue;
+        const int lb = uf_find(P.ccl, k);
+        P.ccl[k] = lb;
         const Node a = unidx(k, P.Nx, P.Ny);
         for (int dir = 0; dir < 6; dir++) {
             int kb; double h, ar;
@@ -166,24 +175,14 @@ int float_fix(Inst &d, int hole) {
     const dim3 g(c.nodes_blocks(), 1);
     double *const g_ffbuf = d.g.h.ffbuf;
     int *const g_ffint = d.g.h.ffint;
-    int *changed = g_ffint, *count = g_ffint + 1, *roots = g_ffint + 16;
-    SS_LAUNCH(PF_CCL, d.N, k_ff_init, g, TPB, c.st, c.dP, hole);
-    int h = 1, cycles = 0;
-    const int maxcyc = d.Nx + d.Ny + d.Nz + 8;
-    if (d.unstr) { ff_label_g(d, changed); h = 0; }           // labels over the graph's edges, anchors
-    while (h && cycles < maxcyc) {
-        cudaMemsetAsync(changed, 0, sizeof(int), c.st);
-        for (int ax = 0; ax < 3; ax++) {
-            const int n = ax == 0 ? d.Nx : (ax == 1 ? d.Ny : d.Nz);
-            const int nb = ((int)d.N / n + TPB - 1) / TPB;
-            SS_LAUNCH(PF_CCL, d.N, k_ff_sweep, dim3(nb, 1), TPB, c.st, c.dP, ax, changed);
-        }
-        cudaMemcpyAsync(&h, changed, sizeof(int), cudaMemcpyDeviceToHost, c.st);
-        cudaStreamSynchronize(c.st);
-        cycles++;
+    int *count = g_ffint + 1, *roots = g_ffint + 16;
+    SS_LAUNCH(PF_CCL, d.N, k_ff_init, g, TPB, c.st, c.dP, hole, count);
+    if (d.unstr) {
+        ff_label_g(d);                                        // over the graph's edges, anchors
+    } else {
+        SS_LAUNCH(PF_CCL, d.N, k_ff_merge, g, TPB, c.st, c.dP);
+        SS_LAUNCH(PF_CCL, d.N, k_ff_anchor, g, TPB, c.st, c.dP);
     }
-    if (!d.unstr) SS_LAUNCH(PF_CCL, d.N, k_ff_anchor, g, TPB, c.st, c.dP);
-    cudaMemsetAsync(count, 0, sizeof(int), c.st);
     SS_LAUNCH(PF_CCL, d.N, k_ff_roots, g, TPB, c.st, c.dP, count, roots);
     int nb = 0;
     cudaMemcpyAsync(&nb, count, sizeof(int), cudaMemcpyDeviceToHost, c.st);
