@@ -644,10 +644,9 @@ int pcg_graph(Inst &d, int maxit, double rtol) {
     Ctx c = make_ctx(d);
     double *x = d.g.h.sol, *b = d.g.h.rhs;
     double *r = d.g.h.wk[0], *z = d.g.h.wk[1], *p = d.g.h.wk[2], *q = d.g.h.wk[3];
-    gmg_setup(d, c, 0, nullptr);
-    if (persist_enabled()) {                      // the whole solve in one persistent launch
+    if (persist_enabled()) {                      // set-up and solve in one persistent launch
         lin(c, d.g.h.wk[7], 0.0, x, 1.0);        // start backup
-        const int pr = persist_graph(d, 0, maxit, rtol, 0.0, nullptr, false);
+        const int pr = persist_graph(d, 0, maxit, rtol, 0.0, 0, false);
         if (pr == 1) {
             KrylovS hs{};
             cudaMemcpyAsync(&hs, c.h.ks, sizeof(KrylovS), cudaMemcpyDeviceToHost, c.st);
@@ -656,6 +655,7 @@ int pcg_graph(Inst &d, int maxit, double rtol) {
         }
         if (pr < 0) lin(c, x, 0.0, d.g.h.wk[7], 1.0);
     }
+    gmg_setup(d, c, 0, nullptr);
     matvec(c, x, q);
     lin(c, r, 0.0, b, 1.0, q, -1.0);
     gmg_apply(d, c, r, z, nullptr, false);
@@ -694,10 +694,9 @@ int bicg_graph(Inst &d, int maxit, double rtol, double atol, double *rn_out, dou
     double *r = d.g.h.wk[0], *rh = d.g.h.wk[1], *p = d.g.h.wk[2], *v = d.g.h.wk[3], *ph = d.g.h.wk[4],
            *sh = d.g.h.wk[5], *t = d.g.h.wk[6];
     const double *w = d.g.h.dsc;
-    gmg_setup(d, c, qsign, w);
-    if (persist_enabled()) {                      // the whole solve in one persistent launch
+    if (persist_enabled()) {                      // set-up and solve in one persistent launch
         lin(c, d.g.h.wk[7], 0.0, x, 1.0);        // start backup
-        const int pr = persist_graph(d, 1, maxit, rtol, atol, w, ilu_only);
+        const int pr = persist_graph(d, 1, maxit, rtol, atol, qsign, ilu_only);
         if (pr == 1) {
             KrylovS hs{};
             cudaMemcpyAsync(&hs, c.h.ks, sizeof(KrylovS), cudaMemcpyDeviceToHost, c.st);
@@ -708,6 +707,7 @@ int bicg_graph(Inst &d, int maxit, double rtol, double atol, double *rn_out, dou
         }
         if (pr < 0) lin(c, x, 0.0, d.g.h.wk[7], 1.0);
     }
+    gmg_setup(d, c, qsign, w);
     matvec(c, x, t);
     lin(c, r, 0.0, b, 1.0, t, -1.0);
     lin(c, rh, 0.0, r, 1.0);

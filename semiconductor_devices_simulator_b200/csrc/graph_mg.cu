@@ -396,7 +396,7 @@ void gmg_free(Inst &d) {
     if (d.g.gmgblock) cudaFree(d.g.gmgblock);
     d.g.gmgblock = nullptr;
     if (d.g.gptab) cudaFree(d.g.gptab);
-    d.g.gptab = nullptr;
+    d.g.gptab = d.g.gprow = nullptr;
     d.g.glev.clear();
 }
 
@@ -511,6 +511,14 @@ int gmg_build(Inst &d, cudaStream_t st) {
         v.inv = (L == nl - 1 && n <= GMG_DENSE_MAX) ? (double *)(blk + o.inv) : nullptr;
     }
     if (cudaStreamSynchronize(st) != cudaSuccess) ok = false;
+    if (ok) {
+        std::vector<GpLevelIn> lv(nl);
+        for (int L = 0; L < nl; L++) {
+            const LevelBuild &b = B[L];
+            lv[L] = GpLevelIn{b.g.N, b.ncolor, &b.g.rp, &b.g.cj, &b.agg, &b.emap, &b.color, &b.cptr, &b.cnodes};
+        }
+        gpersist_build(d, lv, st);
+    }
     if (d.verbose)
         std::fprintf(stderr, "semisim-b200: graph multigrid %d levels, coarsest %d unknowns\n", nl, B.back().g.N);
     return ok ? 1 : 0;

@@ -82,7 +82,8 @@ struct Gpu {
     void *gmgblock = nullptr;    // graph multigrid levels (one allocation)
     std::vector<GLevHost> glev;  // graph multigrid hierarchy, level 0 = the mesh
     std::vector<GmgCycle> gcyc;  // its V-cycles captured as CUDA graphs (per operand set)
-    void *gptab = nullptr;       // the hierarchy's level table for the persistent graph solves (device)
+    void *gptab = nullptr;       // persistent graph solves: level table, colour-ordered levels (one allocation)
+    void *gprow = nullptr;       //   and, inside it, the dense inverse's pivot rows
     bool gcyc_off = false;       // capture failed once: launch the V-cycle directly
     void *trblock = nullptr;     // deep-level trap entries (CSR per node) and species
     void *coblock = nullptr;     // Coulomb interface entries and every node's nearest one
@@ -224,7 +225,14 @@ void launch_node_Jc_g(const Ctx &c, int which, double *out);
 void launch_emax_g(const Ctx &c);
 int pcg_graph(Inst &d, int maxit, double rtol);
 int bicg_graph(Inst &d, int maxit, double rtol, double atol, double *rn, double *r0, int qsign, bool ilu_only);
-int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, const double *w, bool ilu_only);
+int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qsign, bool ilu_only);
+// a level of the graph hierarchy on the host as the persistent solves' tables are built from it
+struct GpLevelIn {
+    int N, ncolor;
+    const std::vector<int> *rp, *cj, *agg, *emap;      // CSR; aggregates and coarse CSR entries (not the coarsest)
+    const std::vector<int> *color, *cptr, *cnodes;     // colours, and the nodes listed by colour
+};
+void gpersist_build(Inst &d, const std::vector<GpLevelIn> &lv, cudaStream_t st);
 // aggregation multigrid of a graph mesh (graph_mg.cu)
 int gmg_build(Inst &d, cudaStream_t st);
 void gmg_free(Inst &d);
