@@ -39,7 +39,7 @@ constexpr int OW1 = 0, OB1 = OW1 + MH * MI, OW2 = OB1 + MH, OB2 = OW2 + MH * MH,
 constexpr int QW1 = 0, QW2 = QW1 + MH * MI, QW3 = QW2 + MH * MH, QW4 = QW3 + MH * MH, NWB = QW4 + MO * MH;
 constexpr int NBIAS = 3 * MH + MO;
 // shared-memory row pitches (elements)
-constexpr int P1 = MI + 8, PH = MH + 8, PT4 = MO + 8;
+constexpr int P1 = MI + 8, PH = MH + 8;
 
 typedef __nv_bfloat16 bf16;
 
@@ -124,17 +124,39 @@ struct MlpSmem {
     bf16 W1[MH * P1], W2[MH * PH], W3[MH * PH], W4[MO * PH];
     float b1[MH], b2[MH], b3[MH], b4[MO];
 };
-__device__ __forceinline__ void load_weights(MlpSmem &s, const bf16 *Wb, const float *bias) {
-    for (int e = threadIdx.x; e < MH * MI; e += blockDim.x) s.W1[(e / MI) * P1 + e % MI] = Wb[QW1 + e];
-    for (int e = threadIdx.x; e < MH * MH; e += blockDim.x) {
-        s.W2[(e / MH) * PH + e % MH] = Wb[QW2 + e];
-        s.W3[(e / MH) * PH + e % MH] = Wb[QW3 + e];
+__device__ __forceinline__ bool al16p(const void *p) { return (reinterpret_cast<size_t>(p) & 15) == 0; }
+// rows x cols BF16 (cols a multiple of 8) into shared rows of `pitch`, 16 bytes at a time where
+// the source allows it (a caller's pointer may be less aligned)
+__device__ __forceinline__ void copy_rows(bf16 *dst, int pitch, const bf16 *src, int rows, int cols) {
+    const int c8 = cols / 8;
+    if (al16p(src)) {
+        for (int e = threadIdx.x; e < rows * c8; e += blockDim.x) {
+            const int r = e / c8, c = 8 * (e - r * c8);
+            *reinterpret_cast<uint4 *>(dst + r * pitch + c) = *reinterpret_cast<const uint4 *>(src + (size_t)r * cols + c);
+        }
+    } else {
+        for (int e = threadIdx.x; e < rows * cols; e += blockDim.x) dst[(e / cols) * pitch + e % cols] = src[e];
     }
-    for (int e = threadIdx.x; e < MO * MH; e += blockDim.x) s.W4[(e / MH) * PH + e % MH] = Wb[QW4 + e];
+}
+__device__ __forceinline__ void load_weights(MlpSmem &s, const bf16 *Wb, const float *bias) {
+    copy_rows(s.W1, P1, Wb + QW1, MH, MI);
+    copy_rows(s.W2, PH, Wb + QW2, MH, MH);
+    copy_rows(s.W3, PH, Wb + QW3, MH, MH);
+    copy_rows(s.W4, PH, Wb + QW4, MO, MH);
     for (int e = threadIdx.x; e < MH; e += blockDim.x) {
         s.b1[e] = bias[0 * MH + e]; s.b2[e] = bias[1 * MH + e]; s.b3[e] = bias[2 * MH + e];
     }
     for (int e = threadIdx.x; e < MO; e += blockDim.x) s.b4[e] = bias[3 * MH + e];
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const bf16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
 // one hidden layer of a warp's 16 rows: acc = A W^T + b (16 x 128), A given as BF16
@@ -142,18 +164,23 @@ __device__ __forceinline__ void load_weights(MlpSmem &s, const bf16 *Wb, const f
 template <int KS, int PW>
 __device__ __forceinline__ void layer_mma(float (&acc)[16][4], const uint32_t (&a)[KS][4], const bf16 *W,
                                           const float *b) {
-    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const int t = threadIdx.x & 3;
 #pragma unroll
     for (int nt = 0; nt < 16; nt++) {
         const float b0 = b[8 * nt + 2 * t], b1 = b[8 * nt + 2 * t + 1];
         acc[nt][0] = b0; acc[nt][1] = b1; acc[nt][2] = b0; acc[nt][3] = b1;
     }
+    // two output tiles' B fragments per ldmatrix: matrices (tile, k half) = (0,0) (0,1) (1,0) (1,1)
+    const int lane = threadIdx.x & 31;
+    const bf16 *w = W + (8 * (lane >> 4) + (lane & 7)) * PW + ((lane >> 3) & 1) * 8;
 #pragma unroll
     for (int ks = 0; ks < KS; ks++)
 #pragma unroll
-        for (int nt = 0; nt < 16; nt++) {
-            const bf16 *w = W + (8 * nt + g) * PW + 16 * ks + 2 * t;
-            mma16816(acc[nt], a[ks], ld32(w), ld32(w + 8));
+        for (int nt = 0; nt < 16; nt += 2) {
+            uint32_t f[4];
+            ldsm4(f, w + 8 * nt * PW + 16 * ks);
+            mma16816(acc[nt], a[ks], f[0], f[1]);
+            mma16816(acc[nt + 1], a[ks], f[2], f[3]);
         }
 }
 // SiLU of the accumulators repacked as the next layer's A fragments
@@ -190,7 +217,7 @@ __device__ __forceinline__ void out_mma(float (&o)[4], const uint32_t (&a)[8][4]
 // x_next = x1 + s (x1 - x0) + VT * MLP(X) for psi, phi_n, phi_p of every node; X the
 // node features (k_seed_features), 128 nodes per CTA pass (8 warps x 16 rows), x1 = h1 and
 // x0 = e2 of the instance
-constexpr int SEED_TPB = 128, SEED_ROWS = 64;            // training kernels
+constexpr int SEED_TPB = 256, SEED_ROWS = 128;           // training kernels
 constexpr int INF_TPB = 256, INF_ROWS = 128;             // inference
 __global__ void __launch_bounds__(INF_TPB) k_mlp_seed(const DevP *__restrict__ Ps, const bf16 *__restrict__ Wb,
                                                        const float *__restrict__ bias, SeedIn in,
@@ -245,6 +272,11 @@ __global__ void __launch_bounds__(INF_TPB) k_mlp_seed(const DevP *__restrict__ P
 }
 
 // ------------------------------------------------------------------ training kernels
+// Forward and backward passes: 128 rows a block (8 warps of 16), so a batch of 16,384 rows is one
+// block per SM and the weights are staged once per SM, 16 bytes at a time, B fragments of two
+// tiles per ldmatrix.  Bound by the chain of a warp's four layers and by writing Z and H (38 MB):
+// forward 22 us, backward 25 us at 16,384 rows (39 and 41 us with 64-row blocks that staged two
+// bytes at a time, the backward pass transposed copies of the weights).
 // forward of a batch: X [B][MI] -> Y [B][MO]; saves Z_l (FP32 pre-activations) and H_l
 // (BF16 activations) of the three hidden layers, [B][MH] each
 __global__ void __launch_bounds__(SEED_TPB) k_mlp_train_fwd(const bf16 *__restrict__ X, int B, const bf16 *__restrict__ Wb,
@@ -254,13 +286,23 @@ __global__ void __launch_bounds__(SEED_TPB) k_mlp_train_fwd(const bf16 *__restri
     bf16 *Xs = reinterpret_cast<bf16 *>(smraw + sizeof(MlpSmem));
     load_weights(s, Wb, bias);
     const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const bool xa = al16p(X);
     for (int base = blockIdx.x * SEED_ROWS; base < B; base += gridDim.x * SEED_ROWS) {
         __syncthreads();
-        for (int e = threadIdx.x; e < SEED_ROWS * MI / 2; e += blockDim.x) {
-            const int r = e / (MI / 2), q = 2 * (e % (MI / 2));
-            const int row = base + r;
-            const uint32_t v = row < B ? ld32(X + (size_t)row * MI + q) : 0u;
-            *reinterpret_cast<uint32_t *>(Xs + r * P1 + q) = v;
+        if (xa) {
+            for (int e = threadIdx.x; e < SEED_ROWS * MI / 8; e += blockDim.x) {
+                const int r = e / (MI / 8), q = 8 * (e % (MI / 8)), row = base + r;
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (row < B) v = *reinterpret_cast<const uint4 *>(X + (size_t)row * MI + q);
+                *reinterpret_cast<uint4 *>(Xs + r * P1 + q) = v;
+            }
+        } else {
+            for (int e = threadIdx.x; e < SEED_ROWS * MI / 2; e += blockDim.x) {
+                const int r = e / (MI / 2), q = 2 * (e % (MI / 2));
+                const int row = base + r;
+                const uint32_t v = row < B ? ld32(X + (size_t)row * MI + q) : 0u;
+                *reinterpret_cast<uint32_t *>(Xs + r * P1 + q) = v;
+            }
         }
         __syncthreads();
         uint32_t a0[3][4], a[8][4];
@@ -298,26 +340,20 @@ __global__ void __launch_bounds__(SEED_TPB) k_mlp_train_fwd(const bf16 *__restri
 // backward through the activations: dY = 2 (Y - T) / (3 B) on the 3 channels (loss =
 // mean squared error, accumulated into *loss), then dZ_3, dZ_2, dZ_1 (BF16 [B][MH]) with
 // dH_l = dZ_{l+1} W_{l+1} and dZ_l = dH_l * SiLU'(Z_l); dY is stored BF16 [B][MO]
+// (the products with W transposed read W's rows by ldmatrix.trans)
 struct MlpSmemT {
-    bf16 W2T[MH * PH], W3T[MH * PH], W4T[MH * PT4];
+    bf16 W2[MH * PH], W3[MH * PH], W4[MO * PH];
 };
 __global__ void __launch_bounds__(SEED_TPB) k_mlp_train_bwd(int B, const bf16 *__restrict__ Wb, const float *__restrict__ Y,
                                                              const float *__restrict__ T, const float *__restrict__ Z,
                                                              bf16 *dZ, bf16 *dY, float *loss) {
     extern __shared__ __align__(16) unsigned char smraw[];
     MlpSmemT &s = *reinterpret_cast<MlpSmemT *>(smraw);
-    for (int e = threadIdx.x; e < MH * MH; e += blockDim.x) {       // transposed copies: [in][out]
-        const int o = e / MH, i = e % MH;
-        s.W2T[i * PH + o] = Wb[QW2 + e];
-        s.W3T[i * PH + o] = Wb[QW3 + e];
-    }
-    for (int e = threadIdx.x; e < MH * PT4; e += blockDim.x) s.W4T[e] = __float2bfloat16(0.f);
+    copy_rows(s.W2, PH, Wb + QW2, MH, MH);
+    copy_rows(s.W3, PH, Wb + QW3, MH, MH);
+    copy_rows(s.W4, PH, Wb + QW4, MO, MH);
     __syncthreads();
-    for (int e = threadIdx.x; e < MO * MH; e += blockDim.x) {
-        const int o = e / MH, i = e % MH;
-        s.W4T[i * PT4 + o] = Wb[QW4 + e];
-    }
-    __syncthreads();
+    const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
     const float sc = 2.f / (3.f * (float)B);
     float lsum = 0.f;
@@ -346,11 +382,16 @@ __global__ void __launch_bounds__(SEED_TPB) k_mlp_train_bwd(int B, const bf16 *_
         float acc[16][4];
         {
             const uint32_t ay[4] = {y0, y1, 0u, 0u};
+            const bf16 *wt = s.W4 + (lane & 7) * PH + 8 * (lane >> 3);
 #pragma unroll
-            for (int nt = 0; nt < 16; nt++) {
-                acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-                const bf16 *wt = s.W4T + (8 * nt + g) * PT4 + 2 * t;
-                mma16816(acc[nt], ay, ld32(wt), 0u);
+            for (int nt = 0; nt < 16; nt += 4) {
+                uint32_t f[4];
+                ldsm4t(f, wt + 8 * nt);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    acc[nt + q][0] = acc[nt + q][1] = acc[nt + q][2] = acc[nt + q][3] = 0.f;
+                    mma16816(acc[nt + q], ay, f[q], 0u);
+                }
             }
         }
 #pragma unroll
@@ -373,16 +414,18 @@ __global__ void __launch_bounds__(SEED_TPB) k_mlp_train_bwd(int B, const bf16 *_
                 if (r1 < B) *reinterpret_cast<uint32_t *>(dZL + (size_t)r1 * MH + col) = p1;
             }
             if (L == 0) break;
-            // dH_{L-1} = dZ_L W_L  (B operand: W_L^T, rows = input index)
-            const bf16 *WT = L == 2 ? s.W3T : s.W2T;
+            // dH_{L-1} = dZ_L W_L: matrices (tile, k half) = (0,0) (0,1) (1,0) (1,1) per ldmatrix
+            const bf16 *wt = (L == 2 ? s.W3 : s.W2) + (8 * ((lane >> 3) & 1) + (lane & 7)) * PH + 8 * (lane >> 4);
 #pragma unroll
             for (int nt = 0; nt < 16; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
 #pragma unroll
             for (int ks = 0; ks < 8; ks++)
 #pragma unroll
-                for (int nt = 0; nt < 16; nt++) {
-                    const bf16 *wt = WT + (8 * nt + g) * PH + 16 * ks + 2 * t;
-                    mma16816(acc[nt], a[ks], ld32(wt), ld32(wt + 8));
+                for (int nt = 0; nt < 16; nt += 2) {
+                    uint32_t f[4];
+                    ldsm4t(f, wt + 16 * ks * PH + 8 * nt);
+                    mma16816(acc[nt], a[ks], f[0], f[1]);
+                    mma16816(acc[nt + 1], a[ks], f[2], f[3]);
                 }
         }
     }
@@ -390,103 +433,141 @@ __global__ void __launch_bounds__(SEED_TPB) k_mlp_train_bwd(int B, const bf16 *_
     if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, lsum / (3.f * (float)B));
 }
 
-// weight and bias gradients of one layer: dW[o][i] += sum_b dZ[b][o] H[b][i],
-// db[o] += sum_b dZ[b][o].  dZ [B][OUTP] BF16 (the first OUT columns used), H [B][IN]
-// BF16.  8 warps, warp w owns output rows 16w..16w+15; 64 batch rows staged per pass,
-// both operands read transposed from shared memory by ldmatrix.trans.
-template <int OUT, int OUTP, int IN>
-__global__ void __launch_bounds__(256) k_mlp_wgrad(const bf16 *__restrict__ dZ, const bf16 *__restrict__ H, int B,
-                                                    float *dW, float *db) {
-    constexpr int ZC = OUTP < 16 ? 16 : OUTP, PZ = ZC + 8, PHI = IN + 8, NT = IN / 8, MT = (OUT + 15) / 16;
-    __shared__ __align__(16) bf16 Zs[64 * PZ];
-    __shared__ __align__(16) bf16 Hs[64 * PHI];
+// Weight and bias gradients, dW[o][i] += sum_b dZ[b][o] H[b][i] and db[o] += sum_b dZ[b][o], of
+// all four layers in one launch: the blocks are split over the layers by what they read per
+// batch row (WG_BLK), each takes every n-th tile of 64 rows of its layer.  What bounds it is
+// the staging of dZ and H (26 MB at 16,384 rows) and the final atomics: tiles go to shared
+// memory by 16-byte asynchronous copies, two in flight, both operands are read transposed by
+// ldmatrix, db rides along as one more product with a tile of ones, and a layer has at most 48
+// blocks to add into its gradient, two values an atomic.  (Four launches of 256 blocks that
+// copied two bytes at a time took 95 us at 16,384 rows, this 13 us.)
+constexpr int WG_TPB = 256, WG_ROWS = 64;
+constexpr int WG_BLK[4] = {48, 48, 32, 20};             // W3, W2, W1, W4: one block per SM in all
+struct WgArgs {
+    const bf16 *X, *H, *dZ, *dY;
+    float *G;
+    int B, off[5];                                       // first block of each layer
+};
+struct WgTile { bf16 z[2][WG_ROWS * PH], h[2][WG_ROWS * PH]; };
+__device__ __forceinline__ void cp16(bf16 *dst, const bf16 *src, bool in) {
+    const int n = in ? 16 : 0;                           // 0 source bytes: zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(n));
+}
+// rows base .. base + 63 of src (C columns) into dst, zeros past B
+template <int C>
+__device__ __forceinline__ void wg_stage(bf16 *dst, const bf16 *src, int base, int B, bool vec) {
+    for (int e = threadIdx.x; e < WG_ROWS * (C / 8); e += WG_TPB) {
+        const int r = e / (C / 8), c = 8 * (e % (C / 8));
+        const bool in = base + r < B;
+        const bf16 *p = src + (size_t)(in ? base + r : 0) * C + c;
+        if (vec) cp16(dst + r * PH + c, p, in);
+        else
+            for (int q = 0; q < 8; q++) dst[r * PH + c + q] = in ? p[q] : __float2bfloat16(0.f);
+    }
+}
+__device__ __forceinline__ void add2(float *p, float x, float y, bool vec) {
+    if (vec) atomicAdd(reinterpret_cast<float2 *>(p), make_float2(x, y));
+    else { atomicAdd(p, x); atomicAdd(p + 1, y); }
+}
+// ZC: columns of dZ (8: the output layer's padded rows, of which 3 count), IN: columns of H.
+// Warp w: output rows 16 w and every column tile; the output layer: rows 0-7, two column tiles
+// a warp.
+template <int ZC, int IN>
+__device__ __forceinline__ void wgrad_layer(WgTile &sm, const bf16 *dZ, const bf16 *H, int B, int blk, int nblk,
+                                            float *dW, float *db) {
+    constexpr bool OUTL = ZC < 16;
+    constexpr int NT = OUTL ? 2 : IN / 8;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    float acc[NT][4];
+    const int m0 = OUTL ? 0 : 16 * w, n0 = OUTL ? 16 * w : 0;
+    const bool vec = al16p(dZ) && al16p(H);
+    float acc[NT][4], bs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-    float bsum = 0.f;
-    for (int base = blockIdx.x * 64; base < B; base += gridDim.x * 64) {
+    if (OUTL)                                            // columns 8-15 of the padded rows stay zero
+        for (int e = threadIdx.x; e < 2 * WG_ROWS * 8; e += WG_TPB)
+            sm.z[e / (WG_ROWS * 8)][(e / 8 % WG_ROWS) * PH + 8 + e % 8] = __float2bfloat16(0.f);
+    const int nt_all = (B + WG_ROWS - 1) / WG_ROWS;
+    auto stage = [&](int tile, int buf) {
+        if (tile < nt_all) {
+            wg_stage<ZC>(sm.z[buf], dZ, tile * WG_ROWS, B, vec);
+            wg_stage<IN>(sm.h[buf], H, tile * WG_ROWS, B, vec);
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+    stage(blk, 0);
+    int buf = 0;
+    for (int tile = blk; tile < nt_all; tile += nblk, buf ^= 1) {
+        stage(tile + nblk, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;");
         __syncthreads();
-        for (int e = threadIdx.x; e < 64 * ZC; e += blockDim.x) {
-            const int r = e / ZC, c = e % ZC;
-            Zs[r * PZ + c] = (base + r < B && c < OUTP) ? dZ[(size_t)(base + r) * OUTP + c] : __float2bfloat16(0.f);
-        }
-        for (int e = threadIdx.x; e < 64 * IN; e += blockDim.x) {
-            const int r = e / IN, c = e % IN;
-            Hs[r * PHI + c] = base + r < B ? H[(size_t)(base + r) * IN + c] : __float2bfloat16(0.f);
+        const bf16 *Zs = sm.z[buf], *Hs = sm.h[buf];
+#pragma unroll
+        for (int ks = 0; ks < WG_ROWS / 16; ks++) {
+            uint32_t a[4];
+            ldsm4t(a, Zs + (16 * ks + (lane & 7) + (lane >> 4) * 8) * PH + m0 + ((lane >> 3) & 1) * 8);
+            if (!OUTL || w == 0) mma16816(bs, a, 0x3f803f80u, 0x3f803f80u);      // BF16 ones
+#pragma unroll
+            for (int nt = 0; nt < NT; nt += 2) {
+                uint32_t f[4];
+                ldsm4t(f, Hs + (16 * ks + (lane & 7) + ((lane >> 3) & 1) * 8) * PH + n0 + 8 * nt + 8 * (lane >> 4));
+                mma16816(acc[nt], a, f[0], f[1]);
+                mma16816(acc[nt + 1], a, f[2], f[3]);
+            }
         }
         __syncthreads();
-        if (threadIdx.x < OUT)
-            for (int r = 0; r < 64; r++) bsum += __bfloat162float(Zs[r * PZ + threadIdx.x]);
-        if (w < MT) {
-            const int m0 = 16 * w;
-#pragma unroll
-            for (int ks = 0; ks < 4; ks++) {
-                const int k0 = 16 * ks;
-                uint32_t a[4];
-                {
-                    const int mi = lane >> 3, r = lane & 7;
-                    const bf16 *p = Zs + (k0 + r + (mi >> 1) * 8) * PZ + m0 + (mi & 1) * 8;
-                    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
-                                 : "r"(addr));
-                }
-#pragma unroll
-                for (int nt = 0; nt < NT; nt++) {
-                    uint32_t b0, b1;
-                    const bf16 *p = Hs + (k0 + (lane & 15)) * PHI + 8 * nt;
-                    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-                                 : "=r"(b0), "=r"(b1)
-                                 : "r"(addr));
-                    mma16816(acc[nt], a, b0, b1);
-                }
-            }
-        }
     }
-    if (threadIdx.x < OUT) atomicAdd(db + threadIdx.x, bsum);
-    if (w < MT) {
-        const int m0 = 16 * w;
+    asm volatile("cp.async.wait_group 0;");
+    if (blk >= nt_all) return;                           // nothing summed
+    const bool v2 = (reinterpret_cast<size_t>(dW) & 7) == 0;
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++) {
-            const int col = 8 * nt + 2 * t;
-            if (m0 + g < OUT) {
-                atomicAdd(dW + (m0 + g) * IN + col, acc[nt][0]);
-                atomicAdd(dW + (m0 + g) * IN + col + 1, acc[nt][1]);
-            }
-            if (m0 + g + 8 < OUT) {
-                atomicAdd(dW + (m0 + g + 8) * IN + col, acc[nt][2]);
-                atomicAdd(dW + (m0 + g + 8) * IN + col + 1, acc[nt][3]);
-            }
-        }
+    for (int nt = 0; nt < NT; nt++) {
+        const int col = n0 + 8 * nt + 2 * t;
+        if (!OUTL || g < MOUT) add2(dW + (m0 + g) * IN + col, acc[nt][0], acc[nt][1], v2);
+        if (!OUTL) add2(dW + (m0 + g + 8) * IN + col, acc[nt][2], acc[nt][3], v2);
     }
+    if (t == 0 && (!OUTL || (w == 0 && g < MOUT))) {     // every column of the ones' tile holds the sum
+        atomicAdd(db + m0 + g, bs[0]);
+        if (!OUTL) atomicAdd(db + m0 + g + 8, bs[2]);
+    }
+}
+__global__ void __launch_bounds__(WG_TPB) k_mlp_wgrad(WgArgs a) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    WgTile &sm = *reinterpret_cast<WgTile *>(smraw);
+    const size_t L = (size_t)a.B * MH;
+    const int b = blockIdx.x;
+    if (b < a.off[1]) wgrad_layer<MH, MH>(sm, a.dZ + 2 * L, a.H + L, a.B, b, a.off[1], a.G + OW3, a.G + OB3);
+    else if (b < a.off[2]) wgrad_layer<MH, MH>(sm, a.dZ + L, a.H, a.B, b - a.off[1], a.off[2] - a.off[1], a.G + OW2, a.G + OB2);
+    else if (b < a.off[3]) wgrad_layer<MH, MI>(sm, a.dZ, a.X, a.B, b - a.off[2], a.off[3] - a.off[2], a.G + OW1, a.G + OB1);
+    else wgrad_layer<MO, MH>(sm, a.dY, a.H + 2 * L, a.B, b - a.off[3], a.off[4] - a.off[3], a.G + OW4, a.G + OB4);
 }
 
 // Adam on the FP32 parameters with bias-corrected moments (c1 = 1 - b1^t, c2 = 1 - b2^t)
+// BF16 weight pack and bias vector [b1 | b2 | b3 | b4] entry of FP32 parameter i
+__device__ __forceinline__ void pack_param(int i, float v, bf16 *Wb, float *bias) {
+    if (i < OB1) Wb[QW1 + i - OW1] = __float2bfloat16(v);
+    else if (i < OW2) bias[i - OB1] = v;
+    else if (i < OB2) Wb[QW2 + i - OW2] = __float2bfloat16(v);
+    else if (i < OW3) bias[MH + i - OB2] = v;
+    else if (i < OB3) Wb[QW3 + i - OW3] = __float2bfloat16(v);
+    else if (i < OW4) bias[2 * MH + i - OB3] = v;
+    else if (i < OB4) Wb[QW4 + i - OW4] = __float2bfloat16(v);
+    else bias[3 * MH + i - OB4] = v;
+}
 __global__ void k_mlp_adam(float *P, const float *G, float *M, float *V, int n, float lr, float b1, float b2, float eps,
-                           float c1, float c2) {
+                           float c1, float c2, bf16 *Wb, float *bias) {
     SS_GRID_LOOP(i, n) {
         const float gr = G[i];
         const float m = b1 * M[i] + (1.f - b1) * gr, v = b2 * V[i] + (1.f - b2) * gr * gr;
         M[i] = m;
         V[i] = v;
-        P[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+        const float p = P[i] - lr * (m / c1) / (sqrtf(v / c2) + eps);
+        P[i] = p;
+        pack_param(i, p, Wb, bias);
     }
 }
-// BF16 weight pack + bias vector [b1 | b2 | b3 | b4] of an FP32 parameter vector
 __global__ void k_mlp_pack(const float *P, bf16 *Wb, float *bias) {
-    SS_GRID_LOOP(i, NPARAM) {
-        const float v = P[i];
-        if (i < OB1) Wb[QW1 + i - OW1] = __float2bfloat16(v);
-        else if (i < OW2) bias[i - OB1] = v;
-        else if (i < OB2) Wb[QW2 + i - OW2] = __float2bfloat16(v);
-        else if (i < OW3) bias[MH + i - OB2] = v;
-        else if (i < OB3) Wb[QW3 + i - OW3] = __float2bfloat16(v);
-        else if (i < OW4) bias[2 * MH + i - OB3] = v;
-        else if (i < OB4) Wb[QW4 + i - OW4] = __float2bfloat16(v);
-        else bias[3 * MH + i - OB4] = v;
-    }
+    SS_GRID_LOOP(i, NPARAM) pack_param(i, P[i], Wb, bias);
 }
 
 static size_t seed_smem() { return sizeof(MlpSmem) + (size_t)SEED_ROWS * P1 * sizeof(bf16); }
@@ -497,6 +578,7 @@ static void mlp_attrs() {
     cudaFuncSetAttribute(k_mlp_seed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inf_smem());
     cudaFuncSetAttribute(k_mlp_train_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seed_smem());
     cudaFuncSetAttribute(k_mlp_train_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmemT));
+    cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WgTile));
     g_mlp_attr = true;
 }
 
@@ -615,14 +697,13 @@ int b200m_mlp_backward(const void *X, int B, const void *Wb, const float *Y, con
     int nb = (B + SEED_ROWS - 1) / SEED_ROWS;
     if (nb > 1184) nb = 1184;
     k_mlp_train_bwd<<<nb, SEED_TPB, sizeof(MlpSmemT), st>>>(B, (const bf16 *)Wb, Y, T, Z, (bf16 *)dZ, (bf16 *)dY, loss);
-    const bf16 *Hb = (const bf16 *)H, *dZb = (const bf16 *)dZ;
-    const size_t L = (size_t)B * MH;
-    int ng = (B + 63) / 64;
-    if (ng > 296) ng = 296;
-    k_mlp_wgrad<MH, MH, MI><<<ng, 256, 0, st>>>(dZb, (const bf16 *)X, B, G + OW1, G + OB1);
-    k_mlp_wgrad<MH, MH, MH><<<ng, 256, 0, st>>>(dZb + L, Hb, B, G + OW2, G + OB2);
-    k_mlp_wgrad<MH, MH, MH><<<ng, 256, 0, st>>>(dZb + 2 * L, Hb + L, B, G + OW3, G + OB3);
-    k_mlp_wgrad<MOUT, MO, MH><<<ng, 256, 0, st>>>((const bf16 *)dY, Hb + 2 * L, B, G + OW4, G + OB4);
+    WgArgs a{};
+    a.X = (const bf16 *)X; a.H = (const bf16 *)H; a.dZ = (const bf16 *)dZ; a.dY = (const bf16 *)dY;
+    a.G = G;
+    a.B = B;
+    const int tiles = (B + WG_ROWS - 1) / WG_ROWS;
+    for (int l = 0; l < 4; l++) a.off[l + 1] = a.off[l] + (tiles < WG_BLK[l] ? tiles : WG_BLK[l]);
+    if (a.off[4] > 0) k_mlp_wgrad<<<a.off[4], WG_TPB, sizeof(WgTile), st>>>(a);
     return cudaGetLastError() == cudaSuccess ? 1 : 0;
 }
 // one Adam step (t >= 1) on P with gradient G and moments M, V; then the BF16 pack and
@@ -631,8 +712,7 @@ int b200m_mlp_adam(float *P, const float *G, float *M, float *V, float lr, int t
     cudaStream_t st = (cudaStream_t)stream;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
-    k_mlp_adam<<<64, 256, 0, st>>>(P, G, M, V, NPARAM, lr, b1, b2, 1e-8f, c1, c2);
-    k_mlp_pack<<<64, 256, 0, st>>>(P, (bf16 *)Wb, bias);
+    k_mlp_adam<<<(NPARAM + 255) / 256, 256, 0, st>>>(P, G, M, V, NPARAM, lr, b1, b2, 1e-8f, c1, c2, (bf16 *)Wb, bias);
     return cudaGetLastError() == cudaSuccess ? 1 : 0;
 }
 int b200m_mlp_sizes(int *nparam, int *nwb, int *nbias) {

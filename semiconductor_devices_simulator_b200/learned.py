@@ -128,7 +128,8 @@ class Trainer:
         self.P = torch.tensor(P0, **f32)
         self.M = torch.zeros(self.nparam, **f32)
         self.V = torch.zeros(self.nparam, **f32)
-        self.G = torch.zeros(self.nparam, **f32)
+        self.GL = torch.zeros(self.nparam + 1, **f32)      # gradient and loss: zeroed together
+        self.G, self.loss = self.GL[:-1], self.GL[-1:]
         self.Wb = torch.zeros(nw.value, dtype=torch.bfloat16, device=dev)
         self.bias = torch.zeros(nb.value, **f32)
         B = batch
@@ -137,7 +138,6 @@ class Trainer:
         self.H = torch.zeros((3, B, MH), dtype=torch.bfloat16, device=dev)
         self.dZ = torch.zeros((3, B, MH), dtype=torch.bfloat16, device=dev)
         self.dY = torch.zeros((B, MO), dtype=torch.bfloat16, device=dev)
-        self.loss = torch.zeros(1, **f32)
         self.t = 0
         self._check(lib.b200m_mlp_pack(_ptr(self.P), _ptr(self.Wb), _ptr(self.bias), _stream(torch)))
 
@@ -150,8 +150,7 @@ class Trainer:
         """Loss and gradient (in self.G) of a batch of exactly `batch` rows."""
         lib, torch = self.lib, self.torch
         st = _stream(torch)
-        self.G.zero_()
-        self.loss.zero_()
+        self.GL.zero_()
         B = X.shape[0]
         self._check(lib.b200m_mlp_forward(_ptr(X), B, _ptr(self.Wb), _ptr(self.bias), _ptr(self.Y), _ptr(self.Z),
                                           _ptr(self.H), st))
