@@ -585,7 +585,8 @@ void vcycle(Inst &d, const Ctx &c, int L, const double *b, double *x, const doub
     SS_LAUNCH(PF_RESID_RESTRICT, cv.N, k_gmg_restrict, grid_for(cv.N), TPB, c.st, v, cv.N, v.r, cv.b,
               L == 0 ? w : nullptr);
     vcycle(d, c, L + 1, cv.b, cv.x, w, false);
-    SS_LAUNCH(PF_PROLONG, v.N, k_gmg_prolong, grid_for(v.N), TPB, c.st, v, cv.x, x, g_knobs.mg_alpha);
+    SS_LAUNCH(PF_PROLONG, v.N, k_gmg_prolong, grid_for(v.N), TPB, c.st, v, cv.x, x,
+              w ? g_knobs.mg_alpha : g_knobs.mg_alpha * MG_OVER);
     matvec_L(c, v, x, b, v.r);                            // post-smoothing
     ilu_apply(d, c, L, v.r, v.r);
     SS_LAUNCH(PF_PROLONG, v.N, k_gmg_add, grid_for(v.N), TPB, c.st, v.N, x, v.r);

@@ -1007,7 +1007,7 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
     a.ilu_only = ilu_only ? 1 : 0;
     a.qsign = qsign;
     a.onecl = cluster ? 1 : 0;
-    a.alpha = g_knobs.mg_alpha;
+    a.alpha = kind ? g_knobs.mg_alpha : g_knobs.mg_alpha * MG_OVER;
     a.rtol = rtol;
     a.atol = atol;
     const DevP *dp = c.dP;

@@ -405,7 +405,8 @@ __global__ void __launch_bounds__(SMALL_TPB) k_vcycle_smem(const DevP *__restric
 }
 
 int g_small_nodes = 2048;           // levels at or below this size run in the cluster kernel
-int g_l0_sweeps = 2;                // red-black applications per smoothing step on the finest level
+int g_l0_sweeps = 2;                // red-black applications per smoothing step on the finest level (BiCGSTAB;
+                                    //   PCG takes one, see MG_OVER)
 int g_deep_levels = 1;              // levels (from the finest) that get the second application
 static int g_cluster = 0;           // CTAs per cluster of the small-level kernel (set on first use)
 static size_t g_smem_max = 0;       // dynamic shared memory of the shared-memory small-level kernel (0: off)
@@ -557,26 +558,27 @@ static void vcycle_t(const Ctx &c, const MGHost &mg, int bsel, int xsel, int wse
     }
     size_t smem = 0;
     const int Ls = small_plan<T>(c, mg, &smem);
+    const double alpha = wsel ? mg.alpha : mg.alpha * MG_OVER;      // wsel 0: Poisson
     for (int L = 0; L < Ls; L++) {
         SS_LAUNCH_PDL(SB, mg.maxN[L], smooth_fn<T>(0, 1), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
         SS_LAUNCH_PDL(SR, mg.maxN[L], smooth_fn<T>(0, 0), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
-        if (L < g_deep_levels && g_l0_sweeps > 1) {     // second application (finest levels)
+        if (L < g_deep_levels && g_l0_sweeps > 1 && wsel) {   // second application (finest levels, continuity)
             SS_LAUNCH_PDL(SB, mg.maxN[L], smooth_fn<T>(2, 1), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
             SS_LAUNCH_PDL(SR, mg.maxN[L], smooth_fn<T>(2, 0), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
         }
         SS_LAUNCH_PDL(pf<T>(PF_RESID_RESTRICT), mg.maxN[L], k_resid_restrict2<T>, grid_rr(c, L, mg), block_rr(c), c.st, c.dP, L, bsel,
                   xsel, wsel, gate);
     }
-    if (smem) launch_smem<T>(c, mg.maxN[Ls], Ls, mg.alpha, gate, smem);
-    else launch_small<T>(c, mg.maxN[Ls], Ls, bsel, xsel, wsel, mg.alpha, gate);
+    if (smem) launch_smem<T>(c, mg.maxN[Ls], Ls, alpha, gate, smem);
+    else launch_small<T>(c, mg.maxN[Ls], Ls, bsel, xsel, wsel, alpha, gate);
     for (int L = Ls - 1; L >= 0; L--) {
         SS_LAUNCH_PDL(pf<T>(PF_PROLONG), mg.maxN[L], k_prolong<T>, grid_full(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel,
-                  mg.alpha, gate);
+                  alpha, gate);
         SS_LAUNCH_PDL(pf<T>(PF_LEVEL_RESID), mg.maxN[L], k_level_resid<T>, grid_full(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel,
                   xsel, gate);
         SS_LAUNCH_PDL(SB, mg.maxN[L], smooth_fn<T>(1, 1), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
         SS_LAUNCH_PDL(SR, mg.maxN[L], smooth_fn<T>(1, 0), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
-        if (L < g_deep_levels && g_l0_sweeps > 1) {
+        if (L < g_deep_levels && g_l0_sweeps > 1 && wsel) {
             SS_LAUNCH_PDL(SB, mg.maxN[L], smooth_fn<T>(2, 1), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
             SS_LAUNCH_PDL(SR, mg.maxN[L], smooth_fn<T>(2, 0), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
         }

@@ -1517,8 +1517,8 @@ int persist_pcg(const Ctx &c, const MGHost &mg, int mixed) {
     if (a.Ls < 1) return 0;
     a.qsign = 0;
     a.deep = g_deep_levels;
-    a.sweeps2 = g_l0_sweeps > 1;
-    a.alpha = mg.alpha;
+    a.sweeps2 = 0;                              // one application (MG_OVER, solver_ctx.h)
+    a.alpha = mg.alpha * MG_OVER;
     a.barmode = g_barmode;
     PGrid h{};
     const int rc = mixed ? persist_run<float, PK_PCG>(c, a.Ls, smem, a, &h)
