@@ -23,6 +23,7 @@ constexpr int K_SEMI = 0, K_INS = 1, K_METAL = 2;
 constexpr int TPB = 256;            // threads per block of the node kernels
 constexpr int RED_MAX_BLOCKS = 2048; // grid cap of reducing kernels (partials per instance)
 constexpr int RED_NV = 16;          // doubles per block partial record
+constexpr int RED_AA = 24;          // ... of the Anderson pass (2 AA_MAX sums)
 constexpr int COARSE_MAX = 64;      // unknowns of the coarsest multigrid level
 constexpr int ION_W = 4;            // doubles per node of the ionisation constants
 
@@ -202,7 +203,7 @@ struct DevP {
     double *gram;                 // AA_MAX*AA_MAX
     double *aagam;                // AA_MAX coefficients
     // reductions
-    double *part;                 // RED_MAX_BLOCKS*RED_NV
+    double *part;                 // RED_MAX_BLOCKS*RED_AA
     unsigned *ticket;             // one counter per reduction slot (16)
     double *partc;                // terminal-current partials: 256 blocks x 96
     double *ffbuf;                // floating-block sums: 6 x 1024

@@ -120,7 +120,7 @@ static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &lev
     P.aaG = cv.take<float>((size_t)AA_MAX * 3 * N);
     P.aaf = cv.take<double>(3 * N); P.aag = cv.take<double>(3 * N);
     P.gram = cv.take<double>(AA_MAX * AA_MAX); P.aagam = cv.take<double>(AA_MAX);
-    P.part = cv.take<double>((size_t)RED_MAX_BLOCKS * RED_NV);
+    P.part = cv.take<double>((size_t)RED_MAX_BLOCKS * RED_AA);
     P.ticket = cv.take<unsigned>(16);
     P.partc = cv.take<double>(256 * 96);
     P.ffbuf = cv.take<double>(6 * 1024);
@@ -1619,17 +1619,14 @@ static void aa_reset(Inst &d) { d.aa_n = 0; d.aa_pos = 0; d.aa_have = 0; }
 static void aa_step(Inst &d) {                      // semiconductor_3d.c:3709-3757
     Ctx c = make_ctx(d);
     const int M = d.aa_m < g_knobs.aa_depth ? d.aa_m : g_knobs.aa_depth;
+    int slot = 0;
     if (M > 0 && d.aa_have) {
-        const int s = d.aa_pos;
+        slot = d.aa_pos;
         if (d.aa_n < M) d.aa_n++;
-        aa_update_history(c, s, d.aa_n);
-        d.aa_pos = (s + 1) % M;
+        d.aa_pos = (slot + 1) % M;
     }
-    aa_store_fg(c);
+    aa_pass(c, slot, d.aa_n);
     d.aa_have = 1;
-    const int m = d.aa_n;
-    if (m == 0) return;
-    aa_solve_mix(c, m, nullptr);
 }
 
 // ------------------------------------------------------------------ Gummel

@@ -308,8 +308,7 @@ void launch_fill_sel(const Ctx &c, int ysel, double v);
 void launch_copy_sel(const Ctx &c, int ysel, int xsel);
 
 // Anderson (kernels_aa.cu)
-void aa_update_history(const Ctx &c, int slot, int nfill);
-void aa_store_fg(const Ctx &c);
-void aa_solve_mix(const Ctx &c, int m, int *ok_host);
+// store f and g; with m > 0 columns also the new history column `slot` and the mix
+void aa_pass(const Ctx &c, int slot, int m);
 
 }  // namespace ss
