@@ -132,6 +132,18 @@ __device__ __forceinline__ double bern(double x) {
     return x / expm1(x);
 }
 
+// B(x) and B(-x) from one expm1: B(|x|) is the small one, and B(-|x|) = B(|x|) + |x| adds
+// positive terms only (the difference the other way round would cancel)
+__device__ __forceinline__ void bern2(double x, double &bp, double &bm) {
+    const double a = fabs(x);
+    double s;
+    if (a < 1e-6) s = 1.0 - a / 2.0 + a * a / 12.0;
+    else s = a > 700.0 ? 0.0 : a / expm1(a);
+    const double l = s + a;
+    bp = x < 0.0 ? l : s;
+    bm = x < 0.0 ? s : l;
+}
+
 struct Node {
     int i, j, l;
 };
@@ -156,6 +168,33 @@ __device__ __forceinline__ bool nbr(const DevP &P, const Node &a, int k, int dir
     case 4: if (a.l == 0) return false; kb = k - P.Nx * P.Ny; h = P.zs[a.l] - P.zs[a.l - 1]; ar = P.Lx[a.i] * P.Ly[a.j]; return true;
     default: if (a.l == P.Nz - 1) return false; kb = k + P.Nx * P.Ny; h = P.zs[a.l + 1] - P.zs[a.l]; ar = P.Lx[a.i] * P.Ly[a.j]; return true;
     }
+}
+
+// The six neighbours of node k in the order of nbr(), for kernels that load them all at once
+// (loads behind one another's branches are waited for one by one): a missing neighbour is k
+// itself, `ok` says which exist; the area over spacing of the dual faces from the reciprocal
+// spacings
+struct Nbr6 {
+    int kb[6];
+    bool ok[6];
+};
+__device__ __forceinline__ Nbr6 nbr6(const DevP &P, const Node &a, int k) {
+    Nbr6 n;
+    const int NxNy = P.Nx * P.Ny;
+    n.ok[0] = a.i > 0; n.ok[1] = a.i < P.Nx - 1; n.ok[2] = a.j > 0; n.ok[3] = a.j < P.Ny - 1;
+    n.ok[4] = a.l > 0; n.ok[5] = a.l < P.Nz - 1;
+    n.kb[0] = n.ok[0] ? k - 1 : k; n.kb[1] = n.ok[1] ? k + 1 : k;
+    n.kb[2] = n.ok[2] ? k - P.Nx : k; n.kb[3] = n.ok[3] ? k + P.Nx : k;
+    n.kb[4] = n.ok[4] ? k - NxNy : k; n.kb[5] = n.ok[5] ? k + NxNy : k;
+    return n;
+}
+__device__ __forceinline__ void area_over_h(const DevP &P, const Node &a, double (&g)[6], double &vol) {
+    const double lx = P.Lx[a.i], ly = P.Ly[a.j], lz = P.Lz[a.l];
+    const double x0 = P.ihx[a.i > 0 ? a.i - 1 : 0], x1 = P.ihx[a.i], y0 = P.ihy[a.j > 0 ? a.j - 1 : 0], y1 = P.ihy[a.j],
+                 z0 = P.ihz[a.l > 0 ? a.l - 1 : 0], z1 = P.ihz[a.l];
+    const double ax = ly * lz, ay = lx * lz, az = lx * ly;
+    g[0] = ax * x0; g[1] = ax * x1; g[2] = ay * y0; g[3] = ay * y1; g[4] = az * z0; g[5] = az * z1;
+    vol = lx * ax;
 }
 
 __device__ __forceinline__ double bgn_of(const DevP &P, int k) { return P.bgn ? P.bgn[k] : 0.0; }

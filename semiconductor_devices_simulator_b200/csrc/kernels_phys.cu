@@ -13,6 +13,16 @@
 
 namespace ss {
 
+// The node kernels of this file are bound by the latency of their loads: all loads of a row are
+// issued before the first branch (nbr6, area_over_h), and the register limits keep several
+// blocks on an SM. Measured at 576k / 1.9M nodes, before -> now: k_poisson 63 / 188 us ->
+// 36 / 84 (3.0 TB/s), k_cont_assemble 100 / 356 -> 51 / 149 (2.4 TB/s), k_cont_update 52 / 145
+// -> 24 / 49 (3.6 TB/s), k_upd_mob 101 / 313 -> 77 / 215 (bound by its FP64 pow calls).
+// Blocks per SM, 1.9M nodes: k_poisson 2: 117 us, 3: 101, 4: 84, 5: 105 (spills);
+// k_cont_assemble 1: 233, 2: 149, 3: 199 (spills); k_upd_mob 1: 300, 3: 245, 4: 215, 8: 245.
+constexpr int PO_BLK = 4, CA_BLK = 2, MO_BLK = 4;
+
+
 int Ctx::nodes_blocks() const {
     int b = (maxN + TPB - 1) / TPB;
     if (b > grid_cap) b = grid_cap;
@@ -27,7 +37,7 @@ static inline dim3 grid_of(const Ctx &c) { return dim3(c.nodes_blocks(), c.ninst
 // Jacobian (-dF/dpsi) as a 7-point stencil and ||F/diag|| (semiconductor_3d.c:2732-2789).
 // src: 0 psi = P.phi, 1 psi = P.tr.  build: write A, sc and F into rhs; else F into P.F
 // and the norm uses the sc of the last build (as the reference's line search does).
-__global__ void k_poisson(const DevP *__restrict__ Ps, int src, int build) {
+__global__ void __launch_bounds__(TPB, PO_BLK) k_poisson(const DevP *__restrict__ Ps, int src, int build) {
     const DevP &P = Ps[blockIdx.y];
     const double *phi = src ? P.tr : P.phi;
     double *F = build ? P.rhs : P.F;
@@ -45,22 +55,27 @@ __global__ void k_poisson(const DevP *__restrict__ Ps, int src, int build) {
             continue;
         }
         const Node a = unidx(k, P.Nx, P.Ny);
+        const Nbr6 nb = nbr6(P, a, k);
+        uint32_t fb[6];
+        double pb[6], gh[6], vol;
+#pragma unroll
+        for (int dir = 0; dir < 6; dir++) { fb[dir] = P.flags[nb.kb[dir]]; pb[dir] = phi[nb.kb[dir]]; }
+        area_over_h(P, a, gh, vol);
         const MatD &m = P.mats[fl_mat(f)];
         const double ek = m.eps, pk = phi[k];
         double fk = 0.0, dg = 0.0, off[6];
 #pragma unroll
         for (int dir = 0; dir < 6; dir++) {
-            int kb; double h, ar;
-            off[dir] = 0.0;
-            if (!nbr(P, a, k, dir, kb, h, ar)) continue;
-            const uint32_t fb = P.flags[kb];
-            const double eb = P.mats[fl_mat(fb)].eps;
-            const double cf = (2.0 * ek * eb / (ek + eb)) * ar / h;
-            fk += cf * (phi[kb] - pk);
+            double cf = ek;                       // the faces' permittivity: harmonic mean
+            if (fl_mat(fb[dir]) != fl_mat(f)) {
+                const double eb = P.mats[fl_mat(fb[dir])].eps;
+                cf = 2.0 * ek * eb / (ek + eb);
+            }
+            cf = nb.ok[dir] ? cf * gh[dir] : 0.0;
+            fk += cf * (pb[dir] - pk);
             dg += cf;
-            if (!fl_con(fb)) off[dir] = -cf;
+            off[dir] = fl_con(fb[dir]) ? 0.0 : -cf;
         }
-        const double vol = P.Lx[a.i] * P.Ly[a.j] * P.Lz[a.l];
         if (fl_kind(f) == K_SEMI) {
             const double n = nK(P, m, k, pk, P.phin[k]), p = pK(P, m, k, pk, P.phip[k]);
             if (ion_node(P, k)) {                 // incompletely ionised dopants
@@ -125,10 +140,6 @@ __global__ void k_rebuild_np(const DevP *__restrict__ Ps) {
 }
 void launch_rebuild_np(const Ctx &c) { SS_LAUNCH(PF_REBUILD, c.maxN, k_rebuild_np, grid_of(c), TPB, c.st, c.dP); }
 
-// Face mobility of the edge k -> k+e_ax from the node low-field mobilities, with
-// Caughey-Thomas saturation driven by the harmonic-mean field when models bit 2 is set
-// (semiconductor_3d.c:2962-3006), and Lombardi surface scattering near insulator / gate walls
-// when models bit 4 is set (the Coulomb term of 4H-SiC is not built).
 // potential gradient along ax taken inside the semiconductor (one-sided at an interface,
 // semiconductor_3d.c:2909-2917)
 __device__ __forceinline__ double grad_semi(const DevP &P, const Node &a, int k, int ax) {
@@ -147,70 +158,74 @@ __device__ __forceinline__ double fnorm2(const DevP &P, const Node &a, int k, in
     return g1 * g1 + g2 * g2;
 }
 
-__global__ void k_upd_mob(const DevP *__restrict__ Ps) {
+// Face mobility of the edge k -> k+e_ax from the node low-field mobilities, with
+// Caughey-Thomas saturation driven by the harmonic-mean field when models bit 2 is set
+// (semiconductor_3d.c:2962-3006), and Lombardi surface scattering near insulator / gate walls
+// when models bit 4 is set. One thread per edge (blockIdx.z is the axis): a third of the
+// serial pow chain of a thread per node, in 64 registers instead of 154.
+__global__ void __launch_bounds__(TPB, MO_BLK) k_upd_mob(const DevP *__restrict__ Ps) {
     const DevP &P = Ps[blockIdx.y];
+    const int ax = blockIdx.z;
     const bool sat = (P.models & 4) != 0, lb = (P.models & 16) != 0;
     SS_GRID_LOOP(k, P.N) {
-        const uint32_t f = P.flags[k];
         const Node a = unidx(k, P.Nx, P.Ny);
-#pragma unroll
-        for (int ax = 0; ax < 3; ax++) {
-            int kp; double h, ar;
-            if (fl_kind(f) != K_SEMI || !nbr(P, a, k, 2 * ax + 1, kp, h, ar) || fl_kind(P.flags[kp]) != K_SEMI) {
-                P.fmu[ax][k] = 0.0; P.fmu[3 + ax][k] = 0.0;
-                continue;
-            }
-            const MatD &m = P.mats[fl_mat(f)];
-            double mn = 0.5 * (P.mu0n[k] + P.mu0n[kp]), mp = 0.5 * (P.mu0p[k] + P.mu0p[kp]);
-            if (ax == P.caxis) {
-                if (m.ani_n > 0.0) mn *= m.ani_n;
-                if (m.ani_p > 0.0) mp *= m.ani_p;
-            }
-            if (lb && m.lb_on) {
-                const double Dw = exp(-0.5 * (P.qd[k] + P.qd[kp]) / 1e-8);
-                if (Dw > 1e-8) {
-                    Node b = a;
-                    if (ax == 0) b.i++; else if (ax == 1) b.j++; else b.l++;
-                    const double F = sqrt(0.5 * (fnorm2(P, a, k, ax) + fnorm2(P, b, kp, ax)));
-                    const double Nt = 0.5 * (P.Nd[k] + P.Na[k] + P.Nd[kp] + P.Na[kp]);
-                    double ic = 0.0;
-                    if (P.if_NC && m.lbc_on) {          // Coulomb scattering, n from the reference levels
-                        const double nn = 0.5 * (nK(P, m, k, P.phi[k], P.phin[k]) +
-                                                 nK(P, P.mats[fl_mat(P.flags[kp])], kp, P.phi[kp], P.phin[kp]));
-                        const int ea = P.qi[k], eb = P.qi[kp];
-                        const double NC = ea >= 0 && eb >= 0 ? 0.5 * (P.if_NC[ea] + P.if_NC[eb])
-                                        : (ea >= 0 ? P.if_NC[ea] : (eb >= 0 ? P.if_NC[eb] : 0.0));
-                        ic = coul_inv(m, F, nn, NC, 0.5 * (P.Na[k] + P.Na[kp]));
-                    }
-                    if (m.lb_on & 1) mn = lombardi(m, mn, F, Nt, Dw, 0, ic);
-                    if (m.lb_on & 2) mp = lombardi(m, mp, F, Nt, Dw, 1, 0.0);
-                }
-            }
-            // velocity saturation, tapered off across the barrier region of a metal contact
-            // (te_vsat_w, semiconductor_3d.c:810-824)
-            double wv = 0.0;
-            if (sat) {
-                wv = 1.0;
-                if (P.te_vw) {
-                    auto node_w = [&](int kk) {
-                        const double w = P.te_vw[kk];
-                        if (w >= 1.0) return 1.0;
-                        const double c2 = P.te_ax[kk] == ax ? 1.0 : 0.0;
-                        return 1.0 - (1.0 - w) * c2;
-                    };
-                    wv = 0.5 * (node_w(k) + node_w(kp));
-                }
-            }
-            if (wv > 0.0) {
-                const double dps = P.phi[kp] - P.phi[k];
-                const double Fn = heat_field(P.phin[kp] - P.phin[k], dps, h);
-                const double Fp = heat_field(P.phip[kp] - P.phip[k], dps, h);
-                const double sn = mob_hf(mn, Fn, m.vsat_n, m.beta_n), sp = mob_hf(mp, Fp, m.vsat_p, m.beta_p);
-                mn += wv * (sn - mn);
-                mp += wv * (sp - mp);
-            }
-            P.fmu[ax][k] = mn; P.fmu[3 + ax][k] = mp;
+        const bool last = ax == 0 ? a.i == P.Nx - 1 : ax == 1 ? a.j == P.Ny - 1 : a.l == P.Nz - 1;
+        const int kp = last ? k : k + (ax == 0 ? 1 : ax == 1 ? P.Nx : P.Nx * P.Ny);
+        const uint32_t f = P.flags[k], fp = P.flags[kp];    // both ends' values, all loads at once
+        const double dps = P.phi[kp] - P.phi[k], dqn = P.phin[kp] - P.phin[k], dqp = P.phip[kp] - P.phip[k];
+        double mn = 0.5 * (P.mu0n[k] + P.mu0n[kp]), mp = 0.5 * (P.mu0p[k] + P.mu0p[kp]);
+        if (fl_kind(f) != K_SEMI || last || fl_kind(fp) != K_SEMI) {
+            P.fmu[ax][k] = 0.0; P.fmu[3 + ax][k] = 0.0;
+            continue;
         }
+        const double h = ax == 0 ? P.xs[a.i + 1] - P.xs[a.i] : ax == 1 ? P.ys[a.j + 1] - P.ys[a.j] : P.zs[a.l + 1] - P.zs[a.l];
+        const MatD &m = P.mats[fl_mat(f)];
+        if (ax == P.caxis) {
+            if (m.ani_n > 0.0) mn *= m.ani_n;
+            if (m.ani_p > 0.0) mp *= m.ani_p;
+        }
+        if (lb && m.lb_on) {
+            const double Dw = exp(-0.5 * (P.qd[k] + P.qd[kp]) / 1e-8);
+            if (Dw > 1e-8) {
+                Node b = a;
+                if (ax == 0) b.i++; else if (ax == 1) b.j++; else b.l++;
+                const double F = sqrt(0.5 * (fnorm2(P, a, k, ax) + fnorm2(P, b, kp, ax)));
+                const double Nt = 0.5 * (P.Nd[k] + P.Na[k] + P.Nd[kp] + P.Na[kp]);
+                double ic = 0.0;
+                if (P.if_NC && m.lbc_on) {          // Coulomb scattering, n from the reference levels
+                    const double nn = 0.5 * (nK(P, m, k, P.phi[k], P.phin[k]) +
+                                             nK(P, P.mats[fl_mat(P.flags[kp])], kp, P.phi[kp], P.phin[kp]));
+                    const int ea = P.qi[k], eb = P.qi[kp];
+                    const double NC = ea >= 0 && eb >= 0 ? 0.5 * (P.if_NC[ea] + P.if_NC[eb])
+                                    : (ea >= 0 ? P.if_NC[ea] : (eb >= 0 ? P.if_NC[eb] : 0.0));
+                    ic = coul_inv(m, F, nn, NC, 0.5 * (P.Na[k] + P.Na[kp]));
+                }
+                if (m.lb_on & 1) mn = lombardi(m, mn, F, Nt, Dw, 0, ic);
+                if (m.lb_on & 2) mp = lombardi(m, mp, F, Nt, Dw, 1, 0.0);
+            }
+        }
+        // velocity saturation, tapered off across the barrier region of a metal contact
+        // (te_vsat_w, semiconductor_3d.c:810-824)
+        double wv = 0.0;
+        if (sat) {
+            wv = 1.0;
+            if (P.te_vw) {
+                auto node_w = [&](int kk) {
+                    const double w = P.te_vw[kk];
+                    if (w >= 1.0) return 1.0;
+                    const double c2 = P.te_ax[kk] == ax ? 1.0 : 0.0;
+                    return 1.0 - (1.0 - w) * c2;
+                };
+                wv = 0.5 * (node_w(k) + node_w(kp));
+            }
+        }
+        if (wv > 0.0) {
+            const double Fn = heat_field(dqn, dps, h), Fp = heat_field(dqp, dps, h);
+            const double sn = mob_hf(mn, Fn, m.vsat_n, m.beta_n), sp = mob_hf(mp, Fp, m.vsat_p, m.beta_p);
+            mn += wv * (sn - mn);
+            mp += wv * (sp - mp);
+        }
+        P.fmu[ax][k] = mn; P.fmu[3 + ax][k] = mp;
     }
 }
 // N_C of every Coulomb interface entry: fixed charge plus the charged trap states of the
@@ -238,7 +253,7 @@ void launch_coul_update(const Ctx &c) {
 }
 void launch_upd_mob(const Ctx &c) {
     launch_coul_update(c);
-    SS_LAUNCH(PF_UPDMOB, c.maxN, k_upd_mob, grid_of(c), TPB, c.st, c.dP);
+    SS_LAUNCH(PF_UPDMOB, c.maxN, k_upd_mob, dim3(c.nodes_blocks(), c.ninst, 3), TPB, c.st, c.dP);
 }
 
 // ------------------------------------------------------------------ continuity
@@ -246,7 +261,7 @@ void launch_upd_mob(const Ctx &c) {
 //   electrons D = dpsi/VT + d(ln Nc_eff), self = g B(-D), nb = g B(D)
 //   holes     D = dpsi/VT - d(ln Nv_eff), self = g B(D),  nb = g B(-D)
 // linearised recombination on the diagonal, row scale 1/(diag s_k).
-__global__ void k_cont_assemble(const DevP *__restrict__ Ps, int hole) {
+__global__ void __launch_bounds__(TPB, CA_BLK) k_cont_assemble(const DevP *__restrict__ Ps, int hole) {
     const DevP &P = Ps[blockIdx.y];
     const double *car = hole ? P.p : P.n;
     SS_GRID_LOOP(k, P.N) {
@@ -262,35 +277,45 @@ __global__ void k_cont_assemble(const DevP *__restrict__ Ps, int hole) {
             continue;
         }
         const Node a = unidx(k, P.Nx, P.Ny);
+        const Nbr6 nbk = nbr6(P, a, k);
+        uint32_t fbk[6];
+        double pb[6], cb[6], mu[6], bg[6], gh[6], vol;
+#pragma unroll
+        for (int dir = 0; dir < 6; dir++) {
+            const int kb = nbk.kb[dir];
+            fbk[dir] = P.flags[kb];
+            pb[dir] = P.phi[kb];
+            cb[dir] = car[kb];
+            mu[dir] = P.fmu[(hole ? 3 : 0) + (dir >> 1)][(dir & 1) ? k : kb];    // the edge's lower node
+            bg[dir] = P.bgn ? P.bgn[kb] : 0.0;
+        }
+        area_over_h(P, a, gh, vol);
         const MatD &m = P.mats[fl_mat(f)];
-        const double VT = m.VT, sk = fmax(car[k], NFLOOR);
+        const double *qc = hole ? P.qcp : P.qcn;
+        const double VT = m.VT, iVT = 1.0 / VT, sk = fmax(car[k], NFLOOR);
         const double lk = hole ? lnvK(P, m, k) : lncK(P, m, k);
         const double pk = P.phi[k];
         double dg = 0.0, b = 0.0, off[6];
 #pragma unroll
         for (int dir = 0; dir < 6; dir++) {
-            int kb; double h, ar;
             off[dir] = 0.0;
-            if (!nbr(P, a, k, dir, kb, h, ar)) continue;
-            const uint32_t fb = P.flags[kb];
-            if (fl_kind(fb) != K_SEMI) continue;
-            const MatD &mb = P.mats[fl_mat(fb)];
-            const double lb = hole ? lnvK(P, mb, kb) : lncK(P, mb, kb);
-            const double D = (P.phi[kb] - pk) / VT + (hole ? -(lb - lk) : (lb - lk));
-            const int kl = k < kb ? k : kb;
-            const double g = ar * P.fmu[(hole ? 3 : 0) + (dir >> 1)][kl] * VT / h;
-            const double bp = bern(D), bm = bern(-D);
+            if (!nbk.ok[dir] || fl_kind(fbk[dir]) != K_SEMI) continue;
+            const MatD &mb = P.mats[fl_mat(fbk[dir])];
+            const double lb = (hole ? mb.lnv : mb.lnc) + bg[dir] + (qc ? qc[nbk.kb[dir]] : 0.0);
+            const double D = (pb[dir] - pk) * iVT + (hole ? -(lb - lk) : (lb - lk));
+            const double g = gh[dir] * mu[dir] * VT;
+            double bp, bm;
+            bern2(D, bp, bm);
             const double self = hole ? g * bp : g * bm;
             const double nb = hole ? g * bm : g * bp;
             dg += self;
-            if (fl_fix(fb)) b += nb * car[kb];
-            else off[dir] = -nb * fmax(car[kb], NFLOOR);
+            if (fl_fix(fbk[dir])) b += nb * cb[dir];
+            else off[dir] = -nb * fmax(cb[dir], NFLOOR);
         }
         double R, dRn, dRp;
         recombK(P, m, k, P.n[k], P.p[k], R, dRn, dRp);
         double dR = hole ? dRp : dRn;
         if (dR < 0.0) dR = 0.0;
-        const double vol = P.Lx[a.i] * P.Ly[a.j] * P.Lz[a.l];
         dg += vol * dR;
         b += vol * (dR * car[k] - R);
         if (P.tk) { dg += P.tk[k]; b += P.tg[k]; }   // metal-contact exchange: sink tk c - tg
@@ -317,21 +342,22 @@ __global__ void k_cont_update(const DevP *__restrict__ Ps, int hole, double lo, 
     double dmax = 0.0;
     SS_GRID_LOOP(k, P.N) {
         const uint32_t f = P.flags[k];
+        double u = P.sol[k];
+        const double sk = P.sc[k], ps = P.phi[k], q0 = qf[k], ot = oth[k], nd = P.Nd[k], na = P.Na[k];
         if (fl_kind(f) != K_SEMI || fl_fix(f)) { dq[k] = 0.0; continue; }
         const MatD &m = P.mats[fl_mat(f)];
-        double u = P.sol[k];
         if (!(u > 1e-30)) u = 1e-30;
         else if (u > 1e30) u = 1e30;
-        const double cc = P.sc[k] * u;
-        double qn = hole ? P.phi[k] + m.VT * (log(cc) - lnvK(P, m, k)) : P.phi[k] - m.VT * (log(cc) - lncK(P, m, k));
+        const double cc = sk * u, lk = hole ? lnvK(P, m, k) : lncK(P, m, k);
+        double qn = hole ? ps + m.VT * (log(cc) - lk) : ps - m.VT * (log(cc) - lk);
         if (qn < lo) qn = lo;
         else if (qn > hi) qn = hi;
-        const double ch = qn - qf[k];
+        const double ch = qn - q0;
         qf[k] = qn;
         dq[k] = ch;
-        const double cn = hole ? pK(P, m, k, P.phi[k], qn) : nK(P, m, k, P.phi[k], qn);
+        const double cn = exp(clampe(hole ? lk + (qn - ps) / m.VT : lk + (ps - qn) / m.VT));
         car[k] = cn;
-        const double scale = cn + oth[k] + fabs(P.Nd[k] - P.Na[k]);
+        const double scale = cn + ot + fabs(nd - na);
         const double r = scale > 0.0 ? cn / scale : 0.0;
         if (r > 1e-6) {
             const double w = r >= 1e-3 ? 1.0 : r * 1e3;

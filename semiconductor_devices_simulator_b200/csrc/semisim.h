@@ -147,6 +147,7 @@ struct DevP {
     int models, caxis, ncon, ref_mat;
     double VTref, Cref;
     const double *xs, *ys, *zs, *Lx, *Ly, *Lz;
+    const double *ihx, *ihy, *ihz;   // reciprocal spacings, 1 / (x[i+1] - x[i]) (0 past the last)
     const uint32_t *flags;
     const double *Nd, *Na, *Nf, *bgn, *robA;
     const double *qd;             // distance to the nearest insulator / gate wall (display)

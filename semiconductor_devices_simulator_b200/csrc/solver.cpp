@@ -99,6 +99,7 @@ static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &lev
     P.bgn = cv.take<double>(N); P.robA = cv.take<double>(N); P.qd = cv.take<double>(N);
     P.xs = cv.take<double>(d.Nx); P.ys = cv.take<double>(d.Ny); P.zs = cv.take<double>(d.Nz);
     P.Lx = cv.take<double>(d.Nx); P.Ly = cv.take<double>(d.Ny); P.Lz = cv.take<double>(d.Nz);
+    P.ihx = cv.take<double>(d.Nx); P.ihy = cv.take<double>(d.Ny); P.ihz = cv.take<double>(d.Nz);
     P.mats = cv.take<MatD>(NM_MAX);
     P.cons = cv.take<ConD>(NC_MAX);
     P.cnode = cv.take<int>(N > 0 ? N : 1);
@@ -1448,6 +1449,16 @@ int prepare(Inst &d) {
     CK(cudaMemcpyAsync((void *)P.Lx, d.Lx.data(), d.Nx * 8, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync((void *)P.Ly, d.Ly.data(), d.Ny * 8, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync((void *)P.Lz, d.Lz.data(), d.Nz * 8, cudaMemcpyHostToDevice, st));
+    std::vector<double> ih[3];
+    if (!d.unstr) {
+        const std::vector<double> *cs[3] = {&d.xs, &d.ys, &d.zs};
+        const double *to[3] = {P.ihx, P.ihy, P.ihz};
+        for (int q = 0; q < 3; q++) {
+            ih[q].assign(cs[q]->size(), 0.);
+            for (size_t i = 0; i + 1 < cs[q]->size(); i++) ih[q][i] = 1. / ((*cs[q])[i + 1] - (*cs[q])[i]);
+            CK(cudaMemcpyAsync((void *)to[q], ih[q].data(), ih[q].size() * 8, cudaMemcpyHostToDevice, st));
+        }
+    }
     if (want_ion)
         CK(cudaMemcpyAsync(d.g.ion, ionx.data(), ionx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d.g.d, &P, sizeof(DevP), cudaMemcpyHostToDevice, st));
