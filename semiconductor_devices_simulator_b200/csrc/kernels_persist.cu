@@ -55,6 +55,11 @@
 #define PG_PASS __forceinline__
 #endif
 
+// the set-up functions are shared by the large levels and block 0's small ones: code met for
+// the first time in a launch is fetched from L2 line by line (the small levels' own inlined
+// copies took 5 us each there, 0.7 us warm)
+#define PG_SETUP __noinline__
+
 namespace ss {
 
 // 512 threads of 128 registers: with 1024 of 64 the half sweeps' operands spilled to local
@@ -132,7 +137,8 @@ template <class T>
 struct PTab {
     SWork<T> w;
     SLev<T> sv[MAXLEV];          // block 0: the levels it keeps in shared memory (index L - Ls)
-    int slot[COARSE_MAX];        // block 0: the coarsest level's slots in the order of its dense inverse
+    int slot[COARSE_MAX];        // block 0: the coarsest level's slots in the order of its dense inverse's rows
+    int cslot[COARSE_MAX];       // and in the order of its columns
     SLev<T> cur0;                // level 0 with the running V-cycle's b and x
     const double *A64;           // the FP64 level-0 operator in natural order (coupling q at A64 + q * ap64 + k)
     int ap64;
@@ -384,13 +390,13 @@ __device__ __noinline__ void blk_cycle(const PTab<T> &tb, int Ls, int nl, T al, 
     if (L == nl - 1) {                            // coarsest level: x = inverse b, 8 lanes per row
         const SLev<T> &v = sv[nl - 1 - Ls];
         const int n = v.N, q0 = tid & 7;
-        const int *slot = tb.slot;
+        const int *slot = tb.slot, *cslot = tb.cslot;
         if (tid < v.nt) {
             for (int r = tid >> 3; r < ((n + 3) & ~3); r += v.nt >> 3) {
                 T sum = 0;
                 if (r < n) {
 #pragma unroll 4
-                    for (int q = q0; q < n; q += 8) sum += v.D[r * n + q] * v.b[slot[q]];
+                    for (int q = q0; q < n; q += 8) sum += v.D[r * n + q] * v.b[cslot[q]];
                 }
                 sum += __shfl_xor_sync(0xffffffffu, sum, 1);
                 sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -782,7 +788,7 @@ __device__ __forceinline__ void pg_load(const DevP &P, const PTab<T> &tb, const 
 // as the reference guards its ILU pivots (semiconductor_3d.c:1937-1938); the red ones, 1 / a_rr,
 // are written with the operator
 template <class T>
-__device__ __forceinline__ void pg_pivots(const SLev<T> &vr, int tid, int nth) {
+__device__ PG_SETUP void pg_pivots(const SLev<T> &vr, int tid, int nth) {
     const SLev<T> v = vr;
     for (int u = tid; u < v.H; u += nth) {
         const Pair p = slot_row(v, u);
@@ -808,7 +814,7 @@ __device__ __forceinline__ void pg_pivots(const SLev<T> &vr, int tid, int nth) {
 // potentials (semiconductor_3d.c:2092-2117); thread per coarse node.  phf / phc: the levels'
 // reference potentials in natural order (phf null: level 0, from the state)
 template <class T>
-__device__ __forceinline__ void pg_weights(const DevP &P, const SLev<T> &f, const SLev<T> &cl, const double *phf,
+__device__ PG_SETUP void pg_weights(const DevP &P, const SLev<T> &f, const SLev<T> &cl, const double *phf,
                                            double *phc, int qsign, int tid, int nth) {
     for (int K = tid; K < cl.N; K += nth) {
         const Node c = unidx(K, cl.Nx, cl.Ny);
@@ -839,7 +845,7 @@ __device__ __forceinline__ void pg_weights(const DevP &P, const SLev<T> &f, cons
 // Petrov-Galerkin coarse operator P^T W A P (semiconductor_3d.c:2003-2027), summed in FP64:
 // lanes as in pg_restrict, each lane the two nodes of one of the aggregate's rows
 template <class T>
-__device__ __forceinline__ void pg_galerkin(const SLev<T> &fr, const SLev<T> &clr, const T *w, int tid, int nth) {
+__device__ PG_SETUP void pg_galerkin(const SLev<T> &fr, const SLev<T> &clr, const T *w, int tid, int nth) {
     const SLev<T> f = fr, cl = clr;
     const int lane = tid & 31, sub = lane >> 3, dj = sub & 1, dl = sub >> 1;
     const int ng = cl.n8 * cl.Ny * cl.Nz, nw = nth >> 5;
@@ -899,87 +905,107 @@ __device__ __forceinline__ void pg_galerkin(const SLev<T> &fr, const SLev<T> &cl
     }
 }
 // Dense inverse of the coarsest level (n <= 64) by Gauss-Jordan with partial pivoting in FP64
-// (tiny pivots guarded as semiconductor_3d.c:2066 does), by the first 8 n threads: 8 lanes
-// hold a row in registers, rows are never moved (row piv[c] plays row c), and per column the
-// lanes exchange the column and the pivot row through shared memory (two barriers of those
-// warps).  For 24 unknowns 19 us, a matrix in shared memory with row swaps 29 us, a thread per
-// row with a serial pivot search 50 us.
-template <class T>
-__device__ __noinline__ void blk_invert(const SLev<T> &v) {
-    __shared__ double col[2][COARSE_MAX], prow[2][COARSE_MAX];
-    __shared__ int piv[COARSE_MAX];
-    const int n = v.N, nt = (8 * n + 31) & ~31, tid = threadIdx.x, lane = tid & 31, r = tid >> 3, q0 = tid & 7;
-    if (tid < nt) {
-        double a[8];
-        const bool row = r < n;
+// (tiny pivots guarded as semiconductor_3d.c:2066 does).  A chain of n dependent steps, so what
+// counts is the length of one: two or four warps only (warp w: rows 32 (w / 2) + lane, the
+// columns of parity w & 1, NC of them in registers), rows are never moved and stay unscaled
+// until the end (row piv[c] plays row c), and the columns turn by one register when their
+// parity's pivot is done, so that the pivot column is always a[0] and no step selects by the
+// column's number.  Per step the warps exchange the column and the pivot row through shared
+// memory (two barriers of those warps).  D[c n + q] is left as element (c, piv[q]) of the
+// inverse.  24 unknowns 10 us, 60 unknowns 22 us; 8 lanes per row of all 16 warps took 16 and
+// 50 us.
+template <class T, int NC>
+__device__ __noinline__ void invert_rows(T *D, int n, int nt, int *piv) {
+    __shared__ double col[2][COARSE_MAX];
+    __shared__ __align__(16) double prow[2][2][COARSE_MAX / 2];
+    const int tid = threadIdx.x, lane = tid & 31, ch = (tid >> 5) & 1, r = 32 * (tid >> 6) + lane;
+    const bool row = r < n;
+    double a[NC];
+#pragma unroll
+    for (int i = 0; i < NC; i++) a[i] = row && 2 * i + ch < n ? (double)D[r * n + 2 * i + ch] : 0.0;
+    bool open0 = lane < n, open1 = lane + 32 < n;            // rows lane and lane + 32 not used yet
+    int mine = 0;                                            // the column this row was the pivot of
+    double scale = 0.0;                                      // and its reciprocal pivot
+    for (int c = 0; c < n; c++) {
+        double *cc = col[c & 1];
+        const bool own = ch == (c & 1);
+        if (own) cc[r] = a[0];                               // (rows past n: zeros)
+        warps_sync(1, nt);
+        unsigned key = 0;                                    // |a| to 17 bits, ties to the lower row
         {
-            const Node c = unidx(row ? r : 0, v.Nx, v.Ny);
-            const int m = sslot(v, c.i, c.j, c.l);
-            const T *A = v.A + m;
-            const T g = v.G[m], e[6] = {A[0], A[v.ap], A[2 * v.ap], A[3 * v.ap], A[4 * v.ap], A[5 * v.ap]};
+            const unsigned h0 = (unsigned)__double2hiint(cc[lane]), k0 = ((h0 << 1) & ~63u) | (unsigned)(63 - lane);
+            key = open0 ? k0 : 0u;
+            if (NC > 16) {
+                const unsigned h1 = (unsigned)__double2hiint(cc[lane + 32]), k1 = ((h1 << 1) & ~63u) | (unsigned)(31 - lane);
+                key = max(key, open1 ? k1 : 0u);
+            }
+        }
+        const double f = cc[r];
+        const int p = 63 - (int)(__reduce_max_sync(0xffffffffu, key) & 63u);
+        const double d = cc[p], inv = 1.0 / (fabs(d) > 1e-300 ? d : 1e-300);
+        open0 = open0 && p != lane;
+        open1 = open1 && p != lane + 32;
+        double2 *pw = reinterpret_cast<double2 *>(prow[c & 1][ch]);
+        if (r == p) {
+            mine = c;
+            scale = inv;
+            if (own) piv[c] = p;
+#pragma unroll
+            for (int i = 0; i < NC / 2; i++) pw[i] = make_double2(a[2 * i], a[2 * i + 1]);
+        }
+        const double g = r == p ? 0.0 : -f * inv;
+        warps_sync(1, nt);
+        if (own) {
+#pragma unroll
+            for (int i = 0; i < NC / 2; i++) {
+                const double2 q = pw[i];
+                if (i) a[2 * i - 1] = a[2 * i] + g * q.x;
+                a[2 * i] = a[2 * i + 1] + g * q.y;
+            }
+            a[NC - 1] = r == p ? 1.0 : g;
+        } else {
+#pragma unroll
+            for (int i = 0; i < NC / 2; i++) {
+                const double2 q = pw[i];
+                a[2 * i] += g * q.x;
+                a[2 * i + 1] += g * q.y;
+            }
+        }
+    }
+    const int k = (n + 1 - ch) >> 1;                         // columns of this parity: the turns made
+    T *out = D + mine * n + ch + 2 * k;
+    if (row)
+#pragma unroll
+        for (int i = 0; i < NC; i++) {
+            if (i + k >= NC) out[2 * (i - NC)] = (T)(a[i] * scale);   // slots below k: 2 (i + k - NC) + ch
+        }
+}
+// the coarsest level's matrix spread out in v.D (zero before), then its inverse
+template <class T>
+__device__ __forceinline__ void blk_invert(PTab<T> &tb, const SLev<T> &v) {
+    __shared__ int piv[COARSE_MAX];
+    const int n = v.N, tid = threadIdx.x, nt = n > 32 ? 128 : 64;
+    if (tid < nt) {
+        int m = 0;
+        if (tid < n) {
+            const Node c = unidx(tid, v.Nx, v.Ny);
             const int NxNy = v.Nx * v.Ny;
-            const bool ok[6] = {c.i > 0, c.i < v.Nx - 1, c.j > 0, c.j < v.Ny - 1, c.l > 0, c.l < v.Nz - 1};
-            const int at[6] = {r - 1, r + 1, r - v.Nx, r + v.Nx, r - NxNy, r + NxNy};
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int q = q0 + 8 * i;
-                double x = q == r ? (double)g : 0.0;
-#pragma unroll
-                for (int w = 0; w < 6; w++)
-                    if (ok[w] && q == at[w]) x = (double)e[w];   // (a dimension of 1 or 2 nodes: one neighbour each)
-                a[i] = x;
-            }
+            m = sslot(v, c.i, c.j, c.l);
+            const T *A = v.A + m;
+            T *row = v.D + tid * n + tid;
+            row[0] = v.G[m];
+            if (c.i > 0) row[-1] = A[0];
+            if (c.i < v.Nx - 1) row[1] = A[v.ap];
+            if (c.j > 0) row[-v.Nx] = A[2 * v.ap];
+            if (c.j < v.Ny - 1) row[v.Nx] = A[3 * v.ap];
+            if (c.l > 0) row[-NxNy] = A[4 * v.ap];
+            if (c.l < v.Nz - 1) row[NxNy] = A[5 * v.ap];
+            tb.slot[tid] = m;
         }
-        unsigned long long used = 0;
-        int mine = 0;                                        // the column this row was the pivot of
-        for (int c = 0; c < n; c++) {
-            double *cc = col[c & 1], *pr = prow[c & 1];
-            if (row && q0 == (c & 7)) {
-                double x = 0.0;
-#pragma unroll
-                for (int i = 0; i < 8; i++) x = i == (c >> 3) ? a[i] : x;
-                cc[r] = x;
-            }
-            warps_sync(1, nt);
-            unsigned key = 0;                                // |a| to 17 bits, ties to the lower row
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int rr = lane + 32 * h;
-                if (rr < n && !((used >> rr) & 1)) {
-                    const unsigned hi = (unsigned)__double2hiint(cc[rr]) & 0x7fffffffu;
-                    const unsigned k = ((hi >> 5) << 6) | (unsigned)(63 - rr);
-                    key = k > key ? k : key;
-                }
-            }
-            const int p = 63 - (int)(__reduce_max_sync(0xffffffffu, key) & 63u);
-            used |= 1ull << p;
-            const double d = cc[p], inv = 1.0 / (fabs(d) > 1e-300 ? d : 1e-300);
-            if (r == p) {
-                mine = c;
-                if (q0 == 0) piv[c] = p;
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int q = q0 + 8 * i;
-                    a[i] = (q == c ? 1.0 : a[i]) * inv;
-                    if (q < n) pr[q] = a[i];
-                }
-            }
-            warps_sync(1, nt);
-            if (row && r != p) {
-                const double f = cc[r];
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int q = q0 + 8 * i;
-                    if (q < n) a[i] = (q == c ? 0.0 : a[i]) - f * pr[q];
-                }
-            }
-        }
-        if (row)
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int q = q0 + 8 * i;
-                if (q < n) v.D[mine * n + piv[q]] = (T)a[i];
-            }
+        warps_sync(1, nt);
+        if (n > 32) invert_rows<T, 32>(v.D, n, nt, piv);
+        else invert_rows<T, 16>(v.D, n, nt, piv);
+        if (tid < n) tb.cslot[tid] = tb.slot[piv[tid]];
     }
     __syncthreads();
 }
@@ -991,33 +1017,34 @@ __host__ __device__ inline size_t ssm_level(int H, int ap, int n, bool last) {
         return al16((size_t)6 * ap * sizeof(T)) + 3 * al16((size_t)2 * H * sizeof(T)) + al16((size_t)n * n * sizeof(T));
     return al16((size_t)6 * ap * sizeof(T)) + 5 * al16((size_t)2 * H * sizeof(T));
 }
-// views of the levels Ls .. nl-1 in block 0's shared memory (thread 0)
+// Views of the levels Ls .. nl-1 in block 0's shared memory, a thread per level, and all of it
+// zeroed (padding slots, the coarsest matrix); done while the block waits at the first barrier
 template <class T>
-__device__ void ssm_views(PTab<T> &tb, int Ls, int nl, unsigned char *base) {
-    for (int L = Ls; L < nl; L++) {
-        SLev<T> v = tb.w.lev[L];
-        const size_t nb = al16((size_t)2 * v.H * sizeof(T));
+__device__ __forceinline__ void ssm_views(PTab<T> &tb, int Ls, int nl, unsigned char *base, int tid, int nth) {
+    size_t all = 0;
+    for (int L = Ls; L < nl; L++) all += ssm_level<T>(tb.w.lev[L].H, tb.w.lev[L].ap, tb.w.lev[L].N, L == nl - 1);
+    for (int q = tid; q < (int)(all / 16); q += nth) reinterpret_cast<int4 *>(base)[q] = make_int4(0, 0, 0, 0);
+    const int L = Ls + tid;
+    if (L < nl) {
         unsigned char *p = base;
+        for (int K = Ls; K < L; K++) p += ssm_level<T>(tb.w.lev[K].H, tb.w.lev[K].ap, tb.w.lev[K].N, false);
+        SLev<T> &v = tb.sv[L - Ls];
+        v = tb.w.lev[L];
+        const size_t nb = al16((size_t)2 * v.H * sizeof(T));
         v.A = reinterpret_cast<T *>(p); p += al16((size_t)6 * v.ap * sizeof(T));
         v.G = reinterpret_cast<T *>(p); p += nb;
         v.D = reinterpret_cast<T *>(p); p += v.last ? al16((size_t)v.N * v.N * sizeof(T)) : nb;
         if (!v.last) { v.pw = reinterpret_cast<T *>(p); p += nb; }
         v.x = reinterpret_cast<T *>(p); p += nb;
         v.b = reinterpret_cast<T *>(p);
-        tb.sv[L - Ls] = v;
-        base += ssm_level<T>(v.H, v.ap, v.N, v.last);
-    }
-    // threads of a level: a pair of slots each, a warp per 8 coarse nodes of its restriction, 8
-    // lanes per row of the dense inverse, and no fewer than the level below
-    int ntc = 0;
-    for (int L = nl - 1; L >= Ls; L--) {
-        SLev<T> &v = tb.sv[L - Ls];
-        int nt = v.last ? 8 * v.N : v.H >> 1;
-        if (!v.last) {
-            const SLev<T> &c = tb.sv[L + 1 - Ls];
-            nt = max(max(nt, 32 * c.n8 * c.Ny * c.Nz), ntc);
+        // threads of a level: a pair of slots each, a warp per 8 coarse nodes of its restriction,
+        // 8 lanes per row of the dense inverse, and no fewer than the levels below
+        int nt = 0;
+        for (int K = L; K < nl; K++) {
+            const SLev<T> &w = tb.w.lev[K];
+            nt = max(nt, w.last ? 8 * w.N : max(w.H >> 1, 32 * tb.w.lev[K + 1].n8 * tb.w.lev[K + 1].Ny * tb.w.lev[K + 1].Nz));
         }
-        ntc = v.nt = min((nt + 31) & ~31, (int)blockDim.x);
+        v.nt = min((nt + 31) & ~31, (int)blockDim.x);
     }
 }
 // The multigrid set-up of the system loaded by pg_load (the reference's mg_setup,
@@ -1025,8 +1052,7 @@ __device__ void ssm_views(PTab<T> &tb, int Ls, int nl, unsigned char *base) {
 // operator of the next level and that level's weights - and the small levels in block 0's
 // shared memory.  `xr` takes the first red values D r of the solve.
 template <class T>
-__device__ __noinline__ bool pg_setup(const DevP &P, PS &s, const PArgs &a, PTab<T> &tb, int nl, T *xr,
-                                      unsigned char *smem) {
+__device__ __noinline__ bool pg_setup(const DevP &P, PS &s, const PArgs &a, PTab<T> &tb, int nl, T *xr) {
     const int Ls = a.Ls, qsign = a.qsign;
     for (int L = 0; L < Ls; L++) {
         const SLev<T> &f = tb.w.lev[L], &cl = tb.w.lev[L + 1];
@@ -1038,44 +1064,29 @@ __device__ __noinline__ bool pg_setup(const DevP &P, PS &s, const PArgs &a, PTab
         PG_SYNC();
     }
     if (blockIdx.x == 0) {
-        if (threadIdx.x == 0) ssm_views<T>(tb, Ls, nl, smem);
-        __syncthreads();
         const int tid = threadIdx.x, nth = blockDim.x;
         {
-            const SLev<T> &g = tb.w.lev[Ls];
-            const SLev<T> v = tb.sv[0];
-            for (int q = tid; q < 2 * v.H; q += nth) {
-                const int u = q < v.H ? q : q - v.H;
-                const Pair p = slot_row(v, u);
-                const int i = 2 * p.t + ((p.j + p.l + (q >= v.H)) & 1);
-                const bool ok = i < v.Nx;                   // padding slots: zero (nothing writes them in global memory)
-                v.G[q] = ok ? g.G[q] : T(0);
-                if (!v.last && q < v.H) v.D[q] = ok ? g.D[q] : T(0);
-                for (int e = 0; e < 6; e++) v.A[e * v.ap + q] = ok ? g.A[e * v.ap + q] : T(0);
-            }
-        }
-        for (int L = Ls; L < nl - 1; L++) {
-            const SLev<T> v = tb.sv[L - Ls], cl = tb.sv[L + 1 - Ls];
-            for (int q = tid; q < 2 * v.H; q += nth) { v.pw[q] = 0; v.x[q] = 0; v.b[q] = 0; }
-            for (int q = tid; q < 2 * cl.H; q += nth) {
-                cl.G[q] = 0;
-                for (int e = 0; e < 6; e++) cl.A[e * cl.ap + q] = 0;
+            const SLev<T> &g = tb.w.lev[Ls], &v = tb.sv[0];
+            // the first small level as pg_galerkin left it, padding slots included (the black
+            // pivots are stale, pg_pivots writes them below; the coarsest level has none)
+            for (int e = 0; e < (v.last ? 2 : 3); e++) {
+                const int4 *src = reinterpret_cast<const int4 *>(e == 0 ? g.A : e == 1 ? g.G : g.D);
+                int4 *dst = reinterpret_cast<int4 *>(e == 0 ? v.A : e == 1 ? v.G : v.D);
+                const int n = (e == 0 ? 6 * v.ap : 2 * v.H) * (int)sizeof(T) / 16;   // (2 H: a multiple of 4)
+#pragma unroll 4
+                for (int q = tid; q < n; q += nth) dst[q] = src[q];
             }
             __syncthreads();
+        }
+        for (int L = Ls; L < nl - 1; L++) {
+            const SLev<T> &v = tb.sv[L - Ls], &cl = tb.sv[L + 1 - Ls];
             pg_weights<T>(P, v, cl, PT<T>::lev(P, L).ph, PT<T>::lev(P, L + 1).ph, qsign, tid, nth);
             pg_pivots<T>(v, tid, nth);
             __syncthreads();
             pg_galerkin<T>(v, cl, nullptr, tid, nth);
             __syncthreads();
         }
-        const SLev<T> &v = tb.sv[nl - 1 - Ls];
-        for (int q = tid; q < 2 * v.H; q += nth) v.x[q] = v.b[q] = 0;
-        if (tid < v.N) {
-            const Node c = unidx(tid, v.Nx, v.Ny);
-            tb.slot[tid] = sslot(v, c.i, c.j, c.l);
-        }
-        __syncthreads();
-        blk_invert<T>(v);
+        blk_invert<T>(tb, tb.sv[nl - 1 - Ls]);
     }
     return true;
 }
@@ -1137,7 +1148,7 @@ __global__ void __launch_bounds__(PT_TPB, 1) k_persist(const DevP *Ps, PArgs a) 
     double acc[2] = {0.0, 0.0};
     pg_load<T, KIND>(P, tb, s, acc);
     pg_weights<T>(P, tb.w.lev[0], tb.w.lev[1], nullptr, PT<T>::lev(P, 1).ph, a.qsign, s.tid, s.nth);
-    if (!pg_sum<2>(s, acc)) return;
+    if (!pg_sum<2>(s, acc, [&]() { if (blockIdx.x == 0) ssm_views<T>(tb, a.Ls, nl, sraw, threadIdx.x - 32, blockDim.x - 32); })) return;
     if constexpr (KIND != PK_PCG) {
         if (threadIdx.x == 0) {
             KrylovS &rec = KIND == PK_REFINED ? so : sk;
@@ -1154,7 +1165,7 @@ __global__ void __launch_bounds__(PT_TPB, 1) k_persist(const DevP *Ps, PArgs a) 
     const bool go = KIND == PK_PCG || (KIND == PK_REFINED ? so.active : sk.active) != 0;
     int steps = 0;
     if (go) {
-        if (!pg_setup<T>(P, s, a, tb, nl, tb.w.vec[KIND == PK_PCG ? 1 : 4], sraw)) return;
+        if (!pg_setup<T>(P, s, a, tb, nl, tb.w.vec[KIND == PK_PCG ? 1 : 4])) return;
         if constexpr (KIND == PK_PCG) {
             if (!pg_pcg<T>(s, a, tb, nl, sk)) return;
             if (std::is_same<T, double>::value || sk.status == 1)

@@ -71,9 +71,13 @@ __device__ __forceinline__ int pg_poll(PS &s) {
     }
     return 1;
 }
-__device__ __forceinline__ bool pg_sync(PS &s) {
+// `idle`: work that warps 1 .. of the block do while its first thread waits
+struct PgNone { __device__ void operator()() const {} };
+template <class F = PgNone>
+__device__ __forceinline__ bool pg_sync(PS &s, F idle = F()) {
     __shared__ int s_ok;
     if (s.onecl) {                                 // one cluster: barrier.cluster (release / acquire)
+        if (threadIdx.x >= 32) idle();
         cooperative_groups::this_cluster().sync();
         return true;
     }
@@ -98,14 +102,16 @@ __device__ __forceinline__ bool pg_sync(PS &s) {
         }
         s_ok = ok;
         if (s.trace && bn < s.ntrace && blockIdx.x == 0) s.trace[3 * bn + 2] = pg_clock();
+    } else if (threadIdx.x >= 32) {
+        idle();
     }
     __syncthreads();
     return s_ok != 0;
 }
 
 // Sum NV (<= 4) values over the grid; every block returns the same totals in every thread.
-template <int NV>
-__device__ __forceinline__ bool pg_sum(PS &s, double (&v)[NV]) {
+template <int NV, class F = PgNone>
+__device__ __forceinline__ bool pg_sum(PS &s, double (&v)[NV], F idle = F()) {
     __shared__ double tot[4];
     block_sum<NV>(v);
     double *buf = s.g->red[s.rb];
@@ -113,7 +119,7 @@ __device__ __forceinline__ bool pg_sum(PS &s, double (&v)[NV]) {
     if (threadIdx.x == 0)
 #pragma unroll
         for (int q = 0; q < NV; q++) buf[blockIdx.x * 4 + q] = v[q];
-    if (!pg_sync(s)) return false;
+    if (!pg_sync(s, idle)) return false;
     if (threadIdx.x < 32) {
         double a[NV];
 #pragma unroll
