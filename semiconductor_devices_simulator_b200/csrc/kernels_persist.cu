@@ -1264,7 +1264,7 @@ struct KInfo {
     const void *fn = nullptr;
     size_t smem = 0;       // dynamic shared memory the attribute allows
     int blocks = 0;        // co-resident blocks at that size
-    int clusters = 0;      // co-resident clusters at that size (0: no cluster launch)
+    int clusters[2] = {};  // co-resident clusters of 8 / 16 CTAs at that size (0: no such launch)
 };
 std::mutex g_pmu;
 int g_persist_mode = -1;   // -1 unread, 0 off, 1 on
@@ -1276,8 +1276,8 @@ unsigned long long *g_trace = nullptr;   // armed barrier timeline (test hook): 
 int g_trace_n = 0, g_trace_used = 0;     // its barriers; 1 once a launch has filled it
 int g_last_blocks = 0;                   // blocks of the last persistent launch
 int g_barmode = 1;         // grid-barrier form (SEMISIM_B200_BARMODE; 1 measured faster than 0)
-int g_clusters = 1;        // cluster launches: 0 off, 1 grids of one cluster, 2 every grid (SEMISIM_B200_CLUSTERS)
-int g_csz = 8;             // CTAs per cluster (SEMISIM_B200_CSZ: 8 portable, 16 non-portable)
+int g_clusters = 1;        // cluster launches: 0 off, 1 where they gain (persist_run), 2 every grid (SEMISIM_B200_CLUSTERS)
+int g_csz = 16;            // CTAs per cluster at most (SEMISIM_B200_CSZ: 8 portable, 16 non-portable)
 int g_clevel = 1;          // first level the first cluster runs alone (SEMISIM_B200_CLEVEL)
 int g_coop = 1;            // cooperative launch attribute (SEMISIM_B200_COOP=0: plain launch of a
                            //   grid within the co-resident capacity)
@@ -1285,19 +1285,19 @@ int g_coop = 1;            // cooperative launch attribute (SEMISIM_B200_COOP=0:
 template <class T, int KIND>
 const void *kfn() { return reinterpret_cast<const void *>(&k_persist<T, KIND>); }
 
-// co-resident clusters of g_csz CTAs of the kernel at `smem` bytes (0: no clusters)
-int cluster_occupancy(const void *fn, size_t smem) {
-    if (g_csz > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+// co-resident clusters of csz CTAs of the kernel at `smem` bytes (0: no clusters)
+int cluster_occupancy(const void *fn, size_t smem, int csz) {
+    if (csz > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     cudaLaunchConfig_t q = {};
-    q.gridDim = dim3(g_csz);
+    q.gridDim = dim3(csz);
     q.blockDim = dim3(PT_TPB);
     q.dynamicSmemBytes = smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = g_csz; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.x = csz; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     q.attrs = at;
     q.numAttrs = 1;
     int n = 0;
@@ -1330,7 +1330,7 @@ int persist_enabled() {
         if (const char *m = std::getenv("SEMISIM_B200_BARMODE")) g_barmode = std::atoi(m) ? 1 : 0;
         if (const char *m = std::getenv("SEMISIM_B200_CLUSTERS")) g_clusters = std::atoi(m) < 0 ? 0 : (std::atoi(m) > 2 ? 2 : std::atoi(m));
         if (const char *m = std::getenv("SEMISIM_B200_CLEVEL")) g_clevel = std::atoi(m) < 1 ? 1 : std::atoi(m);
-        if (const char *m = std::getenv("SEMISIM_B200_CSZ")) g_csz = std::atoi(m) == 16 ? 16 : 8;
+        if (const char *m = std::getenv("SEMISIM_B200_CSZ")) g_csz = std::atoi(m) == 8 ? 8 : 16;
         if (const char *m = std::getenv("SEMISIM_B200_COOP")) g_coop = std::atoi(m) != 0;
         int dev = 0, coop = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
@@ -1352,12 +1352,13 @@ int persist_thread_blocks(int n) {
     return old;
 }
 
-// Launch the persistent solve `kind` of precision T on instance 0 of the context.  Returns
+// Launch the persistent solve `kind` of precision T on instance 0 of the context (n1: nodes of
+// level 1).  Returns
 // 1 when it ran (results in the Krylov records), 0 when the persistent path does not apply
 // (the caller runs the per-pass path), -1 when a barrier wait ran out (the caller restores
 // the start and runs the per-pass path; the persistent path is off from then on).
 template <class T, int KIND>
-static int persist_run(const Ctx &c, int Ls, size_t smem, const PArgs &a, PGrid *hres) {
+static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGrid *hres) {
     static KInfo info;                           // per instantiation, cached
     static std::mutex mu;
     KInfo ki;
@@ -1368,7 +1369,8 @@ static int persist_run(const Ctx &c, int Ls, size_t smem, const PArgs &a, PGrid 
             k.fn = kfn<T, KIND>();
             k.smem = smem;
             k.blocks = occupancy(k.fn, smem);
-            k.clusters = cluster_occupancy(k.fn, smem);
+            k.clusters[0] = cluster_occupancy(k.fn, smem, 8);
+            k.clusters[1] = g_csz > 8 ? cluster_occupancy(k.fn, smem, 16) : 0;
         }
         ki = k;
     }
@@ -1382,30 +1384,42 @@ static int persist_run(const Ctx &c, int Ls, size_t smem, const PArgs &a, PGrid 
     if (t_persist_blocks > 0 && t_persist_blocks < nb) nb = t_persist_blocks;
     if (nb > PG_MAXB) nb = PG_MAXB;
     if (nb < 1) return 0;
-    // clusters of g_csz CTAs: a grid of at most g_csz blocks becomes one cluster (every
-    // barrier a cluster barrier, 0.3 us against 2 us for a grid barrier).  With g_clusters 2 a
-    // larger grid is a whole number of clusters, the first of which runs the coarse levels
-    // from Lc on alone; that costs the grid the SMs that no whole cluster covers (112 - 120
-    // of 148 blocks), which a full-size solve loses more time to than the coarse levels gain,
-    // so by default larger grids launch without clusters
+    // Clusters.  A grid of at most 8 blocks becomes one cluster of 8 CTAs, up to 31 blocks' worth
+    // one of 16: its barriers are cluster barriers, 0.3 us against 1.2-1.5 us for a grid barrier
+    // (11,520 / 16,128 / 28,672 nodes FP64 38.9 / 39.9 / 45.3 -> 33.6 / 35.9 / 41.0 ms a sweep).  A larger grid is
+    // a whole number of 16-CTA clusters, the first of which runs level 1 .. Ls-1 alone, while
+    // level 1 has at most three (FP32: four) nodes a thread of that cluster: 64,000 nodes 82.5 ->
+    // 78.0 ms, 180,000 96.6 -> 93.6 (FP32 89.1 -> 86.5), FP32 FinFET of 214,000 129.3 -> 127.0.
+    // Beyond, the cluster's passes take longer than the whole grid's with its barriers, and level
+    // 0 misses the SMs that no whole cluster covers (112 of 148 blocks): 230,400 nodes FP64 101.1
+    // -> 103.1, 336,000 118.2 -> 124.9 (FP32 98.4 -> 103.2); clusters of 8 for that part lose
+    // from 180,000 nodes on (101.2).  Only seven clusters of 16 fit the GPU: where fewer such
+    // grids than plain ones run side by side and the process has instances enough to notice, the
+    // grid stays plain (six 36,864-node instances: 74 ms plain, 82 in clusters of 16), as do
+    // capped grids, which share the SMs by blocks.
     PArgs aa = a;
     aa.csz = 0;
     aa.onecl = 0;
     aa.Lc = a.Ls;
-    if (g_clusters && ki.clusters > 0) {
-        if (nb <= g_csz) {
-            nb = g_csz;
-            aa.csz = g_csz;
-            aa.onecl = 1;
-        } else if (g_clusters == 2) {
-            int ncl = nb / g_csz;
-            if (ncl > ki.clusters) ncl = ki.clusters;
-            nb = ncl * g_csz;
-            aa.csz = g_csz;
-            aa.Lc = g_clevel < a.Ls ? g_clevel : a.Ls;
-        }
+    const bool capped = c.pblocks > 0 || t_persist_blocks > 0 || g_persist_blocks > 0;
+    const int c16 = ki.clusters[1], per = sizeof(T) == 4 ? 4 : 3;
+    int csz = 0, ncl = 1;
+    if (g_clusters && ki.clusters[0] > 0 && nb <= 8) {
+        csz = 8;
+    } else if (g_clusters == 2 && (c16 > 0 || ki.clusters[0] > 0)) {
+        csz = c16 > 0 ? 16 : 8;
+        ncl = std::max(1, std::min(nb / csz, c16 > 0 ? c16 : ki.clusters[0]));
+    } else if (g_clusters == 1 && c16 > 0 && !capped && n1 <= per * 16 * PT_TPB) {
+        ncl = std::max(1, std::min(nb / 16, c16));
+        if (2 * nb <= ki.blocks && ncl > 3) ncl = 3;        // two of these grids run side by side
+        if (ki.blocks / nb <= c16 / ncl || live_instances() * ncl <= c16) csz = 16;
     }
-    (void)Ls;
+    if (csz) {
+        nb = ncl * csz;
+        aa.csz = csz;
+        aa.onecl = ncl == 1;
+        if (ncl > 1) aa.Lc = g_clevel < a.Ls ? g_clevel : a.Ls;
+    }
     PGrid *g = c.h.pgrid;
     cudaMemsetAsync(g, 0, 6 * sizeof(unsigned), c.st);      // counter, error word, work counters
     const DevP *dp = c.dP;
@@ -1532,8 +1546,8 @@ int persist_pcg(const Ctx &c, const MGHost &mg, int mixed) {
     a.alpha = mg.alpha * MG_OVER;
     a.barmode = g_barmode;
     PGrid h{};
-    const int rc = mixed ? persist_run<float, PK_PCG>(c, a.Ls, smem, a, &h)
-                         : persist_run<double, PK_PCG>(c, a.Ls, smem, a, &h);
+    const int rc = mixed ? persist_run<float, PK_PCG>(c, mg.maxN[1], smem, a, &h)
+                         : persist_run<double, PK_PCG>(c, mg.maxN[1], smem, a, &h);
     if (rc == 1 && g_prof_on) {
         const double vb = mixed ? vcycle_bytes<float>(mg, a.Ls, a.deep, a.sweeps2)
                                 : vcycle_bytes<double>(mg, a.Ls, a.deep, a.sweeps2);
@@ -1558,7 +1572,7 @@ int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int q
     a.rtol = rtol;
     a.atol = atol;
     PGrid h{};
-    const int rc = persist_run<double, PK_BICG>(c, a.Ls, smem, a, &h);
+    const int rc = persist_run<double, PK_BICG>(c, mg.maxN[1], smem, a, &h);
     if (rc == 1 && g_prof_on) {
         const double vb = vcycle_bytes<double>(mg, a.Ls, a.deep, a.sweeps2);
         const double kb = 2 * kProfBytesPerNode[PF_KRY_SPMV_DOT] + 4 * kProfBytesPerNode[PF_KRY_UPDATE];
@@ -1580,7 +1594,7 @@ int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, in
     a.barmode = g_barmode;
     a.maxsteps = maxsteps;
     PGrid h{};
-    const int rc = persist_run<float, PK_REFINED>(c, a.Ls, smem, a, &h);
+    const int rc = persist_run<float, PK_REFINED>(c, mg.maxN[1], smem, a, &h);
     if (rc == 1) {
         *steps = h.steps;
         if (g_prof_on) {

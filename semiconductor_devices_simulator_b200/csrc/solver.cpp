@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -208,7 +209,11 @@ int mg_levels(int Nx, int Ny, int Nz, int dims[][6]) {
     return nl;
 }
 
+// instances of this process with their device memory set up
+static std::atomic<int> g_live{0};
+int live_instances() { return g_live.load(); }
 void gpu_free(Inst &d) {
+    if (d.g.ready) g_live--;
     for (auto &e : d.g.lg.exec)
         if (e) cudaGraphExecDestroy(e);
     for (auto &e : d.g.tev)
@@ -305,6 +310,7 @@ static int gpu_alloc(Inst &d) {
         mg.maxRows[L] = levs[L].Ny * levs[L].Nz;
     }
     d.g.ready = true;
+    g_live++;
     return 1;
 }
 

@@ -291,6 +291,7 @@ int persist_enabled();
 void persist_set(int mode, int blocks);
 int persist_get_blocks();
 int persist_thread_blocks(int n);
+int live_instances();        // instances of the process with device memory (solver.cpp)
 int persist_pcg(const Ctx &c, const MGHost &mg, int mixed);
 int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int qsign);
 int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign);
