@@ -646,13 +646,9 @@ int pcg_graph(Inst &d, int maxit, double rtol) {
     double *r = d.g.h.wk[0], *z = d.g.h.wk[1], *p = d.g.h.wk[2], *q = d.g.h.wk[3];
     if (persist_enabled()) {                      // set-up and solve in one persistent launch
         lin(c, d.g.h.wk[7], 0.0, x, 1.0);        // start backup
-        const int pr = persist_graph(d, 0, maxit, rtol, 0.0, 0, false);
-        if (pr == 1) {
-            KrylovS hs{};
-            cudaMemcpyAsync(&hs, c.h.ks, sizeof(KrylovS), cudaMemcpyDeviceToHost, c.st);
-            cudaStreamSynchronize(c.st);
-            return hs.it;
-        }
+        KrylovS hs{};
+        const int pr = persist_graph(d, 0, maxit, rtol, 0.0, 0, false, hs);
+        if (pr == 1) return hs.it;
         if (pr < 0) lin(c, x, 0.0, d.g.h.wk[7], 1.0);
     }
     gmg_setup(d, c, 0, nullptr);
@@ -696,11 +692,9 @@ int bicg_graph(Inst &d, int maxit, double rtol, double atol, double *rn_out, dou
     const double *w = d.g.h.dsc;
     if (persist_enabled()) {                      // set-up and solve in one persistent launch
         lin(c, d.g.h.wk[7], 0.0, x, 1.0);        // start backup
-        const int pr = persist_graph(d, 1, maxit, rtol, atol, qsign, ilu_only);
+        KrylovS hs{};
+        const int pr = persist_graph(d, 1, maxit, rtol, atol, qsign, ilu_only, hs);
         if (pr == 1) {
-            KrylovS hs{};
-            cudaMemcpyAsync(&hs, c.h.ks, sizeof(KrylovS), cudaMemcpyDeviceToHost, c.st);
-            cudaStreamSynchronize(c.st);
             *r0_out = hs.r0;
             *rn_out = std::sqrt(hs.rr);
             return hs.it;

@@ -74,6 +74,7 @@ struct GPArgs {
     int qsign;           // Slotboom weights: 0 none, +1 electrons, -1 holes
     int onecl;
     double alpha, rtol, atol;
+    KrylovS rec;         // starting record
 };
 
 // the threads that run a level: the whole grid, or block 0 alone
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(GP_TPB, 1) k_gpersist(const DevP *Ps, GPArgs g
     s.ntrace = 0;
     s.mode = 1;
     s.onecl = ga.onecl;
-    if (threadIdx.x == 0) sk = *P.ks;
+    if (threadIdx.x == 0) sk = ga.rec;
     __syncthreads();
     const PGLev &H0 = lt[0];
     const int N = P.N;
@@ -792,7 +793,7 @@ __global__ void __launch_bounds__(GP_TPB, 1) k_gpersist(const DevP *Ps, GPArgs g
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *P.ks = sk;
+        s.g->rec[0] = sk;
         s.g->iters = sk.it;
     }
 }
@@ -951,9 +952,9 @@ void gpersist_build(Inst &d, const std::vector<GpLevelIn> &lv, cudaStream_t st) 
 
 // Launch the persistent graph solve (kind 0 PCG from the present sol with the stop rule
 // r.z <= rtol^2 r0.z0; kind 1 BiCGSTAB with max(rtol r0, atol floor)).  Returns 1 when it
-// ran (P.ks holds it, rr, r0), 0 when it does not apply (nothing changed), -1 when a barrier
+// ran (k holds it, rr, r0), 0 when it does not apply (nothing changed), -1 when a barrier
 // wait ran out (the caller restores the start).
-int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qsign, bool ilu_only) {
+int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qsign, bool ilu_only, KrylovS &k) {
     if (!persist_enabled() || !d.g.gptab) return 0;
     const int nl = (int)d.g.glev.size();
     int Ls = nl;
@@ -995,7 +996,6 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
     ks0.rtol = rtol;
     ks0.atol = atol;
     ks0.active = 1;
-    cudaMemcpyAsync(c.h.ks, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
     PGrid *g = c.h.pgrid;
     cudaMemsetAsync(g, 0, 6 * sizeof(unsigned), c.st);
     GPArgs a{};
@@ -1010,6 +1010,7 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
     a.alpha = kind ? g_knobs.mg_alpha : g_knobs.mg_alpha * MG_OVER;
     a.rtol = rtol;
     a.atol = atol;
+    a.rec = ks0;
     const DevP *dp = c.dP;
     void *args[] = {(void *)&dp, (void *)&a};
     g_launches++;
@@ -1032,9 +1033,10 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
         cudaGetLastError();
         return 0;
     }
-    PGrid h{};
-    cudaMemcpyAsync(&h, g, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, c.st);
+    const PGridHead &h = *c.pin;                  // status and closing record in one copy
+    cudaMemcpyAsync(c.pin, g, sizeof(PGridHead), cudaMemcpyDeviceToHost, c.st);
     cudaStreamSynchronize(c.st);
+    k = h.rec[0];
     if (h.err) {
         std::fprintf(stderr, "semisim-b200: persistent graph solve abandoned (a barrier wait ran out)\n");
         return -1;

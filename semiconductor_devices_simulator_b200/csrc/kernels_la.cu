@@ -1170,22 +1170,20 @@ int pcg_solve(const Ctx &c, const MGHost &mg, int maxit, double rtol, int check_
     ks0.maxit = maxit;
     ks0.rtol = rtol;
     if (mixed && rtol >= 1e-5) {
-        cudaMemcpyAsync(c.h.ksi, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
-        const int pr = persist_pcg(c, mg, 1);        // set-up and solve in one persistent launch
-        if (pr == 1) {
-            const KrylovS hs = read_ks(c, c.h.ksi);
+        KrylovS hs = ks0;
+        if (persist_pcg(c, mg, 1, hs) == 1) {        // set-up and solve in one persistent launch
             if (hs.status == 1) return hs.it;
             t_ir_fallbacks++;
             launch_fill_sel(c, V_SOL, 0.0);
             return hs.it + pcg_solve(c, mg, maxit, rtol, check_every, 0);
         }
-        if (pr < 0) cudaMemcpyAsync(c.h.ksi, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
+        cudaMemcpyAsync(c.h.ksi, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
         mg_setup_t<float>(c, mg, 0);
         SS_LAUNCH_PDL(PF_KRY_INIT32, c.maxN, k_pcg32_start, grid_nodes(c), TPB, c.st, c.dP);
         vcycle_t<float>(c, mg, 0, 1, 0, 1, 0);
         SS_LAUNCH_PDL(PF_KRY_DOT32, c.maxN, k_pcg_rz<float>, grid_nodes(c), TPB, c.st, c.dP, 0);
         SS_LAUNCH_PDL(PF_KRY_UPDATE32, c.maxN, k_pcg_p<float>, grid_nodes(c), TPB, c.st, c.dP, 1);
-        const KrylovS hs = run_loop(c, mg, 3, maxit, check_every);
+        hs = run_loop(c, mg, 3, maxit, check_every);
         if (hs.status == 1) {
             SS_LAUNCH_PDL(PF_VEC, c.maxN, k_sol_from32, grid_nodes(c), TPB, c.st, c.dP);
             return hs.it;
@@ -1194,16 +1192,14 @@ int pcg_solve(const Ctx &c, const MGHost &mg, int maxit, double rtol, int check_
         launch_fill_sel(c, V_SOL, 0.0);
         return hs.it + pcg_solve(c, mg, maxit, rtol, check_every, 0);
     }
-    cudaMemcpyAsync(c.h.ks, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
     if (c.ninst == 1 && persist_enabled()) {
         launch_copy_sel(c, 7, V_SOL);                // start backup (the persistent path may be abandoned)
-        const int pr = persist_pcg(c, mg, 0);        // set-up and solve in one persistent launch
-        if (pr == 1) return read_ks(c, c.h.ks).it;
-        if (pr < 0) {
-            launch_copy_sel(c, V_SOL, 7);
-            cudaMemcpyAsync(c.h.ks, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
-        }
+        KrylovS hs = ks0;
+        const int pr = persist_pcg(c, mg, 0, hs);    // set-up and solve in one persistent launch
+        if (pr == 1) return hs.it;
+        if (pr < 0) launch_copy_sel(c, V_SOL, 7);
     }
+    cudaMemcpyAsync(c.h.ks, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
     mg_setup_t<double>(c, mg, 0);
     SS_LAUNCH_PDL(PF_KRY_INIT, c.maxN, k_pcg_init_r<double>, grid_nodes(c), TPB, c.st, c.dP);
     vcycle_t<double>(c, mg, 0, 1, 0, 1, 0);                  // z = M r
@@ -1216,28 +1212,23 @@ int pcg_solve(const Ctx &c, const MGHost &mg, int maxit, double rtol, int check_
 // FP64-refined BiCGSTAB with FP32 inner solves (multigrid preconditioner).  A stalled
 // refinement hands the solve to the FP64 solver with the same target.
 static int bicgstab_refined(const Ctx &c, const MGHost &mg, int maxit, double rtol, double atol, int check_every,
-                            double *rn, double *r0, int qsign) {
+                            double *rn, double *r0, int qsign, int saved) {
     KrylovS ko{}, ki{};
     ko.maxit = maxit;
     ko.rtol = rtol;
     ko.atol = atol;
     ki.rtol = g_ir_rtol_min;
     ki.atol = g_ir_factor;
-    cudaMemcpyAsync(c.h.ks, &ko, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
-    cudaMemcpyAsync(c.h.ksi, &ki, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
-    launch_copy_sel(c, 7, V_SOL);                   // start backup
-    KrylovS hs{};
+    if (!saved) launch_copy_sel(c, 7, V_SOL);       // start backup
+    KrylovS hs = ko;
     int steps = 0;
-    const int pr = persist_refined(c, mg, 16, &steps, qsign);   // set-up and every step in one launch
+    const int pr = persist_refined(c, mg, 16, &steps, qsign, ki, hs);   // set-up and every step in one launch
     if (pr == 1) {
-        hs = read_ks(c, c.h.ks);
         t_ir_steps += steps > 0 ? steps : 1;
     } else {
-        if (pr < 0) {                                // abandoned: restore the start, per-pass solve
-            launch_copy_sel(c, V_SOL, 7);
-            cudaMemcpyAsync(c.h.ks, &ko, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
-            cudaMemcpyAsync(c.h.ksi, &ki, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
-        }
+        if (pr < 0) launch_copy_sel(c, V_SOL, 7);    // abandoned: restore the start, per-pass solve
+        cudaMemcpyAsync(c.h.ks, &ko, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
+        cudaMemcpyAsync(c.h.ksi, &ki, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
         mg_setup_t<float>(c, mg, qsign);
         SS_LAUNCH_PDL(PF_REFINE, c.maxN, k_ir_init, grid_nodes(c), TPB, c.st, c.dP);
         for (int step = 0; step < 16; step++) {
@@ -1269,29 +1260,28 @@ static int bicgstab_refined(const Ctx &c, const MGHost &mg, int maxit, double rt
 
 // One BiCGSTAB solve of P.A sol = rhs from the present sol.  Returns the iterations;
 // rn / r0 the final and initial residual norms.  mixed: FP64-refined FP32 solve (with
-// the multigrid preconditioner only; the smoother-only retry stays FP64).
+// the multigrid preconditioner only; the smoother-only retry stays FP64).  saved: work vector 7
+// already holds the start.
 int bicgstab_core(const Ctx &c, const MGHost &mg, int maxit, double rtol, double atol, int mg_on, int check_every,
-                  double *rn, double *r0, int qsign, int mixed) {
-    if (mixed && mg_on && mg.maxlev > 1) return bicgstab_refined(c, mg, maxit, rtol, atol, check_every, rn, r0, qsign);
+                  double *rn, double *r0, int qsign, int mixed, int saved) {
+    if (mixed && mg_on && mg.maxlev > 1)
+        return bicgstab_refined(c, mg, maxit, rtol, atol, check_every, rn, r0, qsign, saved);
     KrylovS ks0{};
     ks0.maxit = maxit;
     ks0.rtol = rtol;
     ks0.atol = atol;
-    cudaMemcpyAsync(c.h.ks, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
     if (mg_on && c.ninst == 1 && persist_enabled()) {
-        launch_copy_sel(c, 7, V_SOL);                // start backup (the persistent path may be abandoned)
-        const int pr = persist_bicg(c, mg, rtol, atol, qsign);   // set-up and solve in one launch
+        if (!saved) launch_copy_sel(c, 7, V_SOL);    // start backup (the persistent path may be abandoned)
+        KrylovS hs = ks0;
+        const int pr = persist_bicg(c, mg, hs, qsign);   // set-up and solve in one launch
         if (pr == 1) {
-            const KrylovS hs = read_ks(c, c.h.ks);
             *rn = sqrt(hs.rr);
             *r0 = hs.r0;
             return hs.it;
         }
-        if (pr < 0) {
-            launch_copy_sel(c, V_SOL, 7);
-            cudaMemcpyAsync(c.h.ks, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
-        }
+        if (pr < 0) launch_copy_sel(c, V_SOL, 7);
     }
+    cudaMemcpyAsync(c.h.ks, &ks0, sizeof(KrylovS), cudaMemcpyHostToDevice, c.st);
     if (mg_on) mg_setup_t<double>(c, mg, qsign);
     else {
         SS_LAUNCH_PDL(PF_ILU_DIAG, c.maxN, k_ilu_diag<double>, grid_nodes(c), TPB, c.st, c.dP, 0);

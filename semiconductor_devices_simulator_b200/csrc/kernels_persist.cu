@@ -83,6 +83,7 @@ struct PArgs {
     int onecl;                   // the whole grid is one cluster
     double alpha;    // prolongation factor
     double rtol, atol;   // stop rule of the FP64 BiCGSTAB start (PK_BICG)
+    KrylovS rec[2];      // starting records: the loop's, and the refinement's (PK_REFINED)
 };
 
 // ---------------------------------------------------------------- layout on the host
@@ -1139,8 +1140,8 @@ __global__ void __launch_bounds__(PT_TPB, 1) k_persist(const DevP *Ps, PArgs a) 
         if (threadIdx.x == 0) {
             tb.A64 = P.A[0];
             tb.ap64 = (int)(P.A[1] - P.A[0]);
-            sk = *PT<T>::ks(P);
-            so = *P.ks;
+            sk = a.rec[0];
+            so = a.rec[1];
         }
     }
     __syncthreads();
@@ -1232,8 +1233,8 @@ __global__ void __launch_bounds__(PT_TPB, 1) k_persist(const DevP *Ps, PArgs a) 
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *PT<T>::ks(P) = sk;
-        if (KIND == PK_REFINED) *P.ks = so;
+        s.g->rec[0] = sk;
+        s.g->rec[1] = so;
         s.g->steps = steps;
         s.g->iters = KIND == PK_REFINED ? so.it : sk.it;
     }
@@ -1358,7 +1359,7 @@ int persist_thread_blocks(int n) {
 // (the caller runs the per-pass path), -1 when a barrier wait ran out (the caller restores
 // the start and runs the per-pass path; the persistent path is off from then on).
 template <class T, int KIND>
-static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGrid *hres) {
+static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGridHead *hres) {
     static KInfo info;                           // per instantiation, cached
     static std::mutex mu;
     KInfo ki;
@@ -1466,8 +1467,12 @@ static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGrid 
         g_persist_broken = true;
         return 0;
     }
-    cudaMemcpyAsync(hres, g, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, c.st);
+    // (into pinned memory: a copy to pageable memory waits for the solve inside the driver and
+    // holds up other threads' launches, eight diodes on eight threads 143 -> 159 ms)
+    if (c.pin) cudaMemcpyAsync(c.pin, g, sizeof(PGridHead), cudaMemcpyDeviceToHost, c.st);
     cudaStreamSynchronize(c.st);
+    if (c.pin) *hres = *c.pin;
+    else cudaMemcpy(hres, g, sizeof(PGridHead), cudaMemcpyDeviceToHost);
     if (hres->err) {
         std::fprintf(stderr, "semisim-b200: persistent solve abandoned (a barrier wait ran out); per-pass solves "
                              "from now on\n");
@@ -1531,10 +1536,11 @@ static int persist_plan(const Ctx &c, const MGHost &mg, size_t *smem) {
     return L;
 }
 
-// Persistent forms of the solves of kernels_la.cu.  Each returns 1 (done: the Krylov
-// records hold the result), 0 (not applicable: nothing was changed) or -1 (abandoned: the
+// Persistent forms of the solves of kernels_la.cu; k: the starting Krylov record (it travels
+// with the launch's parameters) and the closing one (it comes back with the launch's status:
+// one copy and one wait a solve).  Each returns 1 (done), 0 (not applicable: nothing was changed) or -1 (abandoned: the
 // caller restores the start and uses the per-pass solve).
-int persist_pcg(const Ctx &c, const MGHost &mg, int mixed) {
+int persist_pcg(const Ctx &c, const MGHost &mg, int mixed, KrylovS &k) {
     if (c.ninst != 1 || !c.h.pwd || !persist_enabled()) return 0;
     size_t smem = 0;
     PArgs a{};
@@ -1545,9 +1551,11 @@ int persist_pcg(const Ctx &c, const MGHost &mg, int mixed) {
     a.sweeps2 = 0;                              // one application (MG_OVER, solver_ctx.h)
     a.alpha = mg.alpha * MG_OVER;
     a.barmode = g_barmode;
-    PGrid h{};
+    a.rec[0] = k;
+    PGridHead h{};
     const int rc = mixed ? persist_run<float, PK_PCG>(c, mg.maxN[1], smem, a, &h)
                          : persist_run<double, PK_PCG>(c, mg.maxN[1], smem, a, &h);
+    if (rc == 1) k = h.rec[0];
     if (rc == 1 && g_prof_on) {
         const double vb = mixed ? vcycle_bytes<float>(mg, a.Ls, a.deep, a.sweeps2)
                                 : vcycle_bytes<double>(mg, a.Ls, a.deep, a.sweeps2);
@@ -1558,7 +1566,7 @@ int persist_pcg(const Ctx &c, const MGHost &mg, int mixed) {
     }
     return rc;
 }
-int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int qsign) {
+int persist_bicg(const Ctx &c, const MGHost &mg, KrylovS &k, int qsign) {
     if (c.ninst != 1 || !c.h.pwd || !persist_enabled()) return 0;
     size_t smem = 0;
     PArgs a{};
@@ -1569,10 +1577,12 @@ int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int q
     a.sweeps2 = g_l0_sweeps > 1;
     a.alpha = mg.alpha;
     a.barmode = g_barmode;
-    a.rtol = rtol;
-    a.atol = atol;
-    PGrid h{};
+    a.rtol = k.rtol;
+    a.atol = k.atol;
+    a.rec[0] = k;
+    PGridHead h{};
     const int rc = persist_run<double, PK_BICG>(c, mg.maxN[1], smem, a, &h);
+    if (rc == 1) k = h.rec[0];
     if (rc == 1 && g_prof_on) {
         const double vb = vcycle_bytes<double>(mg, a.Ls, a.deep, a.sweeps2);
         const double kb = 2 * kProfBytesPerNode[PF_KRY_SPMV_DOT] + 4 * kProfBytesPerNode[PF_KRY_UPDATE];
@@ -1581,7 +1591,7 @@ int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int q
     }
     return rc;
 }
-int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign) {
+int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign, const KrylovS &inner, KrylovS &k) {
     if (c.ninst != 1 || !c.h.pwd || !persist_enabled()) return 0;
     size_t smem = 0;
     PArgs a{};
@@ -1593,9 +1603,12 @@ int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, in
     a.alpha = mg.alpha;
     a.barmode = g_barmode;
     a.maxsteps = maxsteps;
-    PGrid h{};
+    a.rec[0] = inner;
+    a.rec[1] = k;
+    PGridHead h{};
     const int rc = persist_run<float, PK_REFINED>(c, mg.maxN[1], smem, a, &h);
     if (rc == 1) {
+        k = h.rec[1];
         *steps = h.steps;
         if (g_prof_on) {
             const double vb = vcycle_bytes<float>(mg, a.Ls, a.deep, a.sweeps2);

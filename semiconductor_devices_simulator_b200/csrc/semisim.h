@@ -118,12 +118,16 @@ struct KrylovS {
 // Grid-wide barrier and reduction records of a persistent solve launch (one per
 // instance): the arrival counter (set to 0 before every launch), the error word (1: a
 // barrier wait ran out of time and every block left), the work done (V-cycles, Krylov
-// iterations, refinement steps) for the byte accounting, and two alternating buffers of
-// per-block reduction partials (up to 4 values per block).
+// iterations, refinement steps) for the byte accounting, the solve's closing Krylov records
+// (its own, and the refinement's), all of which the host reads back in one copy, and two
+// alternating buffers of per-block reduction partials (up to 4 values per block).
 constexpr int PG_MAXB = 512;
-struct PGrid {
+struct PGridHead {
     unsigned count, err;
     int vcycles, iters, steps, pad;
+    KrylovS rec[2];
+};
+struct PGrid : PGridHead {
     double red[2][PG_MAXB * 4];
 };
 

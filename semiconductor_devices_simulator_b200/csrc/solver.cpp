@@ -69,6 +69,7 @@ Ctx make_ctx(Inst &d) {
     c.zcap = d.tune.zcap;
     c.rq = d.tune.rq;
     c.pblocks = d.pblocks;
+    c.pin = d.g.pin ? reinterpret_cast<PGridHead *>(d.g.pin + 256) : nullptr;
     return c;
 }
 
@@ -285,7 +286,7 @@ static int gpu_alloc(Inst &d) {
     d.g.h = P;
     CK(cudaMalloc(&d.g.d, sizeof(DevP)));
     CK(cudaStreamCreateWithFlags(&d.g.st, cudaStreamNonBlocking));
-    CK(cudaMallocHost(&d.g.pin, sizeof(double) * 256));
+    CK(cudaMallocHost(&d.g.pin, sizeof(double) * 256 + sizeof(PGridHead)));
     CK(cudaMalloc(&d.g.scratch, sizeof(double) * (d.N > 0 ? d.N : 1)));
     CK(cudaMalloc(&d.g.flag, sizeof(int) * 16));
     for (int L = 0; L < nl; L++)                     // the kernels address A[q] as A[0] + q * apitch
@@ -1555,11 +1556,12 @@ static void load_state(Inst &d, double *const *h) {
 static int poisson_newton(Inst &d, const double *Va, double ntol, int maxit) {
     Ctx c = make_ctx(d);
     upload_voltages(d, Va);
+    double f0 = 0.;
     for (int it = 0; it < maxit; it++) {
         d.newton_its++;
         if (d.unstr) launch_poisson_g(c, nullptr, 1);
         else launch_poisson(c, nullptr, 1, nullptr);
-        const double f0 = read_res(d, R_PNORM);
+        if (!it) f0 = read_res(d, R_PNORM);                 // (later: the accepted trial's)
         if (!(f0 > 0.)) return f0 == 0.;
         launch_fill_sel(c, V_SOL, 0.0);
         const int maxp = d.max_iter_p > 0 ? d.max_iter_p : 2000;
@@ -1573,18 +1575,20 @@ static int poisson_newton(Inst &d, const double *Va, double ntol, int maxit) {
             launch_axpy_sel(c, V_PHI, V_PHI, 1.0, V_SOL);   // psi += dx
             return 1;
         }
-        double lam = 1.;
+        double lam = 1., fn = f0;
         for (int ls = 0; ls < 40; ls++) {
             launch_axpy_sel(c, V_TR, V_PHI, lam, V_SOL);    // trial psi + lam dx
             if (d.unstr) launch_poisson_g(c, d.g.h.tr, 0);
             else launch_poisson(c, d.g.h.tr, 0, nullptr);
             const double f1 = read_res(d, R_PNORM);
+            fn = f1;
             if (f1 <= (1. - 1e-4 * lam) * f0) break;
             lam *= 0.5;
         }
         cudaMemcpyAsync(d.g.h.phi, d.g.h.tr, d.N * 8, cudaMemcpyDeviceToDevice, d.g.st);
         if (d.verbose > 4) std::fprintf(stderr, "      newton it=%d f0=%.3e dm=%.3e lam=%.3e\n", it, f0, dm, lam);
         if (lam * dm < ntol) return 1;
+        f0 = fn;
     }
     return 0;
 }
@@ -1608,7 +1612,7 @@ static int solve_cont(Inst &d, int hole, double lo, double hi, double *dmax) {
     const long long s0 = t_ir_steps, f0 = t_ir_fallbacks;
     int its = d.unstr ? bicg_graph(d, maxit, d.bicg_rtol, atol, &rn, &r0, hole ? -1 : 1, false)
                       : bicgstab_core(c, d.g.mg, maxit, d.bicg_rtol, atol, 1, g_knobs.check_every, &rn, &r0,
-                                      hole ? -1 : 1, use_mixed(d));
+                                      hole ? -1 : 1, use_mixed(d), 1);
     d.ir_steps += t_ir_steps - s0;
     d.ir_fallbacks += t_ir_fallbacks - f0;
     if (!(rn <= std::fmax(r0, 1e-300)) && (d.unstr ? gmg_levels(d) > 1 : d.g.mg.maxlev > 1)) {

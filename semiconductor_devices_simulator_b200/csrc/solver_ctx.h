@@ -236,7 +236,7 @@ void launch_node_Jc_g(const Ctx &c, int which, double *out);
 void launch_emax_g(const Ctx &c);
 int pcg_graph(Inst &d, int maxit, double rtol);
 int bicg_graph(Inst &d, int maxit, double rtol, double atol, double *rn, double *r0, int qsign, bool ilu_only);
-int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qsign, bool ilu_only);
+int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qsign, bool ilu_only, KrylovS &k);
 // a level of the graph hierarchy on the host as the persistent solves' tables are built from it
 struct GpLevelIn {
     int N, ncolor;
@@ -292,15 +292,15 @@ void persist_set(int mode, int blocks);
 int persist_get_blocks();
 int persist_thread_blocks(int n);
 int live_instances();        // instances of the process with device memory (solver.cpp)
-int persist_pcg(const Ctx &c, const MGHost &mg, int mixed);
-int persist_bicg(const Ctx &c, const MGHost &mg, double rtol, double atol, int qsign);
-int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign);
+int persist_pcg(const Ctx &c, const MGHost &mg, int mixed, KrylovS &k);
+int persist_bicg(const Ctx &c, const MGHost &mg, KrylovS &k, int qsign);
+int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign, const KrylovS &inner, KrylovS &k);
 void vcycle_knobs_init();
 int persist_timeout_probe(const Ctx &c, int nb, double wait_s, int *gave_up);
 int persist_trace(int n, unsigned long long *out, int *blocks);
 extern int g_l0_sweeps, g_deep_levels;
 int bicgstab_core(const Ctx &c, const MGHost &mg, int maxit, double rtol, double atol, int mg_on, int check_every,
-                  double *rn, double *r0, int qsign, int mixed = 0);
+                  double *rn, double *r0, int qsign, int mixed = 0, int saved = 0);
 extern thread_local long long t_ir_steps, t_ir_fallbacks;   // refinement steps / FP64 take-overs
 extern double g_ir_factor, g_ir_rtol_min;
 void launch_absmax_sel(const Ctx &c, int xsel, int slot);
