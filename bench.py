@@ -375,9 +375,9 @@ def sweep_points(lib, w, s, fields=False, npts=None, out=None):
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic byte of a kernel
 # class on the default 120x80x60 mesh, from one ncu capture of the bench's --probe 10 case:
-# the persistent refined solve (k_persist<float, 2>, 10 BiCGSTAB iterations) moved 433.2 MB
-# of DRAM traffic for 4516 MB of algorithmic bytes (its hierarchy stays resident in the L2)
-NCU_DRAM_PER_ALG = {"persistent_solve_f32": 433.16e6 / 4516.1e6}
+# the persistent refined solve (k_persist<float, 2>, 10 BiCGSTAB iterations) moved 158.8 MB
+# of DRAM traffic for 3945 MB of algorithmic bytes (its hierarchy stays resident in the L2)
+NCU_DRAM_PER_ALG = {"persistent_solve_f32": 158.79e6 / 3944.6e6}
 
 
 def peaks():
@@ -822,7 +822,7 @@ def run_b200(a, dist):
                     "traffic_source": ("ncu DRAM bytes per algorithmic byte of this class on the probe case, "
                                        "times this run's algorithmic bytes per launch") if traffic else None,
                     "note": ("one cooperative launch per linear solve: its multigrid hierarchy and Krylov vectors "
-                             "stay in the 126 MB L2 (DRAM traffic about a tenth of the algorithmic bytes); "
+                             "stay in the 126 MB L2 (DRAM traffic 4 % of the algorithmic bytes); "
                              "the time goes to the grid barriers between dependent passes")
                             if top[0].startswith("persistent") else None}
             kernels = {r[0]: {"ms": round(r[1], 2), "share": round(r[1] / tot_ms, 4), "launches": r[2],
