@@ -211,7 +211,7 @@ struct DevP {
     double *part;                 // RED_MAX_BLOCKS*RED_AA
     unsigned *ticket;             // one counter per reduction slot (16)
     double *partc;                // terminal-current partials: 256 blocks x 96
-    double *ffbuf;                // floating-block sums: 6 x 1024
+    double *ffbuf;                // floating-block sums and scales: 6 x 1024
     int *ffint;                   // floating-block flags / counts / roots: 16 + 1024
     unsigned long long *ffacc;    // floating-block exact accumulators: 4 sums x 1024 x XS_WORDS
     double *res;                  // scalar results (64)
