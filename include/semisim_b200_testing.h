@@ -86,6 +86,10 @@ int b200x_persist_trace(int n, unsigned long long *out, int *blocks);
    hook): n > 0 caps the grid at n blocks, 0 removes the cap, n < 0 only reads it.  Returns
    the previous cap. */
 int b200x_persist_tblocks(int n);
+/* damped Newton-Poisson loop from the present state at the contact voltages now set, quasi-Fermi
+   levels fixed (semiconductor_3d.c:2791-2823); returns its verdict (1 converged), *norm the
+   ||F/diag|| of the potential it leaves */
+int b200x_poisson_newton(double ntol, int maxit, double *norm);
 /* floating-block balance of a continuity solution (in place) */
 int b200x_float_fix(int hole, double *sol);
 /* learned predictor on the present history arrays (22-24 h1, 25-27 e2 of b200x_set /

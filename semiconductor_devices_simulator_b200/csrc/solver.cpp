@@ -73,8 +73,8 @@ Ctx make_ctx(Inst &d) {
     return c;
 }
 
-static double read_res(Inst &d, int slot) {
-    cudaMemcpyAsync(d.g.pin, d.g.h.res + slot, sizeof(double), cudaMemcpyDeviceToHost, d.g.st);
+static double read_res(Inst &d, int slot, int n = 1) {     // slots slot .. slot + n-1 into pin; the first
+    cudaMemcpyAsync(d.g.pin, d.g.h.res + slot, n * sizeof(double), cudaMemcpyDeviceToHost, d.g.st);
     cudaStreamSynchronize(d.g.st);
     return d.g.pin[0];
 }
@@ -1553,42 +1553,42 @@ static void load_state(Inst &d, double *const *h) {
 // ------------------------------------------------------------------ Newton-Poisson
 // Damped Newton with PCG and a backtracking line search on ||F/diag||
 // (semiconductor_3d.c:2791-2823)
-static int poisson_newton(Inst &d, const double *Va, double ntol, int maxit) {
+int poisson_newton(Inst &d, const double *Va, double ntol, int maxit) {
     Ctx c = make_ctx(d);
     upload_voltages(d, Va);
-    double f0 = 0.;
     for (int it = 0; it < maxit; it++) {
         d.newton_its++;
         if (d.unstr) launch_poisson_g(c, nullptr, 1);
         else launch_poisson(c, nullptr, 1, nullptr);
-        if (!it) f0 = read_res(d, R_PNORM);                 // (later: the accepted trial's)
-        if (!(f0 > 0.)) return f0 == 0.;
         launch_fill_sel(c, V_SOL, 0.0);
         const int maxp = d.max_iter_p > 0 ? d.max_iter_p : 2000;
         const int its = d.unstr ? pcg_graph(d, maxp, d.pcg_rtol)
                                 : pcg_solve(c, d.g.mg, maxp, d.pcg_rtol, g_knobs.check_every, use_mixed(d));
         d.pcg_its += its;
         launch_absmax_sel(c, V_SOL, R_DMAX);
-        const double dm = read_res(d, R_DMAX);
+        // f0 in the scaling of the Jacobian just built, as the trials' norms are (an accepted
+        // trial's norm is in the scaling before it); one wait for both
+        static_assert(R_DMAX == R_PNORM + 1, "read together");
+        read_res(d, R_PNORM, 2);
+        const double f0 = d.g.pin[0], dm = d.g.pin[1];
+        if (!(f0 > 0.)) return f0 == 0.;
         if (dm != dm) return 0;
         if (dm < ntol) {
             launch_axpy_sel(c, V_PHI, V_PHI, 1.0, V_SOL);   // psi += dx
             return 1;
         }
-        double lam = 1., fn = f0;
+        double lam = 1.;
         for (int ls = 0; ls < 40; ls++) {
             launch_axpy_sel(c, V_TR, V_PHI, lam, V_SOL);    // trial psi + lam dx
             if (d.unstr) launch_poisson_g(c, d.g.h.tr, 0);
             else launch_poisson(c, d.g.h.tr, 0, nullptr);
             const double f1 = read_res(d, R_PNORM);
-            fn = f1;
             if (f1 <= (1. - 1e-4 * lam) * f0) break;
             lam *= 0.5;
         }
         cudaMemcpyAsync(d.g.h.phi, d.g.h.tr, d.N * 8, cudaMemcpyDeviceToDevice, d.g.st);
         if (d.verbose > 4) std::fprintf(stderr, "      newton it=%d f0=%.3e dm=%.3e lam=%.3e\n", it, f0, dm, lam);
         if (lam * dm < ntol) return 1;
-        f0 = fn;
     }
     return 0;
 }

@@ -210,6 +210,7 @@ bool gpu_available();
 int select_device(int dev);
 int prepare(Inst &d);
 int equilibrium(Inst &d);
+int poisson_newton(Inst &d, const double *Va, double ntol, int maxit);
 int run_continuation(Inst &d);
 int do_solve(Inst &d, int keep);
 void finish_point(Inst &d);

@@ -279,6 +279,19 @@ int b200x_pcg(int maxit, double rtol, double *sol) {
     sync(d);
     return its;
 }
+// the damped Newton-Poisson loop from the present state at the contact voltages now set;
+// returns its verdict, *norm the ||F/diag|| of the potential it leaves
+int b200x_poisson_newton(double ntol, int maxit, double *norm) {
+    Inst &d = *dev();
+    double Va[NC_MAX];
+    for (int c = 0; c < d.n_cons; c++) Va[c] = d.cons[c].V;
+    const int ok = poisson_newton(d, Va, ntol, maxit);
+    Ctx c = make_ctx(d);
+    if (d.unstr) launch_poisson_g(c, nullptr, 1);
+    else launch_poisson(c, nullptr, 1, nullptr);
+    *norm = res(d, R_PNORM);
+    return ok;
+}
 int b200x_float_fix(int hole, double *sol) {
     Inst &d = *dev();
     cudaMemcpyAsync(d.g.h.sol, sol, d.N * 8, cudaMemcpyHostToDevice, d.g.st);
