@@ -624,9 +624,16 @@ __global__ void __launch_bounds__(GP_TPB, 1) k_gpersist(const DevP *Ps, GPArgs g
         const double rk = bk - sum;
         r[t] = rk;
         if (a.kind) { rh[t] = rk; p[t] = rk; }
+        // a sweep from zero multiplies what lies in its rows by the zero coupling of their padding
+        // slots before it has written them: nothing an earlier solve left there may be a NaN or Inf
+        // (tests for the padding in the sweeps instead cost 5 % of a solve)
+        (a.kind ? P.wk[4] : P.wk[1])[t] = 0.0;
+        if (a.kind) P.wk[5][t] = 0.0;
         acc[0] += rk * rk;
         acc[1] += fl * fl;
     }
+    for (int L = 1; L < a.nl - 1; L++)
+        for (int t = s.tid; t < lt[L].N; t += s.nth) lt[L].x[t] = 0.0;
     if (a.nl > 1 && !a.ilu_only) gp_weights(P, H0, lt[1], 0, a.qsign, s.tid, s.nth);
     {
         double a2[2] = {acc[0], acc[1]};
