@@ -77,6 +77,10 @@ int b200x_pcg(int maxit, double rtol, double *sol);
    Returns the error word (1 when the others gave up after wait_s seconds) and in
    *gave_up how many blocks reported it (nb - 1); -1 if the launch failed. */
 int b200x_persist_probe(int nb, double wait_s, int *gave_up);
+/* The host's verdict on a persistent solve's closing record when the solve before ended well: the
+   CUDA codes of its copy and of the wait, whether the record arrives, and its error word.
+   Returns 1 (taken) or -1 (refused); uses no GPU. */
+int b200x_persist_record(int copy, int wait, int arrives, int err);
 /* Barrier timeline of the next persistent solve (measurement hook): n > 0 arms a timeline of
    n barriers (returns 0); n == 0 copies it to out - per barrier the first and the last
    block's arrival and the release as block 0 saw it (globaltimer ns) - disarms it and

@@ -1040,15 +1040,13 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
         cudaGetLastError();
         return 0;
     }
-    const PGridHead &h = *c.pin;                  // status and closing record in one copy
-    cudaMemcpyAsync(c.pin, g, sizeof(PGridHead), cudaMemcpyDeviceToHost, c.st);
-    cudaStreamSynchronize(c.st);
-    k = h.rec[0];
-    if (h.err) {
-        std::fprintf(stderr, "semisim-b200: persistent graph solve abandoned (a barrier wait ran out)\n");
-        return -1;
-    }
-    return 1;
+    PGridHead h{};                                // status and closing record in one copy
+    const int rc = persist_record(c, g, &h);
+    if (rc == 1) k = h.rec[0];
+    else
+        std::fprintf(stderr, "semisim-b200: persistent graph solve abandoned (%s)\n",
+                     h.err == 1 ? "a barrier wait ran out" : "its closing record did not arrive");
+    return rc;
 }
 
 }  // namespace ss

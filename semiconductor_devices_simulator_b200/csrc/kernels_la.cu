@@ -1113,8 +1113,12 @@ bool g_use_graphs = true;
 
 static KrylovS read_ks(const Ctx &c, const KrylovS *src) {
     KrylovS hs{};
-    cudaMemcpyAsync(&hs, src, sizeof(KrylovS), cudaMemcpyDeviceToHost, c.st);
-    cudaStreamSynchronize(c.st);
+    const cudaError_t copy = cudaMemcpyAsync(&hs, src, sizeof(KrylovS), cudaMemcpyDeviceToHost, c.st);
+    if (cudaStreamSynchronize(c.st) != cudaSuccess || copy != cudaSuccess) {
+        hs = KrylovS{};                           // a device error: no residual that could pass for a solution's
+        hs.rr = NAN;
+        hs.status = 2;
+    }
     return hs;
 }
 

@@ -1353,6 +1353,33 @@ int persist_thread_blocks(int n) {
     return old;
 }
 
+// The closing record of a launch: `rec` is the instance's landing place, which keeps the record of
+// the solve before, so its error word is set before the copy and a copy or wait that failed, or a
+// record that never landed, is no result.  1: arrived and sound, -1: not
+static void record_arm(PGridHead *rec) { rec->err = PG_NO_RECORD; }
+static int record_take(cudaError_t copy, cudaError_t wait, PGridHead *rec) {
+    if (copy != cudaSuccess || wait != cudaSuccess) rec->err = PG_NO_RECORD;
+    return rec->err ? -1 : 1;
+}
+// (into pinned memory: a copy to pageable memory waits for the solve inside the driver and
+// holds up other threads' launches, eight diodes on eight threads 143 -> 159 ms)
+int persist_record(const Ctx &c, const PGrid *g, PGridHead *out) {
+    PGridHead *rec = c.pin ? c.pin : out;
+    record_arm(rec);
+    const cudaError_t copy = cudaMemcpyAsync(rec, g, sizeof(PGridHead), cudaMemcpyDeviceToHost, c.st);
+    const cudaError_t wait = cudaStreamSynchronize(c.st);
+    const int rc = record_take(copy, wait, rec);
+    if (rec != out) *out = *rec;
+    return rc;
+}
+int persist_record_probe(int copy, int wait, int arrives, unsigned err) {
+    PGridHead rec{};                               // the solve before ended well
+    rec.rec[0].status = 1;
+    record_arm(&rec);
+    if (arrives) rec.err = err;
+    return record_take((cudaError_t)copy, (cudaError_t)wait, &rec);
+}
+
 // Launch the persistent solve `kind` of precision T on instance 0 of the context (n1: nodes of
 // level 1).  Returns
 // 1 when it ran (results in the Krylov records), 0 when the persistent path does not apply
@@ -1467,19 +1494,13 @@ static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGridH
         g_persist_broken = true;
         return 0;
     }
-    // (into pinned memory: a copy to pageable memory waits for the solve inside the driver and
-    // holds up other threads' launches, eight diodes on eight threads 143 -> 159 ms)
-    if (c.pin) cudaMemcpyAsync(c.pin, g, sizeof(PGridHead), cudaMemcpyDeviceToHost, c.st);
-    cudaStreamSynchronize(c.st);
-    if (c.pin) *hres = *c.pin;
-    else cudaMemcpy(hres, g, sizeof(PGridHead), cudaMemcpyDeviceToHost);
-    if (hres->err) {
-        std::fprintf(stderr, "semisim-b200: persistent solve abandoned (a barrier wait ran out); per-pass solves "
-                             "from now on\n");
+    const int rc = persist_record(c, g, hres);
+    if (rc < 0) {
+        std::fprintf(stderr, "semisim-b200: persistent solve abandoned (%s); per-pass solves from now on\n",
+                     hres->err == 1 ? "a barrier wait ran out" : "its closing record did not arrive");
         g_persist_broken = true;
-        return -1;
     }
-    return 1;
+    return rc;
 }
 
 // algorithmic bytes of one V-cycle of precision T (the passes the persistent kernel runs): a

@@ -122,6 +122,7 @@ struct KrylovS {
 // (its own, and the refinement's), all of which the host reads back in one copy, and two
 // alternating buffers of per-block reduction partials (up to 4 values per block).
 constexpr int PG_MAXB = 512;
+constexpr unsigned PG_NO_RECORD = 2;     // error word of a record that has not come back (host only)
 struct PGridHead {
     unsigned count, err;
     int vcycles, iters, steps, pad;

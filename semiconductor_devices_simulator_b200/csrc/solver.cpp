@@ -74,8 +74,9 @@ Ctx make_ctx(Inst &d) {
 }
 
 static double read_res(Inst &d, int slot, int n = 1) {     // slots slot .. slot + n-1 into pin; the first
-    cudaMemcpyAsync(d.g.pin, d.g.h.res + slot, n * sizeof(double), cudaMemcpyDeviceToHost, d.g.st);
-    cudaStreamSynchronize(d.g.st);
+    const cudaError_t copy = cudaMemcpyAsync(d.g.pin, d.g.h.res + slot, n * sizeof(double), cudaMemcpyDeviceToHost, d.g.st);
+    if (cudaStreamSynchronize(d.g.st) != cudaSuccess || copy != cudaSuccess)
+        for (int q = 0; q < n; q++) d.g.pin[q] = NAN;       // a device error: not the value read before
     return d.g.pin[0];
 }
 

@@ -296,6 +296,10 @@ int live_instances();        // instances of the process with device memory (sol
 int persist_pcg(const Ctx &c, const MGHost &mg, int mixed, KrylovS &k);
 int persist_bicg(const Ctx &c, const MGHost &mg, KrylovS &k, int qsign);
 int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign, const KrylovS &inner, KrylovS &k);
+// the closing record of the launch on c's stream in one copy and one wait: 1 arrived, -1 abandoned
+// (out->err 1: a barrier wait ran out, PG_NO_RECORD: a device error, nothing arrived)
+int persist_record(const Ctx &c, const PGrid *g, PGridHead *out);
+int persist_record_probe(int copy, int wait, int arrives, unsigned err);
 void vcycle_knobs_init();
 int persist_timeout_probe(const Ctx &c, int nb, double wait_s, int *gave_up);
 int persist_trace(int n, unsigned long long *out, int *blocks);

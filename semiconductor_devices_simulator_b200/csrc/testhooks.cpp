@@ -263,6 +263,11 @@ int b200x_persist_probe(int nb, double wait_s, int *gave_up) {
     Ctx c = make_ctx(d);
     return persist_timeout_probe(c, nb, wait_s, gave_up);
 }
+// the host's verdict on a solve's closing record after a solve that ended well: CUDA codes of the
+// copy and the wait, whether the record arrives and its error word; 1 taken, -1 refused (no GPU used)
+int b200x_persist_record(int copy, int wait, int arrives, int err) {
+    return persist_record_probe(copy, wait, arrives, (unsigned)err);
+}
 // barrier timeline of the next persistent solve: n > 0 arms it, n == 0 reads it (3 n
 // values per barrier: first arrival, last arrival, release; ns) and the launch's blocks
 int b200x_persist_trace(int n, unsigned long long *out, int *blocks) { return persist_trace(n, out, blocks); }
