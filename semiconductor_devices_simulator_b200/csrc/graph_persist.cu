@@ -704,22 +704,10 @@ __global__ void __launch_bounds__(GP_TPB, 1) k_gpersist(const DevP *Ps, GPArgs g
     } else {                                      // BiCGSTAB (gbicgstab)
         double *v = P.wk[3], *ph = P.wk[4], *sh = P.wk[5], *u = P.wk[6];
         // (u serves the V-cycles as the post-smoothing's vector and then holds t = A sh)
+        if (threadIdx.x == 0) bicg_next(sk);      // (before the barrier: kernels_persist.cu)
+        __syncthreads();
         while (sk.active) {
             double a1[1], a2[2];
-            if (threadIdx.x == 0) {
-                if (sk.it >= sk.maxit) { sk.active = 0; sk.status = 3; }
-                else {
-                    sk.it++;
-                    sk.pad0 = 0;
-                    if (fabs(sk.rho1) < 1e-300) {  // breakdown: restart the shadow residual
-                        sk.rho1 = sk.rr;
-                        sk.pad0 = 1;
-                        if (!(sk.rho1 > 0.0)) { sk.active = 0; sk.status = 2; }
-                    }
-                }
-            }
-            __syncthreads();
-            if (!sk.active) break;
             if (sk.pad0) {
                 for (int t = s.tid; t < N; t += s.nth) { rh[t] = r[t]; p[t] = r[t]; }
                 if (!pg_sync(s)) return;
@@ -795,6 +783,7 @@ __global__ void __launch_bounds__(GP_TPB, 1) k_gpersist(const DevP *Ps, GPArgs g
                     if (rn < 0.99 * sk.rbest) { sk.rbest = rn; sk.stall = 0; }
                     else if (++sk.stall > 40) { sk.active = 0; sk.status = 2; }
                 }
+                bicg_next(sk);
             }
             __syncthreads();
         }

@@ -484,22 +484,12 @@ __device__ bool pg_bicg(PS &s, const PArgs &a, PTab<T> &tb, int nl, KrylovS &sk)
     const int H = tb.w.lev[0].H, np = H >> 1;               // pairs of slots per colour
     const T *Dr = tb.w.lev[0].D;
     bool first = true;
+    // (thread 0 decides on the next iteration before the block barrier ahead of the loop's test, not
+    // after the test: a warp late at it would read the later decision and leave a barrier early)
+    if (threadIdx.x == 0) bicg_next(sk);
+    __syncthreads();
     while (sk.active) {
         double acc[3], a1[1], a2[2];
-        if (threadIdx.x == 0) {
-            if (sk.it >= sk.maxit) { sk.active = 0; sk.status = 3; }
-            else {
-                sk.it++;
-                sk.pad0 = 0;
-                if (fabs(sk.rho1) < 1e-300) {               // breakdown: restart the shadow residual
-                    sk.rho1 = sk.rr;
-                    sk.pad0 = 1;
-                    if (!(sk.rho1 > 0.0)) { sk.active = 0; sk.status = 2; }
-                }
-            }
-        }
-        __syncthreads();
-        if (!sk.active) break;
         if (sk.pad0) {
             for (int q = s.tid; q < 2 * np; q += s.nth) {
                 const int m = 2 * q;
@@ -613,6 +603,7 @@ __device__ bool pg_bicg(PS &s, const PArgs &a, PTab<T> &tb, int nl, KrylovS &sk)
                 if (rn < 0.99 * sk.rbest) { sk.rbest = rn; sk.stall = 0; }
                 else if (++sk.stall > 40) { sk.active = 0; sk.status = 2; }
             }
+            bicg_next(sk);
         }
         __syncthreads();
     }

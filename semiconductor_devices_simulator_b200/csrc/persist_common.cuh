@@ -138,5 +138,18 @@ __device__ __forceinline__ bool pg_sum(PS &s, double (&v)[NV], F idle = F()) {
     return true;
 }
 
+// The start of the next BiCGSTAB iteration on an active record, by one thread: the iteration cap
+// (status 3), and the shadow residual's restart after a breakdown (pad0; status 2 at a zero residual)
+__device__ __forceinline__ void bicg_next(KrylovS &sk) {
+    if (!sk.active) return;
+    if (sk.it >= sk.maxit) { sk.active = 0; sk.status = 3; return; }
+    sk.it++;
+    sk.pad0 = 0;
+    if (fabs(sk.rho1) < 1e-300) {
+        sk.rho1 = sk.rr;
+        sk.pad0 = 1;
+        if (!(sk.rho1 > 0.0)) { sk.active = 0; sk.status = 2; }
+    }
+}
 
 }  // namespace ss

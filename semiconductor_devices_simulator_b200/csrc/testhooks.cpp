@@ -251,7 +251,8 @@ int b200x_bicgstab(int maxit, double rtol, double atol, int qsign, const double 
     Ctx c = make_ctx(d);
     if (x0) cudaMemcpyAsync(d.g.h.sol, x0, d.N * 8, cudaMemcpyHostToDevice, d.g.st);
     else launch_fill_sel(c, V_SOL, 1.0);
-    const int its = bicgstab_core(c, d.g.mg, maxit, rtol, atol, 1, 1, rn, r0, qsign, use_mixed(d));
+    const int its = d.unstr ? bicg_graph(d, maxit, rtol, atol, rn, r0, qsign, false)
+                            : bicgstab_core(c, d.g.mg, maxit, rtol, atol, 1, 1, rn, r0, qsign, use_mixed(d));
     if (sol) cudaMemcpyAsync(sol, d.g.h.sol, d.N * 8, cudaMemcpyDeviceToHost, d.g.st);
     sync(d);
     return its;
@@ -279,7 +280,7 @@ int b200x_pcg(int maxit, double rtol, double *sol) {
     Inst &d = *dev();
     Ctx c = make_ctx(d);
     launch_fill_sel(c, V_SOL, 0.0);
-    const int its = pcg_solve(c, d.g.mg, maxit, rtol, 1, use_mixed(d));
+    const int its = d.unstr ? pcg_graph(d, maxit, rtol) : pcg_solve(c, d.g.mg, maxit, rtol, 1, use_mixed(d));
     if (sol) cudaMemcpyAsync(sol, d.g.h.sol, d.N * 8, cudaMemcpyDeviceToHost, d.g.st);
     sync(d);
     return its;
