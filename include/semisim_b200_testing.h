@@ -77,6 +77,9 @@ int b200x_pcg(int maxit, double rtol, double *sol);
    Returns the error word (1 when the others gave up after wait_s seconds) and in
    *gave_up how many blocks reported it (nb - 1); -1 if the launch failed. */
 int b200x_persist_probe(int nb, double wait_s, int *gave_up);
+/* Blocks of the calling thread's last persistent launch since the last call, and the CTAs of its
+   thread-block clusters (0: a plain grid); 0 blocks: no persistent solve was launched. */
+void b200x_persist_shape(int *blocks, int *cluster);
 /* The host's verdict on a persistent solve's closing record when the solve before ended well: the
    CUDA codes of its copy and of the wait, whether the record arrives, and its error word.
    Returns 1 (taken) or -1 (refused); uses no GPU. */

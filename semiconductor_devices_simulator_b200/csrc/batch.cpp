@@ -36,6 +36,7 @@ int clone_into(Inst &w, Inst &src) {
     w.cache.clear();
     w.cache_ok.clear();
     w.seed_on = 0;                             // the learned model stays with the source
+    w.batched = 1;
     if (!prepare(w)) return 0;
     w.clone_src = &src;
     w.clone_gen = src.upload_gen;

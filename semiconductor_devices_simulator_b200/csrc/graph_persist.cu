@@ -1029,6 +1029,7 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
         cudaGetLastError();
         return 0;
     }
+    persist_note(nb, cluster ? GP_CL : 0);
     PGridHead h{};                                // status and closing record in one copy
     const int rc = persist_record(c, g, &h);
     if (rc == 1) k = h.rec[0];

@@ -32,6 +32,7 @@ struct Ctx {
     int rq = 1;                 // coarse rows per block of the residual + restriction pass
     int small_nodes = 0;        // levels at or below this size go to the small-level kernel (0: default)
     int pblocks = 0;            // blocks of the instance's persistent solves (0: the library-wide cap)
+    int batched = 0;            // its solves run beside those of a batched resolve's other workers
     PGridHead *pin = nullptr;   // pinned landing place of a persistent solve's status
     int nodes_blocks() const;
 };

@@ -1267,6 +1267,7 @@ bool g_coop_ok = false;    // the device supports cooperative launches
 unsigned long long *g_trace = nullptr;   // armed barrier timeline (test hook): device buffer
 int g_trace_n = 0, g_trace_used = 0;     // its barriers; 1 once a launch has filled it
 int g_last_blocks = 0;                   // blocks of the last persistent launch
+thread_local int t_shape[2];             // blocks and cluster CTAs of this host thread's last one (test hook)
 int g_barmode = 1;         // grid-barrier form (SEMISIM_B200_BARMODE; 1 measured faster than 0)
 int g_clusters = 1;        // cluster launches: 0 off, 1 where they gain (persist_run), 2 every grid (SEMISIM_B200_CLUSTERS)
 int g_csz = 16;            // CTAs per cluster at most (SEMISIM_B200_CSZ: 8 portable, 16 non-portable)
@@ -1336,6 +1337,12 @@ void persist_set(int mode, int blocks) {
     std::lock_guard<std::mutex> lk(g_pmu);
     if (mode >= 0) g_persist_mode = mode ? 1 : 0;
     if (blocks >= 0) g_persist_blocks = blocks;
+}
+void persist_note(int blocks, int csz) { t_shape[0] = blocks; t_shape[1] = csz; }
+void persist_shape(int *blocks, int *csz) {
+    *blocks = t_shape[0];
+    *csz = t_shape[1];
+    t_shape[0] = t_shape[1] = 0;
 }
 int persist_get_blocks() { return g_persist_blocks; }
 int persist_thread_blocks(int n) {
@@ -1413,9 +1420,10 @@ static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGridH
     // 0 misses the SMs that no whole cluster covers (112 of 148 blocks): 230,400 nodes FP64 101.1
     // -> 103.1, 336,000 118.2 -> 124.9 (FP32 98.4 -> 103.2); clusters of 8 for that part lose
     // from 180,000 nodes on (101.2).  Only seven clusters of 16 fit the GPU: where fewer such
-    // grids than plain ones run side by side and the process has instances enough to notice, the
-    // grid stays plain (six 36,864-node instances: 74 ms plain, 82 in clusters of 16), as do
-    // capped grids, which share the SMs by blocks.
+    // grids than plain ones run side by side, a batched resolve's workers take plain grids (six
+    // of 36,864 nodes: 74 ms plain, 82 in clusters of 16), as do capped grids, which share the SMs by
+    // blocks.  Nothing else of the process enters the choice: the order of the reductions follows
+    // from the solve's size and the caller's own settings.
     PArgs aa = a;
     aa.csz = 0;
     aa.onecl = 0;
@@ -1431,7 +1439,7 @@ static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGridH
     } else if (g_clusters == 1 && c16 > 0 && !capped && n1 <= per * 16 * PT_TPB) {
         ncl = std::max(1, std::min(nb / 16, c16));
         if (2 * nb <= ki.blocks && ncl > 3) ncl = 3;        // two of these grids run side by side
-        if (ki.blocks / nb <= c16 / ncl || live_instances() * ncl <= c16) csz = 16;
+        if (!c.batched || ki.blocks / nb <= c16 / ncl) csz = 16;
     }
     if (csz) {
         nb = ncl * csz;
@@ -1485,6 +1493,7 @@ static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGridH
         g_persist_broken = true;
         return 0;
     }
+    persist_note(nb, aa.csz);
     const int rc = persist_record(c, g, hres);
     if (rc < 0) {
         std::fprintf(stderr, "semisim-b200: persistent solve abandoned (%s); per-pass solves from now on\n",

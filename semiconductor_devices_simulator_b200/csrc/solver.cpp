@@ -69,6 +69,7 @@ Ctx make_ctx(Inst &d) {
     c.zcap = d.tune.zcap;
     c.rq = d.tune.rq;
     c.pblocks = d.pblocks;
+    c.batched = d.batched;
     c.pin = d.g.pin ? reinterpret_cast<PGridHead *>(d.g.pin + 256) : nullptr;
     return c;
 }
@@ -211,11 +212,7 @@ int mg_levels(int Nx, int Ny, int Nz, int dims[][6]) {
     return nl;
 }
 
-// instances of this process with their device memory set up
-static std::atomic<int> g_live{0};
-int live_instances() { return g_live.load(); }
 void gpu_free(Inst &d) {
-    if (d.g.ready) g_live--;
     for (auto &e : d.g.lg.exec)
         if (e) cudaGraphExecDestroy(e);
     for (auto &e : d.g.tev)
@@ -312,7 +309,6 @@ static int gpu_alloc(Inst &d) {
         mg.maxRows[L] = levs[L].Ny * levs[L].Nz;
     }
     d.g.ready = true;
-    g_live++;
     return 1;
 }
 

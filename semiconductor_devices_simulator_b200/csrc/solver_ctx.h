@@ -153,6 +153,7 @@ struct Inst {
     long long ir_steps = 0, ir_fallbacks = 0;
     Tune tune;
     int pblocks = 0;             // grid share of its persistent solves (api3b_set_share; 0: none)
+    int batched = 0;             // worker of a batched resolve: its solves run beside others'
     unsigned long long upload_gen = 0;      // set-up upload this instance's device holds (prepare)
     const Inst *clone_src = nullptr;        // batched-resolve worker: the instance and upload
     unsigned long long clone_gen = 0;       //   generation its set-up was copied from
@@ -292,13 +293,16 @@ int persist_enabled();
 void persist_set(int mode, int blocks);
 int persist_get_blocks();
 int persist_thread_blocks(int n);
-int live_instances();        // instances of the process with device memory (solver.cpp)
 int persist_pcg(const Ctx &c, const MGHost &mg, int mixed, KrylovS &k);
 int persist_bicg(const Ctx &c, const MGHost &mg, KrylovS &k, int qsign);
 int persist_refined(const Ctx &c, const MGHost &mg, int maxsteps, int *steps, int qsign, const KrylovS &inner, KrylovS &k);
 // the closing record of the launch on c's stream in one copy and one wait: 1 arrived, -1 abandoned
 // (out->err 1: a barrier wait ran out, PG_NO_RECORD: a device error, nothing arrived)
 int persist_record(const Ctx &c, const PGrid *g, PGridHead *out);
+// blocks and cluster CTAs (0: none) of the calling thread's last persistent launch, noted by the
+// launch and forgotten by the reading (0, 0: no launch since)
+void persist_note(int blocks, int csz);
+void persist_shape(int *blocks, int *csz);
 int persist_record_probe(int copy, int wait, int arrives, unsigned err);
 void vcycle_knobs_init();
 int persist_timeout_probe(const Ctx &c, int nb, double wait_s, int *gave_up);

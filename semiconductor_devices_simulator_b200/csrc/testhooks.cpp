@@ -264,6 +264,8 @@ int b200x_persist_probe(int nb, double wait_s, int *gave_up) {
     Ctx c = make_ctx(d);
     return persist_timeout_probe(c, nb, wait_s, gave_up);
 }
+// blocks and cluster CTAs of the calling thread's last persistent launch since the last call (0: none)
+void b200x_persist_shape(int *blocks, int *cluster) { persist_shape(blocks, cluster); }
 // the host's verdict on a solve's closing record after a solve that ended well: CUDA codes of the
 // copy and the wait, whether the record arrives and its error word; 1 taken, -1 refused (no GPU used)
 int b200x_persist_record(int copy, int wait, int arrives, int err) {
