@@ -979,13 +979,12 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
     int nb = g_gp_blocks;
     const int want = (int)((d.N + GP_TPB - 1) / GP_TPB);
     if (want < nb) nb = want < 4 ? 4 : want;
-    const int cap = persist_get_blocks();
-    if (cap > 0 && cap < nb) nb = cap;
-    if (d.pblocks > 0 && d.pblocks < nb) nb = d.pblocks;
-    if (nb > PG_MAXB) nb = PG_MAXB;
+    const int cap = persist_cap(d.pblocks);
+    if (cap < nb) nb = cap;
     if (nb < 1) return 0;
-    const bool cluster = g_gp_clusters > 0 && (nb <= GP_CL || d.N <= (size_t)GP_CLUSTER_N);
-    if (cluster) nb = GP_CL;
+    // one cluster of GP_CL blocks, or of what a smaller cap allows
+    const int csz = g_gp_clusters > 0 && (nb <= GP_CL || d.N <= (size_t)GP_CLUSTER_N) ? persist_one_cluster(cap) : 0;
+    if (csz) nb = csz;
     Ctx c = make_ctx(d);
     KrylovS ks0{};
     ks0.maxit = maxit;
@@ -1002,7 +1001,7 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
     a.kind = kind;
     a.ilu_only = ilu_only ? 1 : 0;
     a.qsign = qsign;
-    a.onecl = cluster ? 1 : 0;
+    a.onecl = csz ? 1 : 0;
     a.alpha = kind ? g_knobs.mg_alpha : g_knobs.mg_alpha * MG_OVER;
     a.rtol = rtol;
     a.atol = atol;
@@ -1020,16 +1019,16 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = GP_CL; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    at[1].val.clusterDim.x = csz; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = cluster ? 2 : 1;
+    cfg.numAttrs = csz ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelExC(&cfg, (const void *)k_gpersist, args);
     if (g_prof_on) prof_end(PF_PERSIST, c.st, 0.0);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
-    persist_note(nb, cluster ? GP_CL : 0);
+    persist_note(nb, csz);
     PGridHead h{};                                // status and closing record in one copy
     const int rc = persist_record(c, g, &h);
     if (rc == 1) k = h.rec[0];

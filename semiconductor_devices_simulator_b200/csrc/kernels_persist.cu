@@ -1344,7 +1344,15 @@ void persist_shape(int *blocks, int *csz) {
     *csz = t_shape[1];
     t_shape[0] = t_shape[1] = 0;
 }
-int persist_get_blocks() { return g_persist_blocks; }
+// the smallest of the caps on a launch's blocks: library-wide, the host thread's, and `share`
+int persist_cap(int share) {
+    int cap = PG_MAXB;
+    for (int b : {g_persist_blocks, t_persist_blocks, share})
+        if (b > 0 && b < cap) cap = b;
+    return cap;
+}
+// CTAs of a one-cluster grid within the cap (0: a single block, no cluster)
+int persist_one_cluster(int cap) { return cap >= 8 ? 8 : cap >= 4 ? 4 : cap >= 2 ? 2 : 0; }
 int persist_thread_blocks(int n) {
     const int old = t_persist_blocks;
     if (n >= 0) t_persist_blocks = n;
@@ -1405,13 +1413,11 @@ static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGridH
     // instances' solves can run side by side
     const int want = (c.maxN + 2 * PT_TPB - 1) / (2 * PT_TPB);
     if (want < nb) nb = want < 4 ? 4 : want;
-    if (g_persist_blocks > 0 && g_persist_blocks < nb) nb = g_persist_blocks;
-    if (c.pblocks > 0 && c.pblocks < nb) nb = c.pblocks;
-    if (t_persist_blocks > 0 && t_persist_blocks < nb) nb = t_persist_blocks;
-    if (nb > PG_MAXB) nb = PG_MAXB;
+    const int cap = persist_cap(c.pblocks);
+    if (cap < nb) nb = cap;
     if (nb < 1) return 0;
-    // Clusters.  A grid of at most 8 blocks becomes one cluster of 8 CTAs, up to 31 blocks' worth
-    // one of 16: its barriers are cluster barriers, 0.3 us against 1.2-1.5 us for a grid barrier
+    // Clusters.  A grid of at most 8 blocks becomes one cluster of 8 CTAs (under a cap below 8 of 4
+    // or 2: a cap is a promise to the solves next to it), up to 31 blocks' worth one of 16: its barriers are cluster barriers, 0.3 us against 1.2-1.5 us for a grid barrier
     // (11,520 / 16,128 / 28,672 nodes FP64 38.9 / 39.9 / 45.3 -> 33.6 / 35.9 / 41.0 ms a sweep).  A larger grid is
     // a whole number of 16-CTA clusters, the first of which runs level 1 .. Ls-1 alone, while
     // level 1 has at most three (FP32: four) nodes a thread of that cluster: 64,000 nodes 82.5 ->
@@ -1432,10 +1438,10 @@ static int persist_run(const Ctx &c, int n1, size_t smem, const PArgs &a, PGridH
     const int c16 = ki.clusters[1], per = sizeof(T) == 4 ? 4 : 3;
     int csz = 0, ncl = 1;
     if (g_clusters && ki.clusters[0] > 0 && nb <= 8) {
-        csz = 8;
+        csz = persist_one_cluster(cap);
     } else if (g_clusters == 2 && (c16 > 0 || ki.clusters[0] > 0)) {
-        csz = c16 > 0 ? 16 : 8;
-        ncl = std::max(1, std::min(nb / csz, c16 > 0 ? c16 : ki.clusters[0]));
+        csz = c16 > 0 && cap >= 16 ? 16 : 8;
+        ncl = std::max(1, std::min(nb / csz, csz > 8 ? c16 : ki.clusters[0]));
     } else if (g_clusters == 1 && c16 > 0 && !capped && n1 <= per * 16 * PT_TPB) {
         ncl = std::max(1, std::min(nb / 16, c16));
         if (2 * nb <= ki.blocks && ncl > 3) ncl = 3;        // two of these grids run side by side

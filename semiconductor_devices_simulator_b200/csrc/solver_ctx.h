@@ -291,7 +291,8 @@ template <class T>
 size_t persist_work_layout(char *base, const int dims[][6], int nlev, SWork<T> *w);
 int persist_enabled();
 void persist_set(int mode, int blocks);
-int persist_get_blocks();
+int persist_cap(int share);
+int persist_one_cluster(int cap);
 int persist_thread_blocks(int n);
 int persist_pcg(const Ctx &c, const MGHost &mg, int mixed, KrylovS &k);
 int persist_bicg(const Ctx &c, const MGHost &mg, KrylovS &k, int qsign);
