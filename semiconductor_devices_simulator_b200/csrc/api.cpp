@@ -140,7 +140,7 @@ void api3_init(void) {                                      // semiconductor_3d.
     d.models = 7;
     d.caxis = 1;
     const char *v = env_get("SEMISIM_VERBOSE"); d.verbose = v ? std::atoi(v) : 0;
-    const char *a = env_get("SEMISIM_MGA"); if (a) g_knobs.mg_alpha = std::atof(a);
+    const char *a = env_get("SEMISIM_MGA"); if (a) g_knobs.mg_alpha = g_knobs.mg_alpha_p = std::atof(a);
     if (const char *m = env_get("SEMISIM_GPASS")) g_knobs.gpass = std::atoi(m);
     if (const char *m = env_get("SEMISIM_GBETA")) g_knobs.gbeta = std::atof(m);
     if (const char *m = env_get("SEMISIM_AAM")) { int q = std::atoi(m); g_knobs.aa_depth = q < 0 ? 0 : (q > AA_MAX ? AA_MAX : q); }

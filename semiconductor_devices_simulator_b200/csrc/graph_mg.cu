@@ -586,7 +586,7 @@ void vcycle(Inst &d, const Ctx &c, int L, const double *b, double *x, const doub
               L == 0 ? w : nullptr);
     vcycle(d, c, L + 1, cv.b, cv.x, w, false);
     SS_LAUNCH(PF_PROLONG, v.N, k_gmg_prolong, grid_for(v.N), TPB, c.st, v, cv.x, x,
-              w ? g_knobs.mg_alpha : g_knobs.mg_alpha * MG_OVER);
+              w ? g_knobs.mg_alpha : g_knobs.mg_alpha_p);
     matvec_L(c, v, x, b, v.r);                            // post-smoothing
     ilu_apply(d, c, L, v.r, v.r);
     SS_LAUNCH(PF_PROLONG, v.N, k_gmg_add, grid_for(v.N), TPB, c.st, v.N, x, v.r);

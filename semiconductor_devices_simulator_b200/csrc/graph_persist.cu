@@ -1002,7 +1002,7 @@ int persist_graph(Inst &d, int kind, int maxit, double rtol, double atol, int qs
     a.ilu_only = ilu_only ? 1 : 0;
     a.qsign = qsign;
     a.onecl = csz ? 1 : 0;
-    a.alpha = kind ? g_knobs.mg_alpha : g_knobs.mg_alpha * MG_OVER;
+    a.alpha = kind ? g_knobs.mg_alpha : g_knobs.mg_alpha_p;
     a.rtol = rtol;
     a.atol = atol;
     a.rec = ks0;

@@ -558,7 +558,7 @@ static void vcycle_t(const Ctx &c, const MGHost &mg, int bsel, int xsel, int wse
     }
     size_t smem = 0;
     const int Ls = small_plan<T>(c, mg, &smem);
-    const double alpha = wsel ? mg.alpha : mg.alpha * MG_OVER;      // wsel 0: Poisson
+    const double alpha = wsel ? mg.alpha : mg.alpha_p;      // wsel 0: Poisson
     for (int L = 0; L < Ls; L++) {
         SS_LAUNCH_PDL(SB, mg.maxN[L], smooth_fn<T>(0, 1), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);
         SS_LAUNCH_PDL(SR, mg.maxN[L], smooth_fn<T>(0, 0), grid_half(c, L, mg), ROW_BLOCK, c.st, c.dP, L, bsel, xsel, gate);

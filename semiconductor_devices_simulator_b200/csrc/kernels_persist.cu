@@ -1576,7 +1576,7 @@ int persist_pcg(const Ctx &c, const MGHost &mg, int mixed, KrylovS &k) {
     a.qsign = 0;
     a.deep = g_deep_levels;
     a.sweeps2 = 0;                              // one application (MG_OVER, solver_ctx.h)
-    a.alpha = mg.alpha * MG_OVER;
+    a.alpha = mg.alpha_p;
     a.barmode = g_barmode;
     a.rec[0] = k;
     PGridHead h{};

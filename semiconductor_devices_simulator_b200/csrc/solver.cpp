@@ -1469,6 +1469,7 @@ int prepare(Inst &d) {
     if (want_ion) launch_ion_neutral(make_ctx(d));
     CK(cudaStreamSynchronize(st));
     d.g.mg.alpha = g_knobs.mg_alpha;
+    d.g.mg.alpha_p = g_knobs.mg_alpha_p;
     d.dirty = 0;
     static std::atomic<unsigned long long> gen{0};
     d.upload_gen = ++gen;

@@ -19,7 +19,7 @@ struct MGHost {
     int maxN[MAXLEV] = {0};
     int maxNx[MAXLEV] = {0};       // largest x extent of the level
     int maxRows[MAXLEV] = {0};     // largest Ny*Nz of the level
-    double alpha = 1.0;
+    double alpha = 1.0, alpha_p = 1.0;   // prolongation factors: continuity, Poisson
 };
 double bench_la_kernel(const Ctx &c, const MGHost &mg, int which, int reps);
 extern int g_small_nodes;
@@ -176,7 +176,8 @@ struct Inst {
     int n_tsp = 0;
 };
 
-// Over-correction of the coarse corrections in the Poisson solves, times the knob mg_alpha.
+// Over-correction of the coarse corrections in the Poisson solves, unless the caller sets the
+// factor (SEMISIM_MGA, which is then every solve's as it stands).
 // The prolongation is constant on an aggregate, so the coarse correction of a smooth error is
 // too short; scaled by 1.2 PCG takes 354 iterations instead of 425 (576,000-node MOSFET, FP64 from
 // scratch; 375 at 1.1, 338 at 1.3, 342 at 1.5), and one smoother application on the finest level
@@ -189,7 +190,7 @@ constexpr double MG_OVER = 1.2;
 
 // global knobs (the reference's static tunables, read by api3_init)
 struct Knobs {
-    double mg_alpha = 1.0;
+    double mg_alpha = 1.0, mg_alpha_p = MG_OVER;   // prolongation factors: continuity, Poisson
     int gpass = 3;               // graph multigrid: rounds of pairwise matching per level
     double gbeta = 0.5;          //   and the strength threshold of a match
     int aa_depth = AA_MAX;
