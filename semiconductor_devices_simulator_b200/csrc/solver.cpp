@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cmath>
 #include <atomic>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -54,8 +55,11 @@ int g_precision_default = 0;
 
 int use_mixed(const Inst &d) { return (d.precision < 0 ? g_precision_default : d.precision) == 1 ? 1 : 0; }
 
+static void persist_work(Inst &d);
+
 Ctx make_ctx(Inst &d) {
     if (g_device >= 0) cudaSetDevice(g_device);
+    persist_work(d);
     Ctx c;
     c.dP = d.g.d;
     c.h = d.g.h;
@@ -96,7 +100,7 @@ struct Carver {
 
 // Lay out every device array of an instance in one block (two passes: size, then place).
 static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &levs, std::vector<LevelT<float>> &levsf,
-                  SWork<double> &pwd, SWork<float> &pwf, int nlev, const int dims[][6]) {
+                  int nlev, const int dims[][6]) {
     const size_t N = d.N;
     P.flags = cv.take<uint32_t>(N);
     P.Nd = cv.take<double>(N); P.Na = cv.take<double>(N); P.Nf = cv.take<double>(N);
@@ -183,13 +187,6 @@ static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &lev
         v.pw = cv.take<float>(n);
         v.ph = levs[L].ph;              // set-up scratch, shared with the FP64 twin
     }
-    if (!d.unstr) {                      // the persistent solves' hierarchy (graph meshes have their own)
-        P.pwd = cv.take<SWork<double>>(1);
-        P.pwf = cv.take<SWork<float>>(1);
-        char *area = cv.take<char>(persist_work_layout<double>(nullptr, dims, nlev, nullptr));
-        persist_work_layout<double>(area, dims, nlev, &pwd);
-        persist_work_layout<float>(area, dims, nlev, &pwf);
-    }
 }
 
 // 2x2x2 aggregation hierarchy shape (semiconductor_3d.c:1894-1921)
@@ -218,6 +215,7 @@ void gpu_free(Inst &d) {
     for (auto &e : d.g.tev)
         if (e) cudaEventDestroy(e);
     if (d.g.block) cudaFree(d.g.block);
+    if (d.g.pwblock) cudaFree(d.g.pwblock);
     if (d.g.d) cudaFree(d.g.d);
     if (d.g.pin) cudaFreeHost(d.g.pin);
     if (d.g.scratch) cudaFree(d.g.scratch);
@@ -238,8 +236,52 @@ void gpu_free(Inst &d) {
     d.g = Gpu();
 }
 
+// The persistent solves' hierarchy and vectors (165 B a node; graph meshes have their own): an
+// allocation apart, taken once such solves are on, also when they are switched on later.  Where
+// it does not fit the solves run per pass, so it takes no room from a device that does.
+static void persist_work(Inst &d) {
+    Gpu &g = d.g;
+    if (!g.ready || d.unstr || g.h.pwd || g.pw_off || !persist_enabled()) return;
+    int dims[MAXLEV][6];
+    const int nl = mg_levels(d.Nx, d.Ny, d.Nz, dims);
+    const size_t head = align_up(sizeof(SWork<double>)) + align_up(sizeof(SWork<float>));
+    const size_t bytes = head + persist_work_layout<double>(nullptr, dims, nl, nullptr);
+    void *blk = nullptr;
+    SWork<double> wd{};
+    SWork<float> wf{};
+    g.pw_off = true;
+    if (nl < 2) return;
+    if (cudaMalloc(&blk, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        std::fprintf(stderr, "semisim-b200: no device memory for the persistent solves' workspace; per-pass solves\n");
+        return;
+    }
+    char *const p = static_cast<char *>(blk);
+    persist_work_layout<double>(p + head, dims, nl, &wd);
+    persist_work_layout<float>(p + head, dims, nl, &wf);
+    DevP q = g.h;
+    q.pwd = reinterpret_cast<SWork<double> *>(p);
+    q.pwf = reinterpret_cast<SWork<float> *>(p + align_up(sizeof(SWork<double>)));
+    static_assert(offsetof(DevP, pwf) == offsetof(DevP, pwd) + sizeof q.pwd, "uploaded together");
+    if (cudaMemsetAsync(p, 0, bytes, g.st) != cudaSuccess ||
+        cudaMemcpyAsync(q.pwd, &wd, sizeof wd, cudaMemcpyHostToDevice, g.st) != cudaSuccess ||
+        cudaMemcpyAsync(q.pwf, &wf, sizeof wf, cudaMemcpyHostToDevice, g.st) != cudaSuccess ||
+        cudaMemcpyAsync(reinterpret_cast<char *>(g.d) + offsetof(DevP, pwd), &q.pwd, sizeof q.pwd + sizeof q.pwf,
+                        cudaMemcpyHostToDevice, g.st) != cudaSuccess ||
+        cudaStreamSynchronize(g.st) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(blk);
+        return;
+    }
+    g.pw_off = false;
+    g.pwblock = blk;
+    g.bytes += bytes;
+    g.h.pwd = q.pwd;
+    g.h.pwf = q.pwf;
+}
+
 static int gpu_alloc(Inst &d) {
-    if (d.g.ready && d.g.h.Nx == d.Nx && d.g.h.Ny == d.Ny && d.g.h.Nz == d.Nz && (d.unstr || d.g.h.pwd)) return 1;
+    if (d.g.ready && d.g.h.Nx == d.Nx && d.g.h.Ny == d.Ny && d.g.h.Nz == d.Nz) return 1;
     gpu_free(d);
     if (!gpu_available()) {
         std::fprintf(stderr, "semisim-b200: no CUDA device available - the solver has no CPU path\n");
@@ -265,9 +307,7 @@ static int gpu_alloc(Inst &d) {
     DevP P{};
     std::vector<LevelT<double>> levs;
     std::vector<LevelT<float>> levsf;
-    SWork<double> pwd{};
-    SWork<float> pwf{};
-    carve(d, cv, P, levs, levsf, pwd, pwf, nl, dims);       // sizing pass
+    carve(d, cv, P, levs, levsf, nl, dims);       // sizing pass
     const size_t bytes = cv.off;
     void *blk = nullptr;
     CK(cudaMalloc(&blk, bytes));
@@ -275,7 +315,7 @@ static int gpu_alloc(Inst &d) {
     Carver cv2;
     cv2.base = static_cast<char *>(blk);
     P = DevP{};
-    carve(d, cv2, P, levs, levsf, pwd, pwf, nl, dims);
+    carve(d, cv2, P, levs, levsf, nl, dims);
     P.Nx = d.Nx; P.Ny = d.Ny; P.Nz = d.Nz; P.N = (int)d.N; P.nlev = nl;
     d.g.block = blk;
     d.g.bytes = bytes;
@@ -297,10 +337,6 @@ static int gpu_alloc(Inst &d) {
             }
     CK(cudaMemcpy(P.lev, levs.data(), sizeof(LevelT<double>) * nl, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(P.levf, levsf.data(), sizeof(LevelT<float>) * nl, cudaMemcpyHostToDevice));
-    if (P.pwd) {
-        CK(cudaMemcpy(P.pwd, &pwd, sizeof pwd, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(P.pwf, &pwf, sizeof pwf, cudaMemcpyHostToDevice));
-    }
     MGHost &mg = d.g.mg;
     mg.maxlev = mg.minlev = nl;
     for (int L = 0; L < nl; L++) {
@@ -1466,6 +1502,8 @@ int prepare(Inst &d) {
     if (want_ion)
         CK(cudaMemcpyAsync(d.g.ion, ionx.data(), ionx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d.g.d, &P, sizeof(DevP), cudaMemcpyHostToDevice, st));
+    d.g.pw_off = false;                    // (P is d.g.h: the workspace enters both records)
+    persist_work(d);
     if (want_ion) launch_ion_neutral(make_ctx(d));
     CK(cudaStreamSynchronize(st));
     d.g.mg.alpha = g_knobs.mg_alpha;
