@@ -1609,6 +1609,7 @@ int poisson_newton(Inst &d, const double *Va, double ntol, int maxit) {
         const double f0 = d.g.pin[0], dm = d.g.pin[1];
         if (!(f0 > 0.)) return f0 == 0.;
         if (dm != dm) return 0;
+        if (dm == 0. && f0 > ntol) return 0;             // PCG broke down at its start: no step, no convergence
         if (dm < ntol) {
             launch_axpy_sel(c, V_PHI, V_PHI, 1.0, V_SOL);   // psi += dx
             return 1;
