@@ -399,9 +399,12 @@ __device__ void gp_pivots(const PGLev &v, int c, int tid, int nth) {
     }
 }
 // Dense inverse of the coarsest level by Gauss-Jordan on the diagonal pivots (tiny ones set to
-// 1e-300 as semiconductor_3d.c:2620 does).  The Galerkin operators of these systems keep the
-// sign pattern and the column dominance of the M-matrices they come from, which need no row
-// interchanges; a poor inverse would only cost iterations, the solve checks its own residual.
+// 1e-300 as semiconductor_3d.c:2620 does).  No row interchanges: what leaves a node enters its
+// neighbours, so with the row scaling taken out the columns of these systems sum to what
+// recombination, exchange and contacts take (>= 0), their couplings are not positive, and both
+// survive the sums over aggregates, the prolongation's weights (>= 0) and elimination.  The largest
+// entry of a pivot column is thus its diagonal, which partial pivoting would take too (checked on
+// diode, MOSFET and tunnelling systems by test_gpu_graph_coarse_dominance.py).
 // Up to GP_INV_REG unknowns: nbk blocks own rb rows each, 16 lanes hold a row in registers.
 // Four columns C at a time: their owner publishes the four rows P as they are, and after one
 // barrier every row takes  row -= g P  with g = row_C D^-1, D the 4x4 pivot block (columns C
