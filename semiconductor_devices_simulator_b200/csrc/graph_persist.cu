@@ -32,7 +32,6 @@
 #include <cstdlib>
 #include <vector>
 
-#include "gmg_common.cuh"
 #include "persist_common.cuh"
 #include "prof.h"
 #include "solver_ctx.h"

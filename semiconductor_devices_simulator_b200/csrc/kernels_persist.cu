@@ -35,10 +35,12 @@
 // The stop rules are the reference's (pcg semiconductor_3d.c:2182-2210, bicgstab_core
 // :2234-2320) as the per-pass path applies them, and the refinement the same FP64 rule.
 //
-// Safety: the launch is cooperative (all blocks co-resident).  Every barrier wait is
-// bounded: after 2 s of waiting a block sets the error word and leaves, every other block
+// Safety: the launch is cooperative (all blocks co-resident).  Every wait at a grid barrier is
+// bounded: after 2 s a block sets the error word and leaves, every other block
 // leaves at its next wait, and the host restores the solve's start and repeats it on the
-// per-pass path.
+// per-pass path.  The cluster barriers (one-cluster grids, and the coarse levels in the first
+// cluster) are the hardware's and have no limit: a cluster is scheduled as a whole, its blocks
+// pass the same barriers between two grid barriers, and blocks that have left are not waited for.
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
@@ -923,7 +925,7 @@ __device__ __noinline__ void invert_rows(T *D, int n, int nt, int *piv) {
         const bool own = ch == (c & 1);
         if (own) cc[r] = a[0];                               // (rows past n: zeros)
         warps_sync(1, nt);
-        unsigned key = 0;                                    // |a| to 17 bits, ties to the lower row
+        unsigned key = 0;                                    // |a| to 15 bits of mantissa, ties to the lower row
         {
             const unsigned h0 = (unsigned)__double2hiint(cc[lane]), k0 = ((h0 << 1) & ~63u) | (unsigned)(63 - lane);
             key = open0 ? k0 : 0u;

@@ -1,8 +1,9 @@
-// Device helpers of the 7-point multigrid and Krylov kernels, shared by the per-pass
-// kernels (kernels_la.cu) and the persistent solve kernels (kernels_persist.cu): where
+// Device helpers of the per-pass 7-point multigrid and Krylov kernels (kernels_la.cu): where
 // each precision's vectors and hierarchy live in an instance record, level views, the
 // stencil products, the 2x2x2 aggregate ranges, the red-black D-ILU smoother update of
-// one node, and the shared-memory layout of the small levels.
+// one node, and the shared-memory layout of the small levels.  The persistent solves
+// (kernels_persist.cu) have a layout and passes of their own; they take the precision traits, the
+// aggregate ranges and the nodes' reference potentials from here.
 #pragma once
 #include <type_traits>
 

@@ -542,7 +542,6 @@ __global__ void __launch_bounds__(WG_TPB) k_mlp_wgrad(WgArgs a) {
     else wgrad_layer<MO, MH>(sm, a.dY, a.H + 2 * L, a.B, b - a.off[3], a.off[4] - a.off[3], a.G + OW4, a.G + OB4);
 }
 
-// Adam on the FP32 parameters with bias-corrected moments (c1 = 1 - b1^t, c2 = 1 - b2^t)
 // BF16 weight pack and bias vector [b1 | b2 | b3 | b4] entry of FP32 parameter i
 __device__ __forceinline__ void pack_param(int i, float v, bf16 *Wb, float *bias) {
     if (i < OB1) Wb[QW1 + i - OW1] = __float2bfloat16(v);
@@ -554,6 +553,7 @@ __device__ __forceinline__ void pack_param(int i, float v, bf16 *Wb, float *bias
     else if (i < OB4) Wb[QW4 + i - OW4] = __float2bfloat16(v);
     else bias[3 * MH + i - OB4] = v;
 }
+// Adam on the FP32 parameters with bias-corrected moments (c1 = 1 - b1^t, c2 = 1 - b2^t)
 __global__ void k_mlp_adam(float *P, const float *G, float *M, float *V, int n, float lr, float b1, float b2, float eps,
                            float c1, float c2, bf16 *Wb, float *bias) {
     SS_GRID_LOOP(i, n) {

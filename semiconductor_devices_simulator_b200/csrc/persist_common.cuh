@@ -2,7 +2,8 @@
 // solve) kernels of the tensor and graph solve paths.
 //
 // Barrier: every block arrives (release), thread 0 of each block waits for all arrivals
-// (acquire).  Every wait is bounded: after the launch's limit a block sets the error word
+// (acquire); a grid of one cluster uses the cluster's hardware barrier, which has no limit.  Every
+// other wait is bounded: after the launch's limit a block sets the error word
 // and leaves, every other block leaves at its next wait, and the host, which reads the
 // error word after the launch, repeats the solve on the per-pass path.
 //
@@ -17,10 +18,6 @@
 
 namespace ss {
 
-#ifndef PG_TPB_SET
-#define PG_TPB_SET 1024
-#endif
-constexpr int PG_TPB = PG_TPB_SET;
 constexpr unsigned long long PG_WAIT_NS = 2000000000ull;    // longest barrier wait of a solve (2 s)
 
 __device__ __forceinline__ unsigned long long pg_clock() {
