@@ -75,7 +75,7 @@ def parse():
     ap.add_argument("--predictor", default=None, choices=["quadratic", "secant"],
                     help="sweep predictor of the timed steps: quadratic through the last three points or the "
                          "reference's secant step (default: quadratic, secant for the FinFET, whose on-state "
-                         "currents move by 1.7e-4 with the start at its production tolerances); the other one "
+                         "currents move by 4.4e-4 with the start at its production tolerances); the other one "
                          "is timed on one more step")
     ap.add_argument("--share", default="gummel", choices=["gummel", "none"],
                     help="grid shares of concurrently solved sweeps: by the first step's Gummel iterations, "
