@@ -100,7 +100,7 @@ struct Carver {
 
 // Lay out every device array of an instance in one block (two passes: size, then place).
 static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &levs, std::vector<LevelT<float>> &levsf,
-                  int nlev, const int dims[][6]) {
+                  int nlev, const int dims[][6], size_t work, char **area) {
     const size_t N = d.N;
     P.flags = cv.take<uint32_t>(N);
     P.Nd = cv.take<double>(N); P.Na = cv.take<double>(N); P.Nf = cv.take<double>(N);
@@ -187,6 +187,7 @@ static void carve(Inst &d, Carver &cv, DevP &P, std::vector<LevelT<double>> &lev
         v.pw = cv.take<float>(n);
         v.ph = levs[L].ph;              // set-up scratch, shared with the FP64 twin
     }
+    *area = work ? cv.take<char>(work) : nullptr;
 }
 
 // 2x2x2 aggregation hierarchy shape (semiconductor_3d.c:1894-1921)
@@ -236,37 +237,50 @@ void gpu_free(Inst &d) {
     d.g = Gpu();
 }
 
-// The persistent solves' hierarchy and vectors (165 B a node; graph meshes have their own): an
-// allocation apart, taken once such solves are on, also when they are switched on later.  Where
-// it does not fit the solves run per pass, so it takes no room from a device that does.
+// The persistent solves' hierarchy and vectors (165 B a node; graph meshes have their own), taken
+// where such solves are on.  With the node arrays where the memory allows it (PW_SPARE bytes a
+// node stay free for the models' own arrays): in an allocation apart the smallest devices, whose arrays fill
+// a few pages, took 2 % longer (1,455-node diode 52.6 -> 53.8 ms).  Apart when the solves are switched on
+// later, or when room is left after the rest of the set-up; else the solves run per pass.
+constexpr size_t PW_SPARE = 256;
+constexpr size_t PW_HEAD = ((sizeof(SWork<double>) + 255) & ~size_t(255)) + ((sizeof(SWork<float>) + 255) & ~size_t(255));
+static size_t persist_work_bytes(const Inst &d, const int dims[][6], int nl) {
+    return d.unstr || nl < 2 || !persist_enabled() ? 0 : PW_HEAD + persist_work_layout<double>(nullptr, dims, nl, nullptr);
+}
+// tables of the zeroed workspace p on the device, and its place in `h`
+static bool persist_work_tables(char *p, const int dims[][6], int nl, DevP &h) {
+    SWork<double> wd{};
+    SWork<float> wf{};
+    persist_work_layout<double>(p + PW_HEAD, dims, nl, &wd);
+    persist_work_layout<float>(p + PW_HEAD, dims, nl, &wf);
+    SWork<double> *const td = reinterpret_cast<SWork<double> *>(p);
+    SWork<float> *const tf = reinterpret_cast<SWork<float> *>(p + align_up(sizeof wd));
+    if (cudaMemcpy(td, &wd, sizeof wd, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(tf, &wf, sizeof wf, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess)       // (the instance's stream does not wait for these copies)
+        return false;
+    h.pwd = td;
+    h.pwf = tf;
+    return true;
+}
 static void persist_work(Inst &d) {
     Gpu &g = d.g;
     if (!g.ready || d.unstr || g.h.pwd || g.pw_off || !persist_enabled()) return;
     int dims[MAXLEV][6];
     const int nl = mg_levels(d.Nx, d.Ny, d.Nz, dims);
-    const size_t head = align_up(sizeof(SWork<double>)) + align_up(sizeof(SWork<float>));
-    const size_t bytes = head + persist_work_layout<double>(nullptr, dims, nl, nullptr);
+    const size_t bytes = persist_work_bytes(d, dims, nl);
     void *blk = nullptr;
-    SWork<double> wd{};
-    SWork<float> wf{};
     g.pw_off = true;
-    if (nl < 2) return;
+    if (!bytes) return;
     if (cudaMalloc(&blk, bytes) != cudaSuccess) {
         cudaGetLastError();
         std::fprintf(stderr, "semisim-b200: no device memory for the persistent solves' workspace; per-pass solves\n");
         return;
     }
-    char *const p = static_cast<char *>(blk);
-    persist_work_layout<double>(p + head, dims, nl, &wd);
-    persist_work_layout<float>(p + head, dims, nl, &wf);
-    DevP q = g.h;
-    q.pwd = reinterpret_cast<SWork<double> *>(p);
-    q.pwf = reinterpret_cast<SWork<float> *>(p + align_up(sizeof(SWork<double>)));
-    static_assert(offsetof(DevP, pwf) == offsetof(DevP, pwd) + sizeof q.pwd, "uploaded together");
-    if (cudaMemsetAsync(p, 0, bytes, g.st) != cudaSuccess ||
-        cudaMemcpyAsync(q.pwd, &wd, sizeof wd, cudaMemcpyHostToDevice, g.st) != cudaSuccess ||
-        cudaMemcpyAsync(q.pwf, &wf, sizeof wf, cudaMemcpyHostToDevice, g.st) != cudaSuccess ||
-        cudaMemcpyAsync(reinterpret_cast<char *>(g.d) + offsetof(DevP, pwd), &q.pwd, sizeof q.pwd + sizeof q.pwf,
+    DevP h{};
+    static_assert(offsetof(DevP, pwf) == offsetof(DevP, pwd) + sizeof h.pwd, "uploaded together");
+    if (cudaMemset(blk, 0, bytes) != cudaSuccess || !persist_work_tables(static_cast<char *>(blk), dims, nl, h) ||
+        cudaMemcpyAsync(reinterpret_cast<char *>(g.d) + offsetof(DevP, pwd), &h.pwd, sizeof h.pwd + sizeof h.pwf,
                         cudaMemcpyHostToDevice, g.st) != cudaSuccess ||
         cudaStreamSynchronize(g.st) != cudaSuccess) {
         cudaGetLastError();
@@ -276,8 +290,8 @@ static void persist_work(Inst &d) {
     g.pw_off = false;
     g.pwblock = blk;
     g.bytes += bytes;
-    g.h.pwd = q.pwd;
-    g.h.pwf = q.pwf;
+    g.h.pwd = h.pwd;
+    g.h.pwf = h.pwf;
 }
 
 static int gpu_alloc(Inst &d) {
@@ -307,7 +321,15 @@ static int gpu_alloc(Inst &d) {
     DevP P{};
     std::vector<LevelT<double>> levs;
     std::vector<LevelT<float>> levsf;
-    carve(d, cv, P, levs, levsf, nl, dims);       // sizing pass
+    char *area = nullptr;
+    size_t work = persist_work_bytes(d, dims, nl), avail = 0, total = 0;
+    carve(d, cv, P, levs, levsf, nl, dims, work, &area);       // sizing pass
+    if (work && (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail < cv.off + PW_SPARE * d.N)) {
+        cudaGetLastError();
+        work = 0;
+        cv = Carver();
+        carve(d, cv, P, levs, levsf, nl, dims, work, &area);
+    }
     const size_t bytes = cv.off;
     void *blk = nullptr;
     CK(cudaMalloc(&blk, bytes));
@@ -315,7 +337,7 @@ static int gpu_alloc(Inst &d) {
     Carver cv2;
     cv2.base = static_cast<char *>(blk);
     P = DevP{};
-    carve(d, cv2, P, levs, levsf, nl, dims);
+    carve(d, cv2, P, levs, levsf, nl, dims, work, &area);
     P.Nx = d.Nx; P.Ny = d.Ny; P.Nz = d.Nz; P.N = (int)d.N; P.nlev = nl;
     d.g.block = blk;
     d.g.bytes = bytes;
@@ -337,6 +359,11 @@ static int gpu_alloc(Inst &d) {
             }
     CK(cudaMemcpy(P.lev, levs.data(), sizeof(LevelT<double>) * nl, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(P.levf, levsf.data(), sizeof(LevelT<float>) * nl, cudaMemcpyHostToDevice));
+    if (area && !persist_work_tables(area, dims, nl, d.g.h)) {
+        std::fprintf(stderr, "semisim-b200: the persistent solves' tables could not be uploaded\n");
+        gpu_free(d);
+        return 0;
+    }
     MGHost &mg = d.g.mg;
     mg.maxlev = mg.minlev = nl;
     for (int L = 0; L < nl; L++) {

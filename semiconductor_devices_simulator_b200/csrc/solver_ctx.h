@@ -64,7 +64,7 @@ struct Gpu {
     int dev = 0;
     size_t N = 0, bytes = 0;
     void *block = nullptr;       // one allocation for all node arrays
-    void *pwblock = nullptr;     // the persistent solves' workspace (persist_work, solver.cpp)
+    void *pwblock = nullptr;     // the persistent solves' workspace where it lies apart (persist_work, solver.cpp)
     bool pw_off = false;         //   which does not fit, or serves no solve of this mesh
     DevP h{};                    // host copy of the device record
     DevP *d = nullptr;           // device record
